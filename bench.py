@@ -632,7 +632,7 @@ def run_cells(args, D):
     vol_ms = statistics.mean(r["ms"]["volumes"] for r in reps)
     ach = algo / (vol_ms * 1e-3) / 1e9
     peak, peak_kind = peaks()
-    tuned = int(rep["threads"]["volumes"])  # the e2e calls reuse the CTA size tuned above
+    tuned = int(rep["threads"]["volumes"])  # the CTA size of the device-timed builds
     check = None
     if D.rank == 0 and not args.no_oracle_check:
         check = cells_oracle_error(cm, C.bases(), args.face_material)
@@ -688,7 +688,7 @@ def run_cells(args, D):
                  "inner_iterations_mean": float(rep["inner"].mean()), "inner_iterations_max": int(rep["inner"].max()),
                  "refinement_steps_mean": float(rep["outer"].mean()), "rel_residual_max": float(rep["rel"].max()),
                  "face_rel_residual_max": float(rep["face_rel"].max()), "step_ms_all": ts,
-                 "autotuned_cta_threads": rep["threads"],
+                 "cta_threads": rep["threads"],
                  "inner_precision": "FP64" if PREC == FP64 else "FP32 in FP64 refinement",
                  "comparator_other_precision": other}
         extra["face_material"] = ("material 0 on the face and edge problems, as the reference's own construction"

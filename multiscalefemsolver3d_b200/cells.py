@@ -94,7 +94,7 @@ class Cells:
         self.h = h
 
     def build_bases(self, precision=FP32_IR, tol=1e-8, maxiter=5000, threads=0):
-        """threads = CTA size of the persistent solves; 0 autotunes it on the first build."""
+        """threads = CTA size of the persistent solves; 0 chooses it from the cells' sizes."""
         return check(load().msfem_cells_build_bases(self.h, precision, tol, maxiter, threads), "cells_build_bases")
 
     def set_face_material(self, mode: str):

@@ -1,5 +1,5 @@
-// Batched cell systems: sort-based deterministic portrait + assembly, and a
-// persistent MINRES solver with one CTA per system.
+// Batched cell systems: sort-based deterministic portrait + assembly (the persistent solver is
+// batch_minres.cu).
 //
 // Portrait and assembly.  The reference builds each cell problem's portrait
 // (Grid_forMech::CreationPortrait, FEM/FEM_Grid.h:3236-3287) and adds the element
@@ -13,16 +13,6 @@
 // sorted, diagonal included); the sorted tags are kept, so assembling a block is
 // a gather-sum of its contributions in the same order as the reference's serial
 // scatter -- no colouring, no atomics, the same bits on every run.
-//
-// Solve.  A cell problem has Dirichlet data on its whole boundary and zero
-// source; its matrix is symmetric but, with stiff inclusions, indefinite (the
-// reference's transposed element blocks leave interface terms; a few negative
-// eigenvalues appear), so the inner solver is MINRES on the Jacobi-scaled free
-// block S A_II S.  One persistent launch covers every system: each CTA takes the
-// next system from an atomic queue (largest first), runs the FP64 outer
-// refinement (true residual r = -A x with the Dirichlet values in x) and the
-// inner MINRES for all R right-hand sides at once (one recurrence per
-// right-hand side, one shared sparse product), with CTA barriers only.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -172,7 +162,7 @@ __global__ void k_assemble_given(int64_t nnzb, const int64_t* __restrict__ cstar
     }
 }
 
-// s = 1/sqrt(A_ii[a][a]) (1 when not positive), then the scaled FP32 copy, row by row
+// s = 1/sqrt(A_ii[a][a]) (1 when not positive)
 __global__ void k_batch_scale(int64_t n_nodes, const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
                               const double* __restrict__ val, double* __restrict__ dscale)
 {
@@ -186,452 +176,6 @@ __global__ void k_batch_scale(int64_t n_nodes, const int64_t* __restrict__ row_p
             }
         for (int a = 0; a < 3; a++) dscale[3 * i + a] = d[a] > 0.0 ? 1.0 / sqrt(d[a]) : 1.0;
     }
-}
-
-__global__ void k_batch_val32(int64_t n_nodes, const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
-                              const double* __restrict__ val, const double* __restrict__ dscale, float* __restrict__ v32)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += (int64_t)gridDim.x * blockDim.x) {
-        const double si[3] = {dscale[3 * i], dscale[3 * i + 1], dscale[3 * i + 2]};
-        for (int64_t k = row_ptr[i]; k < row_ptr[i + 1]; k++) {
-            const int64_t j = col[k];
-            const double sj[3] = {dscale[3 * j], dscale[3 * j + 1], dscale[3 * j + 2]};
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) v32[9 * k + 3 * a + b] = (float)(si[a] * val[9 * k + 3 * a + b] * sj[b]);
-        }
-    }
-}
-
-// ------------------------------------------------------------------ persistent solver
-
-struct BatchArgs {
-    int n_sys;
-    const int32_t* order;
-    const int64_t* node_off;
-    const int64_t* row_ptr;
-    const int32_t* col;
-    const double* val64;
-    const float* val32;
-    const double* dscale;
-    const uint8_t* fixed;
-    double* x;
-    const double* rhs;  // [n_nodes][R][3] source term, or null (zero source)
-    void* work;
-    int64_t work_stride;  // elements of VT per vector
-    int* queue;
-    int32_t* iters;
-    int32_t* outers;
-    double* rel;
-    double tol;
-    int maxiter;
-    int max_outer;
-};
-
-struct MrRhs {
-    double alpha, beta, eta, c0, s0, c1, s1, eps, delta, gamma, tau, bnext, b1, target, fnorm2;
-    int active, upd;
-};
-
-// per right-hand-side block reduction: thread t holds a partial of rhs t % R
-template <int R>
-__device__ __forceinline__ void rhs_sum(double v, double* red, double* out)
-{
-#pragma unroll
-    for (int o = 16; o >= R; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane < R) red[warp * R + lane] = v;
-    __syncthreads();
-    if (threadIdx.x < R) {
-        double t = 0.0;
-        for (int w = 0; w < nw; w++) t += red[w * R + threadIdx.x];
-        out[threadIdx.x] = t;
-    }
-    __syncthreads();
-}
-
-// y = S A S v on the free rows of one system (VT float: pre-scaled FP32 values;
-// VT double: FP64 values scaled on the fly); rows of Dirichlet nodes give 0.
-template <int R, class VT>
-__device__ __forceinline__ void row_product(const BatchArgs& A, int64_t n0, int i, int r, const VT* __restrict__ v,
-                                            VT y[3])
-{
-    const int64_t gi = n0 + i;
-    VT acc[3] = {0, 0, 0};
-    for (int64_t k = A.row_ptr[gi]; k < A.row_ptr[gi + 1]; k++) {
-        const int64_t c = A.col[k] - n0;
-        const VT* xv = v + (c * R + r) * 3;
-        if (sizeof(VT) == 4) {
-            const float* a = A.val32 + 9 * k;
-            const VT x0 = xv[0], x1 = xv[1], x2 = xv[2];
-            acc[0] += (VT)a[0] * x0 + (VT)a[1] * x1 + (VT)a[2] * x2;
-            acc[1] += (VT)a[3] * x0 + (VT)a[4] * x1 + (VT)a[5] * x2;
-            acc[2] += (VT)a[6] * x0 + (VT)a[7] * x1 + (VT)a[8] * x2;
-        } else {
-            const double* a = A.val64 + 9 * k;
-            const double* sj = A.dscale + 3 * (n0 + c);
-            const double x0 = (double)xv[0] * sj[0], x1 = (double)xv[1] * sj[1], x2 = (double)xv[2] * sj[2];
-            acc[0] += a[0] * x0 + a[1] * x1 + a[2] * x2;
-            acc[1] += a[3] * x0 + a[4] * x1 + a[5] * x2;
-            acc[2] += a[6] * x0 + a[7] * x1 + a[8] * x2;
-        }
-    }
-    if (sizeof(VT) == 4) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) y[a] = acc[a];
-    } else {
-        const double* si = A.dscale + 3 * gi;
-#pragma unroll
-        for (int a = 0; a < 3; a++) y[a] = (VT)(si[a] * (double)acc[a]);
-    }
-}
-
-// Shared state of one CTA's solve (one system at a time).
-template <int R>
-struct CtaShared {
-    double red[32 * R];
-    double s1[R], s2[R];
-    MrRhs mr[R];
-    double rr_prev[R];
-    int q, active, conv, bad;
-};
-
-// FP64 residual r = -A x on the free rows of the CTA's system (x holds the Dirichlet
-// values), written scaled (v = S r) into V; sums ||r||^2 -> s1, ||v||^2 -> s2 per rhs.
-template <int R, class VT>
-__device__ void residual_pass(const BatchArgs& A, int64_t n0, int np, const uint8_t* fx, const double* X, VT* V,
-                              CtaShared<R>& sh)
-{
-    const int tid = threadIdx.x, T = blockDim.x, r = tid % R;
-    double arr = 0.0, avv = 0.0;
-    for (int p = tid; p < np; p += T) {
-        const int i = p / R;
-        if (fx[i]) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) V[3 * (int64_t)p + c] = 0;
-            continue;
-        }
-        const int64_t gi = n0 + i;
-        double y[3] = {0, 0, 0};
-        if (A.rhs)
-#pragma unroll
-            for (int c = 0; c < 3; c++) y[c] = A.rhs[(n0 * R + p) * 3 + c];
-        for (int64_t k = A.row_ptr[gi]; k < A.row_ptr[gi + 1]; k++) {
-            const int64_t cc = A.col[k] - n0;
-            const double* a = A.val64 + 9 * k;
-            const double* xv = X + (cc * R + r) * 3;
-            y[0] -= a[0] * xv[0] + a[1] * xv[1] + a[2] * xv[2];
-            y[1] -= a[3] * xv[0] + a[4] * xv[1] + a[5] * xv[2];
-            y[2] -= a[6] * xv[0] + a[7] * xv[1] + a[8] * xv[2];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            arr += y[c] * y[c];
-            const VT vs = (VT)(A.dscale[3 * gi + c] * y[c]);
-            V[3 * (int64_t)p + c] = vs;
-            avv += (double)vs * (double)vs;
-        }
-    }
-    rhs_sum<R>(arr, sh.red, sh.s1);
-    rhs_sum<R>(avv, sh.red, sh.s2);
-}
-
-// x += sign * S y on the free rows, for the rhs with want[r] set (all when want is null)
-template <int R, class VT>
-__device__ void apply_correction(const BatchArgs& A, int64_t n0, int np, const uint8_t* fx, double* X, const VT* Y,
-                                 double sign, const int* want)
-{
-    const int tid = threadIdx.x, T = blockDim.x;
-    if (want && !want[tid % R]) return;
-    for (int p = tid; p < np; p += T) {
-        const int i = p / R;
-        if (fx[i]) continue;
-        const int64_t gi = n0 + i;
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-            X[3 * (int64_t)p + c] += sign * A.dscale[3 * gi + c] * (double)Y[3 * (int64_t)p + c];
-    }
-}
-
-// MINRES on S A_II S y = v (v = Vb[1] on entry, ||v|| = mr[r].b1), for all R rhs at once;
-// returns the iterations.  The solution is left in Y.
-template <int R, class VT>
-__device__ int inner_minres(const BatchArgs& A, int64_t n0, int np, const uint8_t* fx, VT* base, CtaShared<R>& sh)
-{
-    const int tid = threadIdx.x, T = blockDim.x;
-    const int rr_ = tid % R;
-    const int64_t S = A.work_stride;
-    VT* Vb[3] = {base, base + S, base + 2 * S};
-    VT* Wb[2] = {base + 3 * S, base + 4 * S};
-    VT* Y = base + 5 * S;
-    {
-        const double b1 = sh.mr[rr_].b1;
-        const VT inv = (VT)(b1 > 0.0 ? 1.0 / b1 : 0.0);
-        for (int p = tid; p < np; p += T)
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const int64_t o = 3 * (int64_t)p + c;
-                Vb[1][o] *= inv;
-                Vb[0][o] = 0;
-                Wb[0][o] = 0;
-                Wb[1][o] = 0;
-                Y[o] = 0;
-            }
-    }
-    __syncthreads();
-    int iv_old = 0, iv = 1, iq = 2, iw2 = 0, iw1 = 1;
-    int k = 0;
-    for (; k < A.maxiter; k++) {
-        VT* vo = Vb[iv_old];
-        VT* v = Vb[iv];
-        VT* qv = Vb[iq];
-        // q = S A S v, alpha = (v, q)
-        double a1 = 0.0;
-        for (int p = tid; p < np; p += T) {
-            const int i = p / R;
-            VT y[3] = {0, 0, 0};
-            if (!fx[i]) row_product<R, VT>(A, n0, i, rr_, v, y);
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                qv[3 * (int64_t)p + c] = y[c];
-                a1 += (double)v[3 * (int64_t)p + c] * (double)y[c];
-            }
-        }
-        rhs_sum<R>(a1, sh.red, sh.s1);
-        // q -= alpha v + beta v_old, ||q||^2
-        const VT al = (VT)sh.s1[rr_], be = (VT)sh.mr[rr_].beta;
-        double a2 = 0.0;
-        for (int p = tid; p < np; p += T)
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const int64_t o = 3 * (int64_t)p + c;
-                const VT t = qv[o] - al * v[o] - be * vo[o];
-                qv[o] = t;
-                a2 += (double)t * (double)t;
-            }
-        rhs_sum<R>(a2, sh.red, sh.s2);
-        if (tid < R) {
-            MrRhs& m = sh.mr[tid];
-            m.upd = m.active;
-            if (m.active) {
-                m.alpha = sh.s1[tid];
-                const double bn = sqrt(sh.s2[tid]);
-                const double eps = m.s0 * m.beta;
-                const double d1 = m.c0 * m.beta;
-                const double delta = m.c1 * d1 + m.s1 * m.alpha;
-                const double g1 = -m.s1 * d1 + m.c1 * m.alpha;
-                const double gamma = sqrt(g1 * g1 + bn * bn);
-                const double c = gamma > 0.0 ? g1 / gamma : 1.0, sn = gamma > 0.0 ? bn / gamma : 0.0;
-                m.eps = eps;
-                m.delta = delta;
-                m.gamma = gamma;
-                m.tau = gamma > 0.0 ? c * m.eta : 0.0;
-                m.eta = -sn * m.eta;
-                m.c0 = m.c1;
-                m.s0 = m.s1;
-                m.c1 = c;
-                m.s1 = sn;
-                m.bnext = bn;
-                if (!(gamma > 0.0) || !(bn > 0.0) || fabs(m.eta) <= m.target * m.b1) m.active = 0;
-                if (!(gamma > 0.0)) m.upd = 0;
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            int na = 0;
-            for (int r = 0; r < R; r++) na += sh.mr[r].active;
-            sh.active = na;
-        }
-        // w = (v - eps w'' - delta w') / gamma into w''; y += tau w; v_next = q / beta'
-        {
-            const MrRhs& m = sh.mr[rr_];
-            VT* w2 = Wb[iw2];
-            const VT* w1 = Wb[iw1];
-            if (m.upd) {
-                const VT ig = (VT)(1.0 / m.gamma), ep = (VT)m.eps, de = (VT)m.delta, ta = (VT)m.tau;
-                const VT ib = (VT)(m.bnext > 0.0 ? 1.0 / m.bnext : 0.0);
-                for (int p = tid; p < np; p += T)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        const int64_t o = 3 * (int64_t)p + c;
-                        const VT w = (v[o] - ep * w2[o] - de * w1[o]) * ig;
-                        w2[o] = w;
-                        Y[o] += ta * w;
-                        qv[o] *= ib;
-                    }
-            } else {
-                // a finished right-hand side keeps its vectors: the rotation below
-                // then leaves v_old = v = the last Lanczos vector (finite, unused)
-                for (int p = tid; p < np; p += T)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) qv[3 * (int64_t)p + c] = v[3 * (int64_t)p + c];
-            }
-        }
-        __syncthreads();
-        if (tid < R && sh.mr[tid].upd) sh.mr[tid].beta = sh.mr[tid].bnext;
-        const int t0 = iv_old;
-        iv_old = iv;
-        iv = iq;
-        iq = t0;
-        const int t1 = iw2;
-        iw2 = iw1;
-        iw1 = t1;
-        const int na = sh.active;
-        __syncthreads();
-        if (na == 0) {
-            k++;
-            break;
-        }
-    }
-    return k;
-}
-
-// One CTA per system, taken from an atomic queue.  FP64 outer refinement; the inner
-// solves start in FP32 (precision MSFEM_FP32_IR) and a system whose FP32 step fails to
-// halve a right-hand side's residual has that step undone and continues with FP64
-// inner solves (ill-conditioned cells: FP32 Lanczos vectors lose orthogonality).
-template <int R>
-__global__ void __launch_bounds__(512) k_batch_minres(BatchArgs A, int start64)
-{
-    __shared__ CtaShared<R> sh;
-    __shared__ int s_bad[R];
-    const int tid = threadIdx.x, T = blockDim.x;
-    char* cta_base = reinterpret_cast<char*>(A.work) + (int64_t)blockIdx.x * 6 * A.work_stride * sizeof(double);
-    float* base32 = reinterpret_cast<float*>(cta_base);
-    double* base64 = reinterpret_cast<double*>(cta_base);
-
-    for (;;) {
-        if (tid == 0) sh.q = atomicAdd(A.queue, 1);
-        __syncthreads();
-        const int q = sh.q;
-        __syncthreads();
-        if (q >= A.n_sys) break;
-        const int sys = A.order[q];
-        const int64_t n0 = A.node_off[sys];
-        const int n = (int)(A.node_off[sys + 1] - n0);
-        const int np = n * R;
-        double* X = A.x + n0 * R * 3;
-        const uint8_t* fx = A.fixed + n0;
-        if (tid < R) {
-            sh.mr[tid].fnorm2 = 0.0;
-            sh.rr_prev[tid] = 0.0;
-            s_bad[tid] = 0;
-        }
-        int use64 = start64, last64 = start64;
-        int inner_total = 0, outer = 0;
-        double relmax = 0.0;
-        for (outer = 0;; outer++) {
-            if (use64) residual_pass<R, double>(A, n0, np, fx, X, base64 + A.work_stride, sh);
-            else residual_pass<R, float>(A, n0, np, fx, X, base32 + A.work_stride, sh);
-            if (tid == 0) {
-                // a right-hand side whose last FP32 step did not halve its residual
-                int bad = 0;
-                if (outer > 0 && !last64)
-                    for (int r = 0; r < R; r++) {
-                        s_bad[r] = (sh.s1[r] > 0.25 * sh.rr_prev[r] && sh.rr_prev[r] > 0.0) ? 1 : 0;
-                        bad |= s_bad[r];
-                    }
-                sh.bad = bad;
-            }
-            __syncthreads();
-            if (sh.bad) {
-                // undo those steps (their corrections are still in Y) and recompute in FP64
-                apply_correction<R, float>(A, n0, np, fx, X, base32 + 5 * A.work_stride, -1.0, s_bad);
-                __syncthreads();
-                use64 = 1;
-                last64 = 1;
-                if (tid < R) s_bad[tid] = 0;
-                residual_pass<R, double>(A, n0, np, fx, X, base64 + A.work_stride, sh);
-            }
-            if (tid == 0) {
-                int conv = 1;
-                double rm = 0.0;
-                for (int r = 0; r < R; r++) {
-                    if (outer == 0) sh.mr[r].fnorm2 = sh.s1[r];
-                    const double rel = sh.mr[r].fnorm2 > 0.0 ? sqrt(sh.s1[r] / sh.mr[r].fnorm2) : 0.0;
-                    rm = fmax(rm, rel);
-                    const bool ok = rel <= A.tol;
-                    conv &= ok ? 1 : 0;
-                    sh.rr_prev[r] = sh.s1[r];
-                    MrRhs& m = sh.mr[r];
-                    m.b1 = sqrt(sh.s2[r]);
-                    m.eta = m.b1;
-                    m.beta = 0.0;
-                    m.c0 = m.c1 = 1.0;
-                    m.s0 = m.s1 = 0.0;
-                    // inner target: FP32 stops near its own precision, FP64 aims past the goal
-                    const double need = rel > 0.0 ? A.tol / rel : 1.0;
-                    m.target = use64 ? fmax(1e-15, 0.1 * need) : fmax(1e-5, fmin(0.5, 0.3 * need));
-                    m.active = (!ok && m.b1 > 0.0) ? 1 : 0;
-                    m.upd = 0;
-                }
-                relmax = rm;
-                sh.s1[0] = rm;
-                sh.conv = conv || outer >= A.max_outer;
-            }
-            __syncthreads();
-            relmax = sh.s1[0];
-            if (sh.conv) break;
-            if (use64) inner_total += inner_minres<R, double>(A, n0, np, fx, base64, sh);
-            else inner_total += inner_minres<R, float>(A, n0, np, fx, base32, sh);
-            last64 = use64;
-            if (use64) apply_correction<R, double>(A, n0, np, fx, X, base64 + 5 * A.work_stride, 1.0, nullptr);
-            else apply_correction<R, float>(A, n0, np, fx, X, base32 + 5 * A.work_stride, 1.0, nullptr);
-            __syncthreads();
-        }
-        if (tid == 0) {
-            A.iters[sys] = inner_total;
-            A.outers[sys] = outer;
-            A.rel[sys] = relmax;
-        }
-        __syncthreads();
-    }
-}
-
-// one persistent launch over the first n_limit systems of the queue (largest first)
-template <int R>
-int launch_minres(BatchSys& b, double* d_x, int start64, double tol, int maxiter, int threads, int n_limit)
-{
-    auto kern = k_batch_minres<R>;
-    int dev = 0, sms = 0, per_sm = 0;
-    MSFEM_CK(cudaGetDevice(&dev));
-    MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MSFEM_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0));
-    if (per_sm < 1) per_sm = 1;
-    const int grid = std::min<int64_t>((int64_t)sms * per_sm, std::max(1, n_limit));
-    const int64_t stride = (((int64_t)b.max_nodes * R * 3) + 31) / 32 * 32;
-    const size_t need = (size_t)grid * 6 * stride * sizeof(double);  // room for FP64 vectors
-    if (b.work.n < need) MSFEM_TRY(b.work.alloc(need));
-    MSFEM_TRY(b.queue.alloc(1));
-    MSFEM_CK(cudaMemsetAsync(b.queue.p, 0, sizeof(int), b.stream));
-    BatchArgs a{};
-    a.n_sys = n_limit;
-    a.order = b.order.p;
-    a.node_off = b.node_off.p;
-    a.row_ptr = b.row_ptr.p;
-    a.col = b.col.p;
-    a.val64 = b.val64.p;
-    a.val32 = b.val32.p;
-    a.dscale = b.dscale.p;
-    a.fixed = b.fixed.p;
-    a.x = d_x;
-    a.work = b.work.p;
-    a.work_stride = stride;
-    a.queue = b.queue.p;
-    a.iters = b.iters.p;
-    a.outers = b.outers.p;
-    a.rel = b.rel.p;
-    a.rhs = b.rhs;
-    a.tol = tol;
-    a.maxiter = maxiter;
-    a.max_outer = 30;
-    b.grid = grid;
-    b.threads = threads;
-    b.work_stride = stride;
-    kern<<<grid, threads, 0, b.stream>>>(a, start64);
-    MSFEM_CK(cudaGetLastError());
-    return 0;
 }
 
 }  // namespace
@@ -782,14 +326,13 @@ int batch_build_pattern(BatchSys& b, const double* d_xyz)
     MSFEM_TRY(b.outers.alloc(std::max(1, b.n_sys)));
     MSFEM_TRY(b.rel.alloc(std::max(1, b.n_sys)));
     MSFEM_CK(cudaStreamSynchronize(st));
-    return 0;
+    return b.fixed.p ? batch_build_free(b) : 0;
 }
 
 int batch_assemble_enqueue(BatchSys& b, const double* d_xyz, const double* d_lame, int n_mat)
 {
     cudaStream_t st = b.stream;
     MSFEM_TRY(b.val64.alloc(std::max<int64_t>(1, 9 * b.nnzb)));
-    MSFEM_TRY(b.val32.alloc(std::max<int64_t>(1, 9 * b.nnzb)));
     MSFEM_TRY(b.dscale.alloc(std::max<int64_t>(1, 3 * b.n_nodes)));
     DBuf<int>& flag = b.aflag;
     MSFEM_TRY(flag.alloc(1));
@@ -804,10 +347,8 @@ int batch_assemble_enqueue(BatchSys& b, const double* d_xyz, const double* d_lam
                                                          d_lame, n_mat, b.val64.p, flag.p);
     }
     const int nblk = (int)std::min<int64_t>((b.n_nodes + 255) / 256, 148 * 16);
-    if (b.n_nodes) {
-        k_batch_scale<<<nblk, 256, 0, st>>>(b.n_nodes, b.row_ptr.p, b.col.p, b.val64.p, b.dscale.p);
-        k_batch_val32<<<nblk, 256, 0, st>>>(b.n_nodes, b.row_ptr.p, b.col.p, b.val64.p, b.dscale.p, b.val32.p);
-    }
+    if (b.n_nodes) k_batch_scale<<<nblk, 256, 0, st>>>(b.n_nodes, b.row_ptr.p, b.col.p, b.val64.p, b.dscale.p);
+    b.s64_ok = b.s32_ok = false;
     MSFEM_CK(cudaGetLastError());
     return 0;
 }
@@ -831,109 +372,18 @@ int batch_assemble_given(BatchSys& b, const double* d_eblocks, bool scaled)
     cudaStream_t st = b.stream;
     MSFEM_TRY(b.val64.alloc(std::max<int64_t>(1, 9 * b.nnzb)));
     if (scaled) {
-        MSFEM_TRY(b.val32.alloc(std::max<int64_t>(1, 9 * b.nnzb)));
         MSFEM_TRY(b.dscale.alloc(std::max<int64_t>(1, 3 * b.n_nodes)));
     }
     const int blocks = (int)std::min<int64_t>((b.nnzb + 255) / 256, 148 * 16);
     if (b.nnzb)
         k_assemble_given<<<blocks, 256, 0, st>>>(b.nnzb, b.cstart.p, b.contrib.p, b.k1, d_eblocks, b.val64.p);
     const int nblk = (int)std::min<int64_t>((b.n_nodes + 255) / 256, 148 * 16);
-    if (scaled && b.n_nodes) {
+    if (scaled && b.n_nodes)
         k_batch_scale<<<nblk, 256, 0, st>>>(b.n_nodes, b.row_ptr.p, b.col.p, b.val64.p, b.dscale.p);
-        k_batch_val32<<<nblk, 256, 0, st>>>(b.n_nodes, b.row_ptr.p, b.col.p, b.val64.p, b.dscale.p, b.val32.p);
-    }
+    b.s64_ok = b.s32_ok = false;
     MSFEM_CK(cudaGetLastError());
     MSFEM_CK(cudaStreamSynchronize(st));
     return 0;
-}
-
-namespace {
-
-int launch_any(BatchSys& b, double* d_x, int start64, double tol, int maxiter, int threads, int n_limit)
-{
-    switch (b.R) {
-    case 4: return launch_minres<4>(b, d_x, start64, tol, maxiter, threads, n_limit);
-    case 8: return launch_minres<8>(b, d_x, start64, tol, maxiter, threads, n_limit);
-    case 1: return launch_minres<1>(b, d_x, start64, tol, maxiter, threads, n_limit);
-    default:
-        set_error("batched solve: %d right-hand sides per system (1, 4 or 8 supported)", b.R);
-        return MSFEM_ERR_ARGUMENT;
-    }
-}
-
-// Autotuner of the persistent launch: the CTA size (threads per system) decides how many
-// row-rhs pairs a pass covers and how many CTAs fit per SM.  Each candidate solves the same
-// sample -- the 2 x #SM largest systems, which dominate the batch's time -- from the same start
-// (x is saved and restored around each trial), timed with CUDA events; the fastest is kept for
-// this batch.  Batches smaller than the sample are not timed (the choice hardly matters there).
-int autotune(BatchSys& b, double* d_x, int start64, double tol, int maxiter)
-{
-    int dev = 0, sms = 0;
-    MSFEM_CK(cudaGetDevice(&dev));
-    MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int sample = 2 * sms;
-    b.tune_ms.clear();
-    if (b.n_sys < 2 * sample) {
-        b.tuned_threads = 256;
-        return 0;
-    }
-    const size_t nx = (size_t)b.n_nodes * b.R * 3;
-    DBuf<double> save;
-    MSFEM_TRY(save.alloc(nx));
-    MSFEM_CK(cudaMemcpyAsync(save.p, d_x, sizeof(double) * nx, cudaMemcpyDeviceToDevice, b.stream));
-    cudaEvent_t e0, e1;
-    MSFEM_CK(cudaEventCreate(&e0));
-    MSFEM_CK(cudaEventCreate(&e1));
-    const int cand[] = {128, 256, 384, 512};
-    float best = 0.f;
-    int best_t = 256;
-    for (int t : cand) {
-        MSFEM_CK(cudaMemcpyAsync(d_x, save.p, sizeof(double) * nx, cudaMemcpyDeviceToDevice, b.stream));
-        MSFEM_CK(cudaEventRecord(e0, b.stream));
-        MSFEM_TRY(launch_any(b, d_x, start64, tol, maxiter, t, sample));
-        MSFEM_CK(cudaEventRecord(e1, b.stream));
-        MSFEM_CK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        MSFEM_CK(cudaEventElapsedTime(&ms, e0, e1));
-        b.tune_ms.push_back(ms);
-        if (b.tune_ms.size() == 1 || ms < best) {
-            best = ms;
-            best_t = t;
-        }
-    }
-    MSFEM_CK(cudaMemcpyAsync(d_x, save.p, sizeof(double) * nx, cudaMemcpyDeviceToDevice, b.stream));
-    MSFEM_CK(cudaStreamSynchronize(b.stream));
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    b.tuned_threads = best_t;
-    return 0;
-}
-
-}  // namespace
-
-int batch_threads(const BatchSys& b, int precision, int threads)
-{
-    if (b.n_sys == 0) return 256;
-    if (threads > 0) return threads;
-    return (b.tuned_threads != 0 && b.tuned_precision == precision) ? b.tuned_threads : 0;
-}
-
-int batch_solve(BatchSys& b, double* d_x, int precision, double tol, int maxiter, int threads)
-{
-    if (b.n_sys == 0) return 0;
-    const int start64 = precision == MSFEM_FP32_IR ? 0 : 1;
-    if (threads <= 0) {
-        if (b.tuned_threads == 0 || b.tuned_precision != precision) {
-            MSFEM_TRY(autotune(b, d_x, start64, tol, maxiter));
-            b.tuned_precision = precision;
-        }
-        threads = b.tuned_threads;
-    }
-    if (threads % 32 != 0 || threads > 512) {
-        set_error("batched solve: threads per system must be a multiple of 32, at most 512");
-        return MSFEM_ERR_ARGUMENT;
-    }
-    return launch_any(b, d_x, start64, tol, maxiter, threads, b.n_sys);
 }
 
 }  // namespace msfem

@@ -33,20 +33,30 @@ struct BatchSys {
     DBuf<int32_t> col;       // [nnzb]
     DBuf<uint32_t> contrib;  // [n_pairs] element << 4 | I << 2 | J, grouped by block, element order
     DBuf<double> val64;      // [9 * nnzb] A[a][b] of each block, row-major
-    DBuf<float> val32;       // [9 * nnzb] s_a A[a][b] s_b (Jacobi scaled)
     DBuf<double> dscale;     // [3 * n_nodes] 1 / sqrt(diagonal)
     DBuf<int32_t> order;     // systems, largest first (the persistent solver's queue)
 
+    // the free block S A_II S in slices of G rows (batch_minres.cu): rows and columns are the system's
+    // free nodes; entry (slice s, position k, row g) has its column at (slice_ptr[s] + k) * G + g and
+    // its 9 values at ((slice_ptr[s] + k) * 9 + e) * G + g; shorter rows end in zero blocks
+    int64_t n_slices = 0, n_entries = 0;
+    int max_slices = 0;        // slices of the largest system
+    DBuf<int64_t> slice_off;   // [n_sys + 1]
+    DBuf<int64_t> slice_ptr;   // [n_slices + 1]
+    DBuf<int32_t> free_node;   // [n_slices * G] node of each free row, -1 past a system's last
+    DBuf<int32_t> lid;         // [n_nodes] free row of a node within its system, -1: Dirichlet
+    DBuf<int32_t> scol;
+    DBuf<double> s64;
+    DBuf<float> s32;
+    bool s64_ok = false, s32_ok = false;  // they hold the current values
+
     // solver scratch and per-system report
-    DBuf<unsigned char> work;  // per-CTA Krylov vectors (bytes: room for FP64)
+    DBuf<unsigned char> work;  // Krylov vectors of each cluster (bytes: room for FP64)
     DBuf<int> queue;
     DBuf<int32_t> iters, outers;
     DBuf<double> rel;
     const double* rhs = nullptr;  // optional source term [n_nodes][R][3] (device), used by batch_solve
-    int grid = 0, threads = 0;
-    int tuned_threads = 0, tuned_precision = -1;  // autotuned CTA size (0: not tuned yet)
-    std::vector<float> tune_ms;                   // trial times of the candidates 128/256/384/512
-    int64_t work_stride = 0;
+    int threads = 0;  // CTA size of the last solve
     float last_ms = 0.f;
     DBuf<int> aflag;  // set by the assembly when an element's material id is out of range
 };
@@ -59,14 +69,17 @@ int batch_assemble(BatchSys& b, const double* d_xyz, const double* d_lame, int n
 // buffers exist): capturable into a CUDA graph; a bad material id is left in b.aflag
 int batch_assemble_enqueue(BatchSys& b, const double* d_xyz, const double* d_lame, int n_mat);
 // values from caller-given element blocks [n_elems][k1][k1][9] (device), each block the sum of
-// its element contributions in element order; scaled: also the Jacobi scale and the FP32 copy
-// the batched solver reads
+// its element contributions in element order; scaled: also the Jacobi scale the
+// batched solver reads
 int batch_assemble_given(BatchSys& b, const double* d_eblocks, bool scaled = true);
+// the free block's pattern (batch_build_pattern calls it when the fixed nodes are known)
+int batch_build_free(BatchSys& b);
 // solves every system; x: [n_nodes][R][3] FP64, fixed entries hold the Dirichlet data on
 // entry, free entries are overwritten.  precision: MSFEM_FP64 or MSFEM_FP32_IR.  threads <= 0:
-// the CTA size is autotuned on the first call (cached per batch and precision).
+// the CTA size is chosen from the batch's sizes.  No host synchronisation, and no allocation from
+// the second call with the same precision on: capturable into a CUDA graph.
 int batch_solve(BatchSys& b, double* d_x, int precision, double tol, int maxiter, int threads);
-// the CTA size batch_solve would use with `threads` (0 when the autotuner has not run yet)
-int batch_threads(const BatchSys& b, int precision, int threads);
+// the CTA size batch_solve uses with `threads`
+int batch_threads(const BatchSys& b, int threads);
 
 }  // namespace msfem

@@ -980,8 +980,7 @@ int set_face_materials(CellsHandle& h, int mode)
 
 // The launches of one stage of the Order1 build: 0 both assemblies, 1 the closed-form edges and
 // the face problems' Dirichlet data, 2 the face batch, 3 the volume problems' Dirichlet data and
-// the volume batch.  `tf` / `tv`: the face / volume CTA sizes (0: batch_solve autotunes, which
-// synchronises).
+// the volume batch.  `tf` / `tv`: the face / volume CTA sizes.
 int cells_stage(CellsHandle& h, int stage, int precision, double tol, int maxiter, int tf, int tv)
 {
     cudaStream_t st = h.stream;
@@ -1022,12 +1021,17 @@ int cells_build(CellsHandle& h, int precision, double tol, int maxiter, int thre
     BatchSys& F = h.faces;
     BatchSys& V = h.vols;
     h.vols_assembled = true;
-    const int tf = batch_threads(F, precision, threads), tv = batch_threads(V, precision, threads);
+    const int tf = batch_threads(F, threads), tv = batch_threads(V, threads);
     const double key[5] = {(double)precision, tol, (double)maxiter, (double)tf, (double)tv};
+    if (h.build_graph[0] && (h.build_work[0] != F.work.p || h.build_work[1] != V.work.p))
+        for (auto& g : h.build_graph) {  // a call with other settings moved the solver's workspace
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
     const bool have_graph = h.build_graph[0] && std::memcmp(key, h.build_key, sizeof(key)) == 0;
     // capture only a build whose launches have run once with this key: every buffer is then
-    // allocated and the CTA sizes tuned, so the capture holds launches and copies only
-    const bool can_capture = tf > 0 && tv > 0 && std::memcmp(key, h.eager_key, sizeof(key)) == 0;
+    // allocated, so the capture holds launches and copies only
+    const bool can_capture = std::memcmp(key, h.eager_key, sizeof(key)) == 0;
     if (have_graph || can_capture) {
         if (!have_graph) {
             for (auto& g : h.build_graph)
@@ -1054,24 +1058,26 @@ int cells_build(CellsHandle& h, int precision, double tol, int maxiter, int thre
                 }
             }
             std::memcpy(h.build_key, key, sizeof(key));
+            h.build_work[0] = F.work.p;
+            h.build_work[1] = V.work.p;
         }
         for (int k = 0; k < 4; k++) {
             MSFEM_CK(cudaEventRecord(h.ev[k], st));
             MSFEM_CK(cudaGraphLaunch(h.build_graph[k], st));
         }
         MSFEM_CK(cudaEventRecord(h.ev[4], st));
+        // the stages assembled the values again and filled the solver's copies in their precision
+        F.s64_ok = V.s64_ok = true;
+        F.s32_ok = V.s32_ok = precision == MSFEM_FP32_IR;
         h.graph_builds++;
     } else {
-        // launch by launch (the first build tunes the persistent launches' CTA sizes, which
-        // synchronises); the next build with the same key is captured
+        // launch by launch; the next build with the same key is captured
         for (int k = 0; k < 4; k++) {
             MSFEM_CK(cudaEventRecord(h.ev[k], st));
             MSFEM_TRY(cells_stage(h, k, precision, tol, maxiter, tf, tv));
         }
         MSFEM_CK(cudaEventRecord(h.ev[4], st));
-        const double k2[5] = {(double)precision, tol, (double)maxiter, (double)batch_threads(F, precision, threads),
-                              (double)batch_threads(V, precision, threads)};
-        std::memcpy(h.eager_key, k2, sizeof(k2));
+        std::memcpy(h.eager_key, key, sizeof(key));
     }
     MSFEM_CK(cudaStreamSynchronize(st));
     for (int k = 0; k < 4; k++) MSFEM_CK(cudaEventElapsedTime(&h.ms[k], h.ev[k], h.ev[k + 1]));

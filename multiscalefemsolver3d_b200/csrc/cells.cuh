@@ -60,6 +60,7 @@ struct CellsHandle {
     // recorded between the graphs
     cudaGraphExec_t build_graph[4] = {nullptr, nullptr, nullptr, nullptr};  // one per stage
     double build_key[5] = {0, 0, 0, 0, 0};
+    const void* build_work[2] = {nullptr, nullptr};  // the solver workspaces the graphs use
     double eager_key[5] = {-1, 0, 0, 0, 0};  // key of the last build run launch by launch
     int graph_builds = 0;  // builds run by replaying the graph
     ~CellsHandle()
