@@ -5,15 +5,16 @@
 // restarted GMRES(M) with Givens rotations and a back substitution.  This is
 // that method laid out for the GPU:
 //   * Arnoldi with classical Gram-Schmidt applied twice (CGS2): the j+1
-//     projections of a step are computed together by one multi-dot kernel and
-//     removed by one update kernel, instead of 2(j+1) dependent passes;
+//     projections of a step are computed together and removed together,
+//     instead of 2(j+1) dependent passes;
 //   * the Hessenberg column, its Givens rotations and the residual estimate
-//     |g_{j+1}| are updated on the device by a one-thread kernel, so a whole
-//     restart cycle (m steps) is one captured CUDA graph with no host wait;
+//     |g_{j+1}| are updated on the device: the host waits once per solve;
 //   * x += M^-1 V y is one fused pass after the cycle.
 // Stopping test: |g_{j+1}| <= tol * ||F|| (the true residual norm in exact
 // arithmetic for right preconditioning).
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "devutil.cuh"
 #include "internal.cuh"
@@ -22,242 +23,348 @@
 namespace msfem {
 namespace {
 
-// layout of the small dense GMRES data in System::gm (doubles)
-struct GmLayout {
-    int m;
-    __host__ __device__ size_t H() const { return 0; }                           // (m+1) x m, row-major H[i*m + j]
-    __host__ __device__ size_t cs() const { return (size_t)(m + 1) * m; }        // m
-    __host__ __device__ size_t sn() const { return cs() + m; }                   // m
-    __host__ __device__ size_t g() const { return sn() + m; }                    // m+1
-    __host__ __device__ size_t y() const { return g() + m + 1; }                 // m
-    __host__ __device__ size_t h1() const { return y() + m; }                    // m+1 (first projection)
-    __host__ __device__ size_t h2() const { return h1() + m + 1; }               // m+1 (second projection)
-    __host__ __device__ size_t misc() const { return h2() + m + 1; }             // [0] steps done this cycle, [1] converged, [2] |g|
-    __host__ __device__ size_t total() const { return misc() + 8; }
+// One cooperative launch runs the whole solve -- every Arnoldi step, restart and residual.  CTA c owns
+// a contiguous range of matrix slices and keeps its rows of the work vector (and, where they fit, of
+// every basis vector) in shared memory, so an Arnoldi step reads the matrix and the gathered vector;
+// its three reductions (the two Gram-Schmidt projections and the norm) are grid barriers.  Every CTA
+// keeps the rotations and the residual estimate itself, from the same sums in the same order; CTA 0
+// keeps the Hessenberg matrix.  The launch-per-kernel cycle this replaces was bound by its launches
+// and by the last block's serial reduction of j + 1 sums: with restart 50 an Arnoldi step took 134 us
+// at 72,522 unknowns, 160 us at 282,962 and 306 us at 949,567 (FP32 basis); here 20, 47 and 179 us.
+// With the basis in global memory 1024 threads beat 512 (47 against 55 us at 282,962 unknowns, FP64 56
+// against 89): more loads in flight per SM; in shared memory 512 leave room for the basis.
+
+struct GmCoop {
+    int n, m, maxiter, rows;  // rows: capacity of a CTA (slices * 32 * bs)
+    double tol;
+    const double* dinv;       // right preconditioner diag(A)^-1, or null
+    void* x;                  // solution, VT
+    const void* b;            // right-hand side, VT
+    int zero_start;           // x = 0 on entry
+    void* gather[2];          // [n] each, VT
+    double* partial;          // [2 m + 4][gridDim.x]
+    void* V;                  // [m + 1][n] basis, VT, when the CTAs' shares do not fit shared memory
+    double* w;                // [n] work vector, when it does not fit either
+    double* H;                // [m (m + 1) / 2] packed upper triangle, column j at j (j + 1) / 2
+    double* y;                // [m]
+    double* out;              // [0] iterations, [1] cycles, [2] |g|^2 at the end, [3] done, [4] ||b||^2
+    GridBar* bar;
 };
 
-// V0 = r / ||r|| (r and V0 may be the same vector), g = (||r||, 0, ...)
-template <class VT>
-__global__ void k_gm_start(int n, const VT* r, VT* V0, double* gm, GmLayout L,
-                           const KState* S)
+// sums of `count` values over the grid: the CTA's value q (written by the caller into vals[q],
+// shared) -> sums[q] (shared), the CTAs added in index order by lanes and a butterfly
+__device__ __forceinline__ bool grid_sums(GridSync& gs, double* partial, const double* vals, double* sums, int count)
 {
-    const double beta = sqrt(S->rr);
-    const double inv = beta > 0 ? 1.0 / beta : 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        V0[i] = (VT)((double)r[i] * inv);
-    if (blockIdx.x == 0) {
-        for (int i = threadIdx.x; i < L.m + 1; i += blockDim.x) gm[L.g() + i] = (i == 0) ? beta : 0.0;
-        if (threadIdx.x == 0) {
-            gm[L.misc()] = 0.0;
-            gm[L.misc() + 1] = 0.0;
-            gm[L.misc() + 2] = beta;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, G = gridDim.x;
+    __syncthreads();
+    for (int q = threadIdx.x; q < count; q += blockDim.x) partial[(size_t)q * G + blockIdx.x] = vals[q];
+    if (!gs.sync()) return false;
+    for (int q = warp; q < count; q += nw) {
+        const double* p = partial + (size_t)q * G;
+        double a[5], t = 0.0;  // 160 CTAs per round of loads: one round on 148 SMs
+        for (int c0 = 0; c0 < G; c0 += 160) {
+#pragma unroll
+            for (int u = 0; u < 5; u++) a[u] = c0 + 32 * u + lane < G ? __ldcg(p + c0 + 32 * u + lane) : 0.0;
+            t += ((a[0] + a[1]) + (a[2] + a[3])) + a[4];
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sums[q] = t;
     }
+    __syncthreads();
+    return true;
 }
 
-// z = M^-1 v (dinv == nullptr: the matrix is already Jacobi-scaled, z = v)
-template <class VT>
-__global__ void k_gm_prec(int n, const VT* __restrict__ v, const double* __restrict__ dinv, VT* __restrict__ z,
-                          const double* gm, GmLayout L)
+// VS: the basis rows are in shared memory
+template <class VT, bool VS>
+__global__ void __launch_bounds__(VS ? 512 : 1024) k_gm_coop(SellView<VT> A, GmCoop P)
 {
-    if (gm[L.misc() + 1] != 0.0) return;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        z[i] = dinv ? (VT)((double)v[i] * dinv[i]) : v[i];
-}
-
-template <class VT>
-__global__ void __launch_bounds__(256) k_gm_spmv(SellView<VT> A, const VT* __restrict__ z, VT* __restrict__ w,
-                                                 const double* gm, GmLayout L)
-{
-    if (gm[L.misc() + 1] != 0.0) return;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= A.n_slices) return;
-    if (A.bs == 1) {
-        const VT v = sell_row_scalar<VT>(A, warp, lane, z);
-        const int row = warp * kSlice + lane;
-        if (row < A.n_rows) w[row] = v;
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ int s_ok;
+    __shared__ double s_warp[32], s_one[1], s_norm[1];
+    __shared__ double s_state[4];  // [0] |g_{j+1}|, [1] stop code
+    const int m = P.m, tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
+    // shared memory: FP64 small arrays, then the basis rows and the work rows
+    double* h1 = reinterpret_cast<double*>(sm);  // own partial dots
+    double* h2 = h1 + m + 1;                     // summed: first projection
+    double* h3 = h2 + m + 1;                     // summed: second projection
+    double* cs = h3 + m + 1;
+    double* sn = cs + m;
+    double* g = sn + m;
+    double* y = g + m + 1;
+    double* w = P.w;                             // the work vector, holding values rounded to VT
+    VT* V = (VT*)P.V;
+    int64_t ldv = P.n;
+    GridSync gs(P.bar, &s_ok);
+    const int G = gridDim.x;
+    const int s0 = (int)((int64_t)A.n_slices * blockIdx.x / G), s1 = (int)((int64_t)A.n_slices * (blockIdx.x + 1) / G);
+    const int row0 = s0 * kSlice * A.bs;
+    const int nr = min((s1 - s0) * kSlice * A.bs, max(0, P.n - row0));  // this CTA's rows
+    if (VS) {
+        V = reinterpret_cast<VT*>(y + m + P.rows);
+        ldv = P.rows;
     } else {
-        VT v[3];
-        sell_row_block<VT>(A, warp, lane, z, v);
-        const int brow = warp * kSlice + lane;
-        if (brow < A.n_brows)
-            for (int c = 0; c < 3; c++) w[3 * (int64_t)brow + c] = v[c];
+        V += row0;
     }
-}
+    if (w) w += row0;
+    else w = y + m;
+    VT* x = reinterpret_cast<VT*>(P.x);
+    const VT* b = reinterpret_cast<const VT*>(P.b);
 
-// h[i] = (V_i, w), i = 0..j (FP64 accumulation for either vector type)
-template <class VT>
-__global__ void __launch_bounds__(kVecThreads) k_gm_multidot(int n, const VT* __restrict__ V, int j,
-                                                             const VT* __restrict__ w, double* __restrict__ partial,
-                                                             unsigned int* ticket, double* gm, GmLayout L, size_t hoff)
-{
-    if (gm[L.misc() + 1] != 0.0) return;
-    __shared__ double sh[32];
-    for (int i = 0; i <= j; i++) {
-        const VT* vi = V + (size_t)i * n;
-        double acc[1] = {0.0};
-        for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-            acc[0] += (double)vi[r] * (double)w[r];
-        block_sum<1>(acc, sh);
-        if (threadIdx.x == 0) partial[(size_t)i * gridDim.x + blockIdx.x] = acc[0];
-    }
-    if (arrive_last(ticket)) {
-        for (int i = 0; i <= j; i++) {
-            double t[1];
-            reduce_partials<1>(partial + (size_t)i * gridDim.x, gridDim.x, 0, t, sh);
-            if (threadIdx.x == 0) gm[hoff + i] = t[0];
+    // w = scale * A v on the CTA's rows
+    auto product = [&](const VT* v, double scale) {
+        for (int sl = s0 + warp; sl < s1; sl += nw) {
+            const int lr = (sl - s0) * kSlice * A.bs + lane * A.bs;
+            if (A.bs == 1) {
+                const VT t = sell_row_scalar<VT, true>(A, sl, lane, v);
+                if (lr < nr) w[lr] = (double)(VT)(t * (VT)scale);
+            } else {
+                VT t[3];
+                sell_row_block<VT, true>(A, sl, lane, v, t);
+                if (lr < nr)
+                    for (int c = 0; c < 3; c++) w[lr + c] = (double)(VT)(t[c] * (VT)scale);
+            }
         }
-        if (threadIdx.x == 0) *ticket = 0;
-    }
-}
-
-// w -= sum_i h[i] V_i ; with LAST, also (w, w) -> the new subdiagonal entry, and H[:, j] = h1 + h2
-template <class VT, bool LAST>
-__global__ void __launch_bounds__(kVecThreads) k_gm_orth(int n, const VT* __restrict__ V, int j,
-                                                         VT* __restrict__ w, double* __restrict__ partial,
-                                                         unsigned int* ticket, double* gm, GmLayout L, size_t hoff)
-{
-    if (gm[L.misc() + 1] != 0.0) return;
-    __shared__ double sh[32];
-    __shared__ double hs[1024];
-    for (int i = threadIdx.x; i <= j; i += blockDim.x) hs[i] = gm[hoff + i];
-    __syncthreads();
-    double acc[1] = {0.0};
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        double t = (double)w[r];
-        for (int i = 0; i <= j; i++) t -= hs[i] * (double)V[(size_t)i * n + r];
-        w[r] = (VT)t;
-        const double tv = (double)w[r];
-        acc[0] += tv * tv;
-    }
-    if (!LAST) return;
-    block_sum<1>(acc, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc[0];
-    if (arrive_last(ticket)) {
-        double t[1];
-        reduce_partials<1>(partial, gridDim.x, 0, t, sh);
-        if (threadIdx.x == 0) {
-            const int m = L.m;
-            for (int i = 0; i <= j; i++) gm[L.H() + (size_t)i * m + j] = gm[L.h1() + i] + gm[L.h2() + i];
-            gm[L.H() + (size_t)(j + 1) * m + j] = sqrt(t[0]);
-            *ticket = 0;
-        }
-    }
-}
-
-// Givens update of column j, residual estimate and stopping test (one thread).
-__global__ void k_gm_givens(int j, double* gm, GmLayout L, KState* S)
-{
-    if (gm[L.misc() + 1] != 0.0) return;
-    const int m = L.m;
-    double* H = gm + L.H();
-    double* cs = gm + L.cs();
-    double* sn = gm + L.sn();
-    double* g = gm + L.g();
-    const double hn = H[(size_t)(j + 1) * m + j];
-    for (int i = 0; i < j; i++) {
-        const double a = H[(size_t)i * m + j], b = H[(size_t)(i + 1) * m + j];
-        H[(size_t)i * m + j] = cs[i] * a + sn[i] * b;
-        H[(size_t)(i + 1) * m + j] = -sn[i] * a + cs[i] * b;
-    }
-    const double a = H[(size_t)j * m + j], b = H[(size_t)(j + 1) * m + j];
-    const double d = sqrt(a * a + b * b);
-    const double c = d > 0 ? a / d : 1.0, s = d > 0 ? b / d : 0.0;
-    cs[j] = c;
-    sn[j] = s;
-    H[(size_t)j * m + j] = d;
-    H[(size_t)(j + 1) * m + j] = 0.0;
-    g[j + 1] = -s * g[j];
-    g[j] = c * g[j];
-    const double res = fabs(g[j + 1]);
-    gm[L.misc()] = j + 1;
-    gm[L.misc() + 2] = res;
-    S->iter += 1;
-    S->rr = res * res;
-    if (res * res <= S->tol2 || !(res == res)) {
-        gm[L.misc() + 1] = 1.0;
-        S->done = 1;
-    } else if (hn == 0.0 || d == 0.0) {
-        gm[L.misc() + 1] = 2.0;  // happy breakdown: the cycle's space holds the solution
-    } else if (S->iter >= S->maxiter) {
-        gm[L.misc() + 1] = 3.0;
-        S->done = 2;
-    }
-}
-
-// V_{j+1} = w / ||w||
-template <class VT>
-__global__ void k_gm_normalize(int n, const VT* __restrict__ w, VT* __restrict__ vnext, int j, const double* gm,
-                               GmLayout L)
-{
-    if (gm[L.misc() + 1] != 0.0) return;
-    // ||w|| was saved before the Givens step rotated H[j+1][j] to zero
-    const double norm = gm[L.misc() + 3];
-    const double inv = norm > 0 ? 1.0 / norm : 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        vnext[i] = (VT)((double)w[i] * inv);
-}
-
-// save ||w|| before the rotation overwrites H[j+1][j]
-__global__ void k_gm_save_norm(int j, double* gm, GmLayout L)
-{
-    if (gm[L.misc() + 1] != 0.0) return;
-    gm[L.misc() + 3] = gm[L.H() + (size_t)(j + 1) * L.m + j];
-}
-
-// y = R^{-1} g over the completed steps (one thread), then x += M^{-1} V y
-__global__ void k_gm_backsolve(double* gm, GmLayout L)
-{
-    const int m = L.m;
-    const int k = (int)gm[L.misc()];
-    const double* H = gm + L.H();
-    const double* g = gm + L.g();
-    double* y = gm + L.y();
-    for (int i = k - 1; i >= 0; i--) {
-        double s = g[i];
-        for (int l = i + 1; l < k; l++) s -= H[(size_t)i * m + l] * y[l];
-        const double d = H[(size_t)i * m + i];
-        y[i] = d != 0.0 ? s / d : 0.0;
-    }
-}
-
-template <class VT>
-__global__ void __launch_bounds__(kVecThreads) k_gm_update(int n, VT* __restrict__ x, const VT* __restrict__ V,
-                                                           const double* __restrict__ dinv, const double* gm, GmLayout L)
-{
-    __shared__ double ys[1024];
-    const int k = (int)gm[L.misc()];
-    for (int i = threadIdx.x; i < k; i += blockDim.x) ys[i] = gm[L.y() + i];
-    __syncthreads();
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+        __syncthreads();
+    };
+    // (w, w) over the grid into s_norm[0]
+    auto norm2 = [&](double* part) -> bool {
         double t = 0.0;
-        for (int i = 0; i < k; i++) t += ys[i] * (double)V[(size_t)i * n + r];
-        x[r] = (VT)((double)x[r] + (dinv ? dinv[r] : 1.0) * t);
+        for (int r = tid; r < nr; r += T) t += w[r] * w[r];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) s_warp[warp] = t;
+        __syncthreads();
+        if (tid == 0) {
+            double u = 0.0;
+            for (int k = 0; k < nw; k++) u += s_warp[k];
+            s_one[0] = u;
+        }
+        return grid_sums(gs, part, s_one, s_norm, 1);
+    };
+    // the vector the next product gathers: w, through the right preconditioner
+    auto publish = [&](VT* to) {
+        for (int r = tid; r < nr; r += T)
+            to[row0 + r] = (VT)(P.dinv ? w[r] * P.dinv[row0 + r] : w[r]);
+    };
+    // h1[i] (+)= (V_i, w) on the CTA's rows [r0, r1), one vector per warp at a time
+    auto dots = [&](int j, int r0, int r1, bool add) {
+        for (int i = warp; i <= j; i += nw) {
+            const VT* v = V + i * ldv;
+            double t[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int r = r0 + lane; r < r1; r += 128)
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (r + 32 * u < r1) t[u] += (double)v[r + 32 * u] * w[r + 32 * u];
+            double q = (t[0] + t[1]) + (t[2] + t[3]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+            if (lane == 0) h1[i] = add ? h1[i] + q : q;
+        }
+    };
+    // w -= sum_i h[i] V_i; with `again`, h1 = the projections of the new w, tile by tile of rows, so
+    // that the second read of the basis finds the tile in the L1
+    auto remove = [&](const double* h, int j, bool again) {
+        for (int r0 = 0; r0 < nr; r0 += T) {
+            const int r = r0 + tid;
+            if (r < nr) {
+                double t[4] = {w[r], 0.0, 0.0, 0.0};
+                int i = 0;
+                for (; i + 3 <= j; i += 4)
+#pragma unroll
+                    for (int u = 0; u < 4; u++) t[u] -= h[i + u] * (double)V[(i + u) * ldv + r];
+                for (; i <= j; i++) t[0] -= h[i] * (double)V[i * ldv + r];
+                w[r] = (double)(VT)((t[0] + t[1]) + (t[2] + t[3]));
+            }
+            if (again) {
+                __syncthreads();
+                dots(j, r0, min(r0 + T, nr), r0 > 0);
+            }
+        }
+        if (again && nr == 0)
+            for (int i = tid; i <= j; i += T) h1[i] = 0.0;
+        __syncthreads();
+    };
+
+    double* part1 = P.partial;
+    double* part2 = part1 + (size_t)(m + 1) * G;
+    double* part3 = part2 + (size_t)(m + 1) * G;
+    double* part4 = part3 + G;
+    int iter = 0, cycles = 0, done = 0;
+    for (int r = tid; r < nr; r += T) w[r] = b[row0 + r];
+    __syncthreads();
+    if (!norm2(part4)) return;
+    const double bb = s_norm[0], tol2 = P.tol * P.tol * bb;
+    double res2 = bb;
+    bool zero = P.zero_start != 0;
+    for (;;) {
+        // r = b - A x, its norm
+        __syncthreads();
+        if (!zero) {  // else w holds b
+            product(x, 1.0);
+            for (int r = tid; r < nr; r += T) w[r] = (double)(VT)((double)b[row0 + r] - w[r]);
+        }
+        zero = false;
+        __syncthreads();
+        publish((VT*)P.gather[0]);
+        if (!norm2(part3)) return;
+        res2 = s_norm[0];
+        if (res2 <= tol2 || done || iter >= P.maxiter || !(res2 == res2)) break;
+        cycles++;
+        double norm = sqrt(res2);
+        for (int i = tid; i <= m; i += T) g[i] = i == 0 ? norm : 0.0;
+        if (tid == 0) s_state[1] = 0.0;
+        int k = 0;
+        for (int j = 0; j < m; j++) {
+            const double inv = norm > 0.0 ? 1.0 / norm : 0.0;
+            for (int r = tid; r < nr; r += T) V[j * ldv + r] = (VT)(w[r] * inv);
+            __syncthreads();
+            product((const VT*)P.gather[j & 1], inv);
+            dots(j, 0, nr, false);
+            if (!grid_sums(gs, part1, h1, h2, j + 1)) return;
+            remove(h2, j, true);
+            if (!grid_sums(gs, part2, h1, h3, j + 1)) return;
+            remove(h3, j, false);
+            publish((VT*)P.gather[(j + 1) & 1]);
+            if (!norm2(part3)) return;
+            norm = sqrt(s_norm[0]);
+            if (tid == 0) {
+                double* Hj = P.H + (size_t)j * (j + 1) / 2;
+                const bool keep = blockIdx.x == 0;
+                double a = h2[0] + h3[0];
+                for (int i = 0; i < j; i++) {
+                    const double nx = h2[i + 1] + h3[i + 1];
+                    if (keep) Hj[i] = cs[i] * a + sn[i] * nx;
+                    a = -sn[i] * a + cs[i] * nx;
+                }
+                const double d = sqrt(a * a + norm * norm);
+                const double c = d > 0 ? a / d : 1.0, s = d > 0 ? norm / d : 0.0;
+                cs[j] = c;
+                sn[j] = s;
+                if (keep) Hj[j] = d;
+                g[j + 1] = -s * g[j];
+                g[j] = c * g[j];
+                const double res = fabs(g[j + 1]);
+                double code = 0.0;
+                if (res * res <= tol2 || !(res == res)) code = 1.0;
+                else if (norm == 0.0 || d == 0.0) code = 2.0;  // the cycle's space holds the solution
+                else if (iter + 1 >= P.maxiter) code = 3.0;
+                s_state[0] = res * res;
+                s_state[1] = code;
+            }
+            __syncthreads();
+            iter++;
+            k = j + 1;
+            if (s_state[1] != 0.0) break;
+        }
+        res2 = s_state[0];
+        if (s_state[1] == 1.0) done = 1;
+        else if (s_state[1] == 3.0) done = 2;
+        // y = R^-1 g, column by column (warp 0 of CTA 0), then x += M^-1 V y on the CTA's rows
+        if (blockIdx.x == 0 && warp == 0) {
+            for (int i = lane; i < k; i += 32) y[i] = g[i];
+            __syncwarp();
+            for (int i = k - 1; i >= 0; i--) {
+                const double* Hi = P.H + (size_t)i * (i + 1) / 2;
+                const double yi = Hi[i] != 0.0 ? y[i] / Hi[i] : 0.0;
+                __syncwarp();
+                for (int l = lane; l < i; l += 32) y[l] -= Hi[l] * yi;
+                if (lane == 0) y[i] = yi;
+                __syncwarp();
+            }
+            for (int i = lane; i < k; i += 32) P.y[i] = y[i];
+        }
+        if (!gs.sync()) return;
+        for (int i = tid; i < k; i += T) y[i] = __ldcg(P.y + i);
+        __syncthreads();
+        for (int r = tid; r < nr; r += T) {
+            double t[4] = {0.0, 0.0, 0.0, 0.0};
+            int i = 0;
+            for (; i + 3 < k; i += 4)
+#pragma unroll
+                for (int u = 0; u < 4; u++) t[u] += y[i + u] * (double)V[(i + u) * ldv + r];
+            for (; i < k; i++) t[0] += y[i] * (double)V[i * ldv + r];
+            const double old = P.zero_start && cycles == 1 ? 0.0 : (double)x[row0 + r];
+            x[row0 + r] = (VT)(old + (P.dinv ? P.dinv[row0 + r] : 1.0) * ((t[0] + t[1]) + (t[2] + t[3])));
+        }
+        if (done) break;
+        if (!gs.sync()) return;  // x is gathered by the next residual
+    }
+    if (P.zero_start && cycles == 0)
+        for (int r = tid; r < nr; r += T) x[row0 + r] = (VT)0;
+    if (blockIdx.x == 0 && tid == 0) {
+        P.out[0] = iter;
+        P.out[1] = cycles;
+        P.out[2] = res2;
+        P.out[3] = done;
+        P.out[4] = bb;
     }
 }
 
-// FP32 residual of the inner solve: V0 = b - w (w = A d), (V0, V0) into S->rr (last block)
-__global__ void __launch_bounds__(kVecThreads) k_gm_res32(int n, const float* __restrict__ b, const float* __restrict__ w,
-                                                          float* __restrict__ V0, double* __restrict__ partial,
-                                                          unsigned int* ticket, KState* S)
+// The launch: one CTA of 512 threads per SM (fewer where there are fewer slices); the basis goes to
+// shared memory while a CTA's share of it fits beside the work vector (restart 50: up to about
+// 140,000 unknowns with an FP32 basis).
+template <class VT>
+struct GmShape {
+    const void* kernel;
+    int G, rows, threads;
+    size_t smem;
+    bool w_shared;
+    static int make(const SellView<VT>& A, int m, GmShape* out)
+    {
+        int dev = 0, sms = 0, most = 0;
+        MSFEM_CK(cudaGetDevice(&dev));
+        MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        MSFEM_CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        out->G = std::max(1, std::min(sms, A.n_slices));
+        out->rows = (A.n_slices + out->G - 1) / out->G * kSlice * A.bs;
+        const size_t small = sizeof(double) * (4 * (size_t)(m + 1) + 3 * (size_t)m) + 1024;
+        const size_t w = sizeof(double) * out->rows, v = sizeof(VT) * (size_t)(m + 1) * out->rows;
+        const bool vs = small + w + v <= (size_t)most;
+        out->w_shared = small + w <= (size_t)most;
+        out->threads = vs ? 512 : 1024;
+        out->smem = small + (out->w_shared ? w : 0) + (vs ? v : 0);
+        out->kernel = vs ? (const void*)k_gm_coop<VT, true> : (const void*)k_gm_coop<VT, false>;
+        MSFEM_CK(cudaFuncSetAttribute(out->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out->smem));
+        return MSFEM_OK;
+    }
+};
+
+// Runs the solve; P: everything but the workspace fields.  V: [m + 1][n], g0 / g1: [n].  out5 (host)
+// receives P.out.
+template <class VT>
+int gm_coop_run(System& s, GmCoop P, VT* V, VT* g0, VT* g1, double* out5)
 {
-    __shared__ double sh[32];
-    double acc[1] = {0.0};
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        const float t = b[r] - w[r];
-        V0[r] = t;
-        acc[0] += (double)t * (double)t;
+    SellView<VT> A = sell_view<VT>(s);
+    GmShape<VT> shape;
+    MSFEM_TRY(GmShape<VT>::make(A, P.m, &shape));
+    const size_t np = (size_t)(2 * P.m + 4) * shape.G, nh = (size_t)P.m * (P.m + 1) / 2;
+    MSFEM_TRY(s.gm.alloc(8 + np + nh + P.m + (shape.w_shared ? 0 : (size_t)P.n)));
+    MSFEM_CK(cudaMemsetAsync(s.gm.p, 0, sizeof(double) * 8, s.stream));
+    P.rows = shape.rows;
+    P.V = V;
+    P.gather[0] = g0;
+    P.gather[1] = g1;
+    P.out = s.gm.p;
+    P.bar = reinterpret_cast<GridBar*>(s.gm.p + 6);
+    P.partial = s.gm.p + 8;
+    P.H = P.partial + np;
+    P.y = P.H + nh;
+    P.w = shape.w_shared ? nullptr : P.y + P.m;
+    void* args[] = {&A, &P};
+    MSFEM_CK(cudaLaunchCooperativeKernel(shape.kernel, dim3(shape.G), dim3(shape.threads), args, shape.smem, s.stream));
+    s.launches += 1;
+    double h[8];
+    MSFEM_CK(cudaMemcpyAsync(h, s.gm.p, sizeof(h), cudaMemcpyDeviceToHost, s.stream));
+    MSFEM_CK(cudaStreamSynchronize(s.stream));
+    unsigned int bar[2];
+    std::memcpy(bar, &h[6], sizeof(bar));
+    if (bar[1]) {
+        set_error("GMRES: a grid barrier expired");
+        return MSFEM_ERR_CUDA;
     }
-    block_sum<1>(acc, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc[0];
-    if (arrive_last(ticket)) {
-        double t[1];
-        reduce_partials<1>(partial, gridDim.x, 0, t, sh);
-        if (threadIdx.x == 0) {
-            S->rr = t[0];
-            *ticket = 0;
-        }
-    }
+    for (int k = 0; k < 5; k++) out5[k] = h[k];
+    return MSFEM_OK;
 }
 
 }  // namespace
@@ -269,198 +376,43 @@ int solve_gmres64(System& s, int m, int maxiter, double tol, int* iters, int* re
         return MSFEM_ERR_ARGUMENT;
     }
     const int n = s.n_rows;
-    // V: (m+1) vectors, plus z (preconditioned v) and w; the first work vector doubles as r
     MSFEM_TRY(s.work64.alloc((size_t)(m + 3) * n));
     double* V = s.work64.p;
-    double* z = V + (size_t)(m + 1) * n;
-    double* w = z + n;
-    GmLayout L{m};
-    MSFEM_TRY(s.gm.alloc(L.total()));
-    MSFEM_TRY(s.partial.alloc((size_t)(m + 2) * kReduceBlocks + 64));
-    KState* S = s.kstate.p;
-    double* part = s.partial.p;
-    MSFEM_CK(cudaMemsetAsync(s.gm.p, 0, sizeof(double) * L.total(), s.stream));
-
-    const SellView<double> A = sell_view<double>(s);
-    const unsigned g = spmv_grid(s);
-    int total = 0, cycles = 0;
-    cudaGraphExec_t exec = nullptr;
-    int rc = MSFEM_OK;
-    // (F, F): the residual kernel on x = 0 gives r = F
-    MSFEM_CK(cudaMemsetAsync(z, 0, sizeof(double) * n, s.stream));
-    MSFEM_TRY(residual64(s, z, s.F.p, w, &S->ff));
-    s.launches += 1;
-    // tol2, maxiter, counters
-    KState init{};
-    MSFEM_CK(cudaMemcpyAsync(s.h_kstate, S, sizeof(KState), cudaMemcpyDeviceToHost, s.stream));
+    GmCoop P{};
+    P.n = n;
+    P.m = m;
+    P.maxiter = maxiter;
+    P.tol = tol;
+    P.dinv = s.dinv64.p;
+    P.x = s.X.p;
+    P.b = s.F.p;
+    double out[5];
+    MSFEM_TRY(gm_coop_run<double>(s, P, V, V + (size_t)(m + 1) * n, V + (size_t)(m + 2) * n, out));
+    // the caller's residual report reads (F, F)
+    MSFEM_CK(cudaMemcpyAsync(&s.kstate.p->ff, &out[4], sizeof(double), cudaMemcpyHostToDevice, s.stream));
     MSFEM_CK(cudaStreamSynchronize(s.stream));
-    init = *s.h_kstate;
-    init.tol2 = tol * tol * init.ff;
-    init.maxiter = maxiter;
-    init.iter = 0;
-    init.done = 0;
-    init.breakdown = 0;
-    for (auto& t : init.ticket) t = 0;
-    *s.h_kstate = init;
-    MSFEM_CK(cudaMemcpyAsync(S, s.h_kstate, sizeof(KState), cudaMemcpyHostToDevice, s.stream));
-
-    while (true) {
-        // r = F - A x into V_0's slot, then V_0 = r / ||r||
-        MSFEM_TRY(residual64(s, s.X.p, s.F.p, V, &S->rr));
-        MSFEM_CK(cudaMemcpyAsync(s.h_kstate, S, sizeof(KState), cudaMemcpyDeviceToHost, s.stream));
-        MSFEM_CK(cudaStreamSynchronize(s.stream));
-        s.launches += 1;
-        if (s.h_kstate->rr <= s.h_kstate->tol2 || s.h_kstate->done || total >= maxiter) break;
-        k_gm_start<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, V, s.gm.p, L, S);
-        s.launches += 1;
-        if (!exec) {
-            cudaGraph_t graph;
-            MSFEM_CK(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
-            for (int j = 0; j < m; j++) {
-                double* vj = V + (size_t)j * n;
-                k_gm_prec<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, vj, s.dinv64.p, z, s.gm.p, L);
-                k_gm_spmv<double><<<g, 256, 0, s.stream>>>(A, z, w, s.gm.p, L);
-                k_gm_multidot<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0], s.gm.p,
-                                                                                   L, L.h1());
-                k_gm_orth<double, false><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0],
-                                                                                      s.gm.p, L, L.h1());
-                k_gm_multidot<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0], s.gm.p,
-                                                                                   L, L.h2());
-                k_gm_orth<double, true><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0],
-                                                                                     s.gm.p, L, L.h2());
-                k_gm_save_norm<<<1, 1, 0, s.stream>>>(j, s.gm.p, L);
-                k_gm_givens<<<1, 1, 0, s.stream>>>(j, s.gm.p, L, S);
-                k_gm_normalize<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, w, V + (size_t)(j + 1) * n, j,
-                                                                                    s.gm.p, L);
-            }
-            k_gm_backsolve<<<1, 1, 0, s.stream>>>(s.gm.p, L);
-            k_gm_update<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, s.X.p, V, s.dinv64.p, s.gm.p, L);
-            cudaError_t e = cudaStreamEndCapture(s.stream, &graph);
-            if (e != cudaSuccess) {
-                set_error("GMRES graph capture failed: %s", cudaGetErrorString(e));
-                return MSFEM_ERR_CUDA;
-            }
-            e = cudaGraphInstantiate(&exec, graph, 0);
-            cudaGraphDestroy(graph);
-            if (e != cudaSuccess) {
-                set_error("GMRES graph instantiate failed: %s", cudaGetErrorString(e));
-                return MSFEM_ERR_CUDA;
-            }
-        }
-        cudaError_t e = cudaGraphLaunch(exec, s.stream);
-        if (e != cudaSuccess) {
-            set_error("GMRES graph launch failed: %s", cudaGetErrorString(e));
-            rc = MSFEM_ERR_CUDA;
-            break;
-        }
-        s.launches += 9 * m + 2;
-        cycles++;
-        MSFEM_CK(cudaMemcpyAsync(s.h_kstate, S, sizeof(KState), cudaMemcpyDeviceToHost, s.stream));
-        MSFEM_CK(cudaStreamSynchronize(s.stream));
-        total = s.h_kstate->iter;
-        if (s.h_kstate->done) break;
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (rc < 0) return rc;
-    *iters = s.h_kstate->iter;
-    *restarts = cycles;
-    return (s.h_kstate->rr <= s.h_kstate->tol2) ? MSFEM_OK : MSFEM_NOT_CONVERGED;
+    *iters = (int)out[0];
+    *restarts = (int)out[1];
+    return out[2] <= tol * tol * out[4] ? MSFEM_OK : MSFEM_NOT_CONVERGED;
 }
 
 // Inner solve of FP32 iterative refinement: GMRES(m) on the FP32 copy of the Jacobi-scaled matrix
 // (unit diagonal, so no preconditioner), A d = b from d = 0, to ||b - A d|| <= tau ||b||.  The
 // Krylov basis is FP32 (half the bytes of the FP64 solver per Arnoldi pass); the Hessenberg
-// matrix, the rotations and every inner product are FP64.  V is (m+1) n floats, w one more n.
-int gmres32_inner(System& s, int m, float* d, const float* b, float* V, float* w, int maxiter, double tau, int* iters)
+// matrix, the rotations and every inner product are FP64.  V is (m+1) n floats, g two more n.
+int gmres32_inner(System& s, int m, float* d, const float* b, float* V, float* g, int maxiter, double tau, int* iters)
 {
-    const int n = s.n_rows;
-    GmLayout L{m};
-    MSFEM_TRY(s.gm.alloc(L.total()));
-    MSFEM_TRY(s.partial.alloc((size_t)(m + 2) * kReduceBlocks + 64));
-    KState* S = s.kstate.p;
-    double* part = s.partial.p;
-    MSFEM_CK(cudaMemsetAsync(s.gm.p, 0, sizeof(double) * L.total(), s.stream));
-    const SellView<float> A = sell_view<float>(s);
-    const unsigned g = spmv_grid(s);
-    // (b, b) -> ff via the residual kernel with w = 0
-    MSFEM_CK(cudaMemsetAsync(w, 0, sizeof(float) * n, s.stream));
-    k_gm_res32<<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, b, w, V, part, &S->ticket[0], S);
-    s.launches += 1;
-    MSFEM_CK(cudaMemcpyAsync(s.h_kstate, S, sizeof(KState), cudaMemcpyDeviceToHost, s.stream));
-    MSFEM_CK(cudaStreamSynchronize(s.stream));
-    KState init = *s.h_kstate;
-    init.ff = init.rr;
-    init.tol2 = tau * tau * init.ff;
-    init.maxiter = maxiter;
-    init.iter = 0;
-    init.done = 0;
-    init.breakdown = 0;
-    for (auto& t : init.ticket) t = 0;
-    *s.h_kstate = init;
-    MSFEM_CK(cudaMemcpyAsync(S, s.h_kstate, sizeof(KState), cudaMemcpyHostToDevice, s.stream));
-    cudaGraphExec_t exec = nullptr;
-    int rc = MSFEM_OK;
-    bool first = true;
-    while (true) {
-        if (!first) {
-            // V_0 = b - A d
-            MSFEM_TRY(spmv32(s, d, w));
-            k_gm_res32<<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, b, w, V, part, &S->ticket[0], S);
-            s.launches += 2;
-            MSFEM_CK(cudaMemcpyAsync(s.h_kstate, S, sizeof(KState), cudaMemcpyDeviceToHost, s.stream));
-            MSFEM_CK(cudaStreamSynchronize(s.stream));
-        }
-        first = false;  // on entry d = 0 and V_0 already holds b
-        if (s.h_kstate->rr <= s.h_kstate->tol2 || s.h_kstate->done || s.h_kstate->iter >= maxiter) break;
-        k_gm_start<float><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, V, s.gm.p, L, S);
-        s.launches += 1;
-        if (!exec) {
-            cudaGraph_t graph;
-            MSFEM_CK(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
-            for (int j = 0; j < m; j++) {
-                const float* vj = V + (size_t)j * n;
-                k_gm_spmv<float><<<g, 256, 0, s.stream>>>(A, vj, w, s.gm.p, L);
-                k_gm_multidot<float><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0], s.gm.p,
-                                                                                  L, L.h1());
-                k_gm_orth<float, false><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0],
-                                                                                     s.gm.p, L, L.h1());
-                k_gm_multidot<float><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0], s.gm.p,
-                                                                                  L, L.h2());
-                k_gm_orth<float, true><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, V, j, w, part, &S->ticket[0],
-                                                                                    s.gm.p, L, L.h2());
-                k_gm_save_norm<<<1, 1, 0, s.stream>>>(j, s.gm.p, L);
-                k_gm_givens<<<1, 1, 0, s.stream>>>(j, s.gm.p, L, S);
-                k_gm_normalize<float><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, w, V + (size_t)(j + 1) * n, j,
-                                                                                   s.gm.p, L);
-            }
-            k_gm_backsolve<<<1, 1, 0, s.stream>>>(s.gm.p, L);
-            k_gm_update<float><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, d, V, nullptr, s.gm.p, L);
-            cudaError_t e = cudaStreamEndCapture(s.stream, &graph);
-            if (e != cudaSuccess) {
-                set_error("GMRES graph capture failed: %s", cudaGetErrorString(e));
-                return MSFEM_ERR_CUDA;
-            }
-            e = cudaGraphInstantiate(&exec, graph, 0);
-            cudaGraphDestroy(graph);
-            if (e != cudaSuccess) {
-                set_error("GMRES graph instantiate failed: %s", cudaGetErrorString(e));
-                return MSFEM_ERR_CUDA;
-            }
-        }
-        cudaError_t e = cudaGraphLaunch(exec, s.stream);
-        if (e != cudaSuccess) {
-            set_error("GMRES graph launch failed: %s", cudaGetErrorString(e));
-            rc = MSFEM_ERR_CUDA;
-            break;
-        }
-        s.launches += 8 * m + 2;
-        MSFEM_CK(cudaMemcpyAsync(s.h_kstate, S, sizeof(KState), cudaMemcpyDeviceToHost, s.stream));
-        MSFEM_CK(cudaStreamSynchronize(s.stream));
-        if (s.h_kstate->done) break;
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (rc < 0) return rc;
-    *iters = s.h_kstate->iter;
+    GmCoop P{};
+    P.n = s.n_rows;
+    P.m = m;
+    P.maxiter = maxiter;
+    P.tol = tau;
+    P.x = d;
+    P.b = b;
+    P.zero_start = 1;
+    double out[5];
+    MSFEM_TRY(gm_coop_run<float>(s, P, V, g, g + s.n_rows, out));
+    *iters = (int)out[0];
     return MSFEM_OK;
 }
 

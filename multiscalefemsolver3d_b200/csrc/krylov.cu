@@ -792,8 +792,8 @@ int solve_refined(System& s, Inner inner, int maxiter, double tol, int* iters, i
         return MSFEM_ERR_ARGUMENT;
     }
     if (inner != INNER_MINRES64) {
-        // GMRES: d, r, then the (m+1) basis vectors and w
-        MSFEM_TRY(s.work32.alloc((inner == INNER_GMRES32 ? (size_t)restart_m + 4 : 5) * (size_t)n));
+        // GMRES: d, r, then the (m+1) basis vectors and two gathered ones
+        MSFEM_TRY(s.work32.alloc((inner == INNER_GMRES32 ? (size_t)restart_m + 5 : 5) * (size_t)n));
         d32 = s.work32.p;
         r32 = d32 + n;
         p32 = r32 + n;

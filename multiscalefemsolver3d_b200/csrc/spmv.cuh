@@ -2,6 +2,7 @@
 #pragma once
 
 #include "devutil.cuh"
+#include "gridsync.cuh"
 #include "internal.cuh"
 
 namespace msfem {
@@ -46,6 +47,15 @@ struct Vec4<double> {
     }
 };
 
+// one element of the gathered vector; LIVE: the running kernel also writes it (the persistent
+// solvers), so the read-only path is closed
+template <bool LIVE, class VT>
+__device__ __forceinline__ VT gather_x(const VT* x)
+{
+    if constexpr (LIVE) return load_shared_vector<VT>(x);
+    else return __ldg(x);
+}
+
 // Row `warp*32 + lane` of a scalar SELL slice times x.  All lanes of the warp
 // must call it (the loop runs to the slice width).
 // 4 consecutive 16-bit column deltas of one lane (one 8-byte load)
@@ -58,8 +68,8 @@ __device__ __forceinline__ void load_delta4(const int16_t* p, int row0, int (&c)
     c[3] = row0 + (int)(short)((unsigned)q.y >> 16);
 }
 
-template <class VT>
-__device__ __forceinline__ VT sell_row_scalar16(const SellView<VT>& A, int warp, int lane, const VT* __restrict__ x)
+template <class VT, bool LIVE = false>
+__device__ __forceinline__ VT sell_row_scalar16(const SellView<VT>& A, int warp, int lane, const VT* x)
 {
     const int64_t base = A.sp[warp];
     const int w = (int)((A.sp[warp + 1] - base) >> 5);
@@ -80,7 +90,7 @@ __device__ __forceinline__ VT sell_row_scalar16(const SellView<VT>& A, int warp,
 #pragma unroll
         for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) xs[q][e] = __ldg(x + c[q][e]);
+            for (int e = 0; e < 4; e++) xs[q][e] = gather_x<LIVE>(x + c[q][e]);
 #pragma unroll
         for (int q = 0; q < 4; q++)
 #pragma unroll
@@ -92,15 +102,15 @@ __device__ __forceinline__ VT sell_row_scalar16(const SellView<VT>& A, int warp,
         load_delta4(cp + (int64_t)k * kSlice, row0, c);
         Vec4<VT>::load(vp + (int64_t)k * kSlice, v);
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc += v[e] * __ldg(x + c[e]);
+        for (int e = 0; e < 4; e++) acc += v[e] * gather_x<LIVE>(x + c[e]);
     }
     return acc;
 }
 
-template <class VT>
-__device__ __forceinline__ VT sell_row_scalar(const SellView<VT>& A, int warp, int lane, const VT* __restrict__ x)
+template <class VT, bool LIVE = false>
+__device__ __forceinline__ VT sell_row_scalar(const SellView<VT>& A, int warp, int lane, const VT* x)
 {
-    if (A.col16) return sell_row_scalar16<VT>(A, warp, lane, x);
+    if (A.col16) return sell_row_scalar16<VT, LIVE>(A, warp, lane, x);
     const int64_t base = A.sp[warp];
     const int w = (int)((A.sp[warp + 1] - base) >> 5);
     const int32_t* cp = A.col + base + lane * kChunk;
@@ -122,10 +132,10 @@ __device__ __forceinline__ VT sell_row_scalar(const SellView<VT>& A, int warp, i
             VT xs[4][4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                xs[q][0] = __ldg(x + c[q].x);
-                xs[q][1] = __ldg(x + c[q].y);
-                xs[q][2] = __ldg(x + c[q].z);
-                xs[q][3] = __ldg(x + c[q].w);
+                xs[q][0] = gather_x<LIVE>(x + c[q].x);
+                xs[q][1] = gather_x<LIVE>(x + c[q].y);
+                xs[q][2] = gather_x<LIVE>(x + c[q].z);
+                xs[q][3] = gather_x<LIVE>(x + c[q].w);
             }
 #pragma unroll
             for (int q = 0; q < 4; q++)
@@ -138,18 +148,17 @@ __device__ __forceinline__ VT sell_row_scalar(const SellView<VT>& A, int warp, i
         const int4 c = __ldcs(reinterpret_cast<const int4*>(cp + (int64_t)k * kSlice));
         VT v[4];
         Vec4<VT>::load(vp + (int64_t)k * kSlice, v);
-        acc += v[0] * __ldg(x + c.x);
-        acc += v[1] * __ldg(x + c.y);
-        acc += v[2] * __ldg(x + c.z);
-        acc += v[3] * __ldg(x + c.w);
+        acc += v[0] * gather_x<LIVE>(x + c.x);
+        acc += v[1] * gather_x<LIVE>(x + c.y);
+        acc += v[2] * gather_x<LIVE>(x + c.z);
+        acc += v[3] * gather_x<LIVE>(x + c.w);
     }
     return acc;
 }
 
 // Block row `warp*32 + lane` of a 3x3-block SELL slice times x (x node-major).
-template <class VT>
-__device__ __forceinline__ void sell_row_block(const SellView<VT>& A, int warp, int lane, const VT* __restrict__ x,
-                                               VT (&acc)[3])
+template <class VT, bool LIVE = false>
+__device__ __forceinline__ void sell_row_block(const SellView<VT>& A, int warp, int lane, const VT* x, VT (&acc)[3])
 {
     const int64_t base = A.sp[warp];
     const int w = (int)((A.sp[warp + 1] - base) >> 5);
@@ -159,7 +168,7 @@ __device__ __forceinline__ void sell_row_block(const SellView<VT>& A, int warp, 
         const int64_t blk = base + (int64_t)k * kSlice;
         const int c = __ldcs(A.col + blk + lane);
         const VT* vb = A.val + 9 * blk + lane;
-        const VT x0 = __ldg(x + 3 * (int64_t)c), x1 = __ldg(x + 3 * (int64_t)c + 1), x2 = __ldg(x + 3 * (int64_t)c + 2);
+        const VT x0 = gather_x<LIVE>(x + 3 * (int64_t)c), x1 = gather_x<LIVE>(x + 3 * (int64_t)c + 1), x2 = gather_x<LIVE>(x + 3 * (int64_t)c + 2);
         VT v[9];
 #pragma unroll
         for (int e = 0; e < 9; e++) v[e] = __ldcs(vb + e * kSlice);
