@@ -30,12 +30,13 @@ namespace {
 // keeps the rotations and the residual estimate itself, from the same sums in the same order; CTA 0
 // keeps the Hessenberg matrix.  The launch-per-kernel cycle this replaces was bound by its launches
 // and by the last block's serial reduction of j + 1 sums: with restart 50 an Arnoldi step took 134 us
-// at 72,522 unknowns, 160 us at 282,962 and 306 us at 949,567 (FP32 basis); here 20, 47 and 179 us.
+// at 72,522 unknowns, 160 us at 282,962 and 306 us at 949,567 (FP32 basis); here 17, 42 and 142 us.
 // With the basis in global memory 1024 threads beat 512 (47 against 55 us at 282,962 unknowns, FP64 56
 // against 89): more loads in flight per SM; in shared memory 512 leave room for the basis.
 
 struct GmCoop {
     int n, m, maxiter, rows;  // rows: capacity of a CTA (slices * 32 * bs)
+    int keep;                 // part of the matrix left in the L2, of 1024
     double tol;
     const double* dinv;       // right preconditioner diag(A)^-1, or null
     void* x;                  // solution, VT
@@ -77,7 +78,7 @@ __device__ __forceinline__ bool grid_sums(GridSync& gs, double* partial, const d
 
 // VS: the basis rows are in shared memory
 template <class VT, bool VS>
-__global__ void __launch_bounds__(VS ? 512 : 1024) k_gm_coop(SellView<VT> A, GmCoop P)
+__global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, GmCoop P)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ int s_ok;
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(VS ? 512 : 1024) k_gm_coop(SellView<VT> A, GmC
     GridSync gs(P.bar, &s_ok);
     const int G = gridDim.x;
     const int s0 = (int)((int64_t)A.n_slices * blockIdx.x / G), s1 = (int)((int64_t)A.n_slices * (blockIdx.x + 1) / G);
-    const int row0 = s0 * kSlice * A.bs;
+    const int row0 = s0 * kSlice * A.bs, kept = s0 + ((s1 - s0) * P.keep + 512) / 1024;
     const int nr = min((s1 - s0) * kSlice * A.bs, max(0, P.n - row0));  // this CTA's rows
     if (VS) {
         V = reinterpret_cast<VT*>(y + m + P.rows);
@@ -116,11 +117,11 @@ __global__ void __launch_bounds__(VS ? 512 : 1024) k_gm_coop(SellView<VT> A, GmC
         for (int sl = s0 + warp; sl < s1; sl += nw) {
             const int lr = (sl - s0) * kSlice * A.bs + lane * A.bs;
             if (A.bs == 1) {
-                const VT t = sell_row_scalar<VT, true>(A, sl, lane, v);
+                const VT t = sell_row_kept<VT>(A, sl, lane, v, sl < kept);
                 if (lr < nr) w[lr] = (double)(VT)(t * (VT)scale);
             } else {
                 VT t[3];
-                sell_row_block<VT, true>(A, sl, lane, v, t);
+                sell_block_kept<VT>(A, sl, lane, v, t, sl < kept);
                 if (lr < nr)
                     for (int c = 0; c < 3; c++) w[lr + c] = (double)(VT)(t[c] * (VT)scale);
             }
@@ -309,7 +310,7 @@ struct GmShape {
     const void* kernel;
     int G, rows, threads;
     size_t smem;
-    bool w_shared;
+    bool w_shared, basis_shared;
     static int make(const SellView<VT>& A, int m, GmShape* out)
     {
         int dev = 0, sms = 0, most = 0;
@@ -321,6 +322,7 @@ struct GmShape {
         const size_t small = sizeof(double) * (4 * (size_t)(m + 1) + 3 * (size_t)m) + 1024;
         const size_t w = sizeof(double) * out->rows, v = sizeof(VT) * (size_t)(m + 1) * out->rows;
         const bool vs = small + w + v <= (size_t)most;
+        out->basis_shared = vs;
         out->w_shared = small + w <= (size_t)most;
         out->threads = vs ? 512 : 1024;
         out->smem = small + (out->w_shared ? w : 0) + (vs ? v : 0);
@@ -342,6 +344,8 @@ int gm_coop_run(System& s, GmCoop P, VT* V, VT* g0, VT* g1, double* out5)
     MSFEM_TRY(s.gm.alloc(8 + np + nh + P.m + (shape.w_shared ? 0 : (size_t)P.n)));
     MSFEM_CK(cudaMemsetAsync(s.gm.p, 0, sizeof(double) * 8, s.stream));
     P.rows = shape.rows;
+    // a basis in global memory would push a kept matrix out of the L2 in turn
+    P.keep = shape.basis_shared ? keep_share(s, sizeof(VT)) : 0;
     P.V = V;
     P.gather[0] = g0;
     P.gather[1] = g1;

@@ -79,6 +79,9 @@ struct DBuf {
 struct Sell {
     int n_slices = 0;
     int64_t stored = 0;  // stored entries (scalar) or blocks (block3), padding included
+    int max_width = 0;   // widest slice, in entries (blocks) per row
+    DBuf<int2> span;     // lowest and highest column (node) of each slice
+    int max_span = 0;    // widest column range of an SM's share of the slices
     DBuf<int64_t> slice_ptr;
     DBuf<int32_t> col;    // absolute column (3x3 blocks, or scalar when deltas do not fit 16 bits)
     DBuf<int16_t> col16;  // scalar: column - min(row, n-1), when every delta fits in 16 bits
@@ -147,6 +150,7 @@ struct System {
     KState* h_ahead = nullptr;   // two pinned snapshots taken after queued iteration chunks
     cudaEvent_t ev_chunk[2] = {nullptr, nullptr};
     DBuf<double> gm;      // GMRES: Hessenberg / rotations / y on the device
+    DBuf<unsigned char> coop;  // grid barrier and posted sums of the one-launch solvers
     DBuf<double> mr64;    // MINRES vectors (FP64)
     DBuf<float> mr32;     // MINRES vectors (FP32)
 
@@ -226,6 +230,11 @@ int ensure_kstate(System& s);
 int solve(System& s, int method, int precision, int restart_m, int maxiter, double tol, double* relres, int* iters);
 int ensure_state(System& s);
 int read_state(System& s);
+// ---- CG in one cooperative launch (krylov_coop.cu): S->tol2 set; iter, rr, done, breakdown left in
+// the host's KState mirror.  FP64 from the residual r; FP32 from x = 0 with right-hand side r, to tol
+// times its norm, or until (r, r) has not set a 2 % low for stall_limit iterations
+int pcg64_coop(System& s, bool jacobi, double* x, double* r, double* p, double* q, double* z, int maxiter);
+int cg32_coop(System& s, float* x, float* r, float* w, float* p, float* sv, double tol, int maxiter, int stall_limit);
 // ---- the MsFEM macro solve on device data (macro.cu)
 int macro_solve_device(int n_vertices, int n_cells, const int32_t* cell_vertex, const double* dK, const double* dF,
                        int n_fixed, const int32_t* fixed_vertices, const double* fixed_values, int precision, double tol,

@@ -49,289 +49,6 @@ __global__ void __launch_bounds__(kVecThreads) k_dot_self(int n, const VT* __res
     }
 }
 
-// PCG as in CSSD_Matrix::MSG_PreconditioningSSOR (CSSD_Matrix.h:1336-1362), with M = diag(A)
-// (or M = I): three kernels per iteration -- q = A p with (p, q) -> alpha; the x/r/z update with
-// (r, z), (r, r) -> beta and the stopping test; p = z + beta p.  Without a preconditioner, and for
-// the FP32 solves on the Jacobi-scaled matrix, z is r itself and is never stored.
-// z = M^{-1} r, p = z, (r,z), (r,r); sets rz, rr and the initial stopping test
-template <class VT, bool JAC>
-__global__ void __launch_bounds__(kVecThreads) k_pcg_init(int n, const VT* r, const VT* __restrict__ dinv, VT* z,
-                                                          VT* __restrict__ p, KState* S,
-                                                          double* __restrict__ partial)
-{
-    __shared__ double sh[64];
-    double acc[2] = {0.0, 0.0};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const VT rv = r[i];
-        const VT zv = JAC ? rv * dinv[i] : rv;
-        if (JAC) z[i] = zv;  // without a preconditioner z is r itself and is never stored
-        p[i] = zv;
-        acc[0] += (double)rv * (double)zv;
-        acc[1] += (double)rv * (double)rv;
-    }
-    block_sum<2>(acc, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = acc[0];
-        partial[gridDim.x + blockIdx.x] = acc[1];
-    }
-    if (arrive_last(&S->ticket[0])) {
-        double t[2];
-        reduce_partials<2>(partial, gridDim.x, gridDim.x, t, sh);
-        if (threadIdx.x == 0) {
-            S->rz = t[0];
-            S->rr = t[1];
-            S->rr_min = t[1];
-            S->stall = 0;
-            S->iter = 0;
-            S->breakdown = 0;
-            S->done = (t[1] <= S->tol2) ? 1 : 0;
-            S->ticket[0] = 0;
-        }
-    }
-}
-
-// q = A p, (p, q) -> alpha = rz / (p, q)
-template <class VT>
-__global__ void __launch_bounds__(256) k_pcg_spmv(SellView<VT> A, const VT* __restrict__ p, VT* __restrict__ q,
-                                                  KState* S, double* __restrict__ partial)
-{
-    if (S->done) return;
-    __shared__ double sh[32];
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    double acc[1] = {0.0};
-    for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < A.n_slices; warp += nw) {
-        if (A.bs == 1) {
-            const VT v = sell_row_scalar<VT>(A, warp, lane, p);
-            const int row = warp * kSlice + lane;
-            if (row < A.n_rows) {
-                q[row] = v;
-                acc[0] += (double)p[row] * (double)v;
-            }
-        } else {
-            VT v[3];
-            sell_row_block<VT>(A, warp, lane, p, v);
-            const int brow = warp * kSlice + lane;
-            if (brow < A.n_brows)
-                for (int c = 0; c < 3; c++) {
-                    q[3 * (int64_t)brow + c] = v[c];
-                    acc[0] += (double)p[3 * (int64_t)brow + c] * (double)v[c];
-                }
-        }
-    }
-    block_sum<1>(acc, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = acc[0];
-    if (arrive_last(&S->ticket[0])) {
-        double t[1];
-        reduce_partials<1>(partial, gridDim.x, 0, t, sh);
-        if (threadIdx.x == 0) {
-            S->pq = t[0];
-            if (t[0] == 0.0 || t[0] != t[0]) {
-                S->breakdown = 1;
-                S->done = 1;
-            }
-            S->alpha = S->rz / t[0];
-            S->ticket[0] = 0;
-        }
-    }
-}
-
-// x += alpha p, r -= alpha q, z = M^{-1} r, (r,z), (r,r) -> beta, stopping test
-template <class VT, bool JAC>
-__global__ void __launch_bounds__(kVecThreads) k_pcg_update(int n, VT* __restrict__ x, VT* r, VT* z,
-                                                            const VT* __restrict__ p,
-                                                            const VT* __restrict__ q, const VT* __restrict__ dinv,
-                                                            KState* S, double* __restrict__ partial)
-{
-    if (S->done) return;
-    __shared__ double sh[64];
-    const VT alpha = (VT)S->alpha;
-    double acc[2] = {0.0, 0.0};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        x[i] += alpha * p[i];
-        const VT rv = r[i] - alpha * q[i];
-        r[i] = rv;
-        const VT zv = JAC ? rv * dinv[i] : rv;
-        if (JAC) z[i] = zv;
-        acc[0] += (double)rv * (double)zv;
-        acc[1] += (double)rv * (double)rv;
-    }
-    block_sum<2>(acc, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = acc[0];
-        partial[gridDim.x + blockIdx.x] = acc[1];
-    }
-    if (arrive_last(&S->ticket[0])) {
-        double t[2];
-        reduce_partials<2>(partial, gridDim.x, gridDim.x, t, sh);
-        if (threadIdx.x == 0) {
-            S->beta = t[0] / S->rz;
-            S->rz = t[0];
-            S->rr = t[1];
-            S->iter += 1;
-            if (t[1] < 0.98 * S->rr_min) {
-                S->rr_min = t[1];
-                S->stall = 0;
-            } else {
-                S->stall += 1;
-            }
-            if (t[1] <= S->tol2) S->done = 1;
-            else if (S->iter >= S->maxiter) S->done = 2;
-            else if (t[1] != t[1]) {
-                S->breakdown = 1;
-                S->done = 3;
-            } else if (S->stall >= S->stall_limit) {
-                S->done = 4;  // stagnated at the precision's attainable accuracy
-            }
-            S->ticket[0] = 0;
-        }
-    }
-}
-
-template <class VT>
-__global__ void __launch_bounds__(kVecThreads) k_pcg_p(int n, const VT* z, VT* __restrict__ p,
-                                                       const KState* S)
-{
-    if (S->done) return;
-    const VT beta = (VT)S->beta;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = z[i] + beta * p[i];
-}
-
-// ------------------------------------------------------------------ FP32 CG in two kernels
-// The FP32 inner solve of the refinement runs CG in the Chronopoulos-Gear arrangement, which needs
-// one reduction phase per iteration instead of two:
-//   w = A r,  gamma = (r, r),  delta = (w, r)                      (k_cg2_spmv)
-//   beta = gamma / gamma_old,  alpha = gamma / (delta - beta gamma / alpha_old)
-//   p = r + beta p,  s = w + beta s,  x += alpha p,  r -= alpha s   (k_cg2_update)
-// k_cg2_spmv writes per-block partial sums and its last block adds them in a fixed order into
-// S->cg2_gd; every block of k_cg2_update forms the step's scalars from those two numbers (so all
-// blocks hold the same scalars, bit for bit) and block 0 records the state.  The scalars of the previous iteration live in one of two slots (parity passed by the
-// host), so no block reads a value that block 0 overwrites in the same launch.
-// Slot layout in KState::mr: [5 * slot + 0] gamma, +1 alpha, +2 iterations, +3 lowest (r, r),
-// +4 iterations since (r, r) last set a 2 % low.
-
-__global__ void __launch_bounds__(256) k_cg2_spmv(SellView<float> A, const float* __restrict__ r,
-                                                  float* __restrict__ w, const KState* S,
-                                                  double* __restrict__ partial)
-{
-    if (S->done) return;
-    __shared__ double sh[64];
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    double acc[2] = {0.0, 0.0};
-    for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < A.n_slices; warp += nw) {
-        if (A.bs == 1) {
-            const float v = sell_row_scalar<float>(A, warp, lane, r);
-            const int row = warp * kSlice + lane;
-            if (row < A.n_rows) {
-                w[row] = v;
-                const double rv = (double)r[row];
-                acc[0] += rv * rv;
-                acc[1] += (double)v * rv;
-            }
-        } else {
-            float v[3];
-            sell_row_block<float>(A, warp, lane, r, v);
-            const int brow = warp * kSlice + lane;
-            if (brow < A.n_brows)
-                for (int c = 0; c < 3; c++) {
-                    const int64_t i = 3 * (int64_t)brow + c;
-                    w[i] = v[c];
-                    const double rv = (double)r[i];
-                    acc[0] += rv * rv;
-                    acc[1] += (double)v[c] * rv;
-                }
-        }
-    }
-    block_sum<2>(acc, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = acc[0];
-        partial[gridDim.x + blockIdx.x] = acc[1];
-    }
-    KState* Sw = const_cast<KState*>(S);
-    if (arrive_last(&Sw->ticket[2])) {
-        double t[2];
-        reduce_partials<2>(partial, gridDim.x, gridDim.x, t, sh);
-        if (threadIdx.x == 0) {
-            Sw->cg2_gd[0] = t[0];
-            Sw->cg2_gd[1] = t[1];
-            Sw->ticket[2] = 0;
-        }
-    }
-}
-
-// first = 1: the start (beta = 0, p = r, s = w); slot: the parity of the previous scalars
-__global__ void __launch_bounds__(kVecThreads) k_cg2_update(int n, float* __restrict__ x, float* __restrict__ r,
-                                                            const float* __restrict__ w, float* __restrict__ p,
-                                                            float* __restrict__ s, KState* S,
-                                                            const double* __restrict__ partial, int g_spmv, int slot,
-                                                            int first)
-{
-    if (S->done) return;
-    __shared__ double sc[4];  // alpha, beta, done
-    (void)partial;
-    (void)g_spmv;
-    if (threadIdx.x == 0) {
-        const double gamma = S->cg2_gd[0], delta = S->cg2_gd[1];
-        const double* old = S->mr + 5 * slot;
-        const int iter = first ? 0 : (int)old[2];
-        double rr_min = first ? gamma : old[3];
-        int stall = first ? 0 : (int)old[4];
-        if (!first) {
-            if (gamma < 0.98 * rr_min) {
-                rr_min = gamma;
-                stall = 0;
-            } else {
-                stall += 1;
-            }
-        }
-        double beta = first ? 0.0 : gamma / old[0];
-        const double den = first ? delta : delta - beta * gamma / old[1];
-        const double alpha = gamma / den;
-        int done = 0;
-        if (gamma <= S->tol2) done = 1;
-        else if (iter >= S->maxiter) done = 2;
-        else if (!(den != 0.0) || den != den || gamma != gamma) done = 3;  // breakdown
-        else if (stall >= S->stall_limit) done = 4;  // FP32 attainable accuracy reached
-        sc[0] = alpha;
-        sc[1] = beta;
-        sc[2] = done;
-        if (blockIdx.x == 0) {
-            double* nw = S->mr + 5 * (1 - slot);
-            nw[0] = gamma;
-            nw[1] = alpha;
-            nw[2] = done ? iter : iter + 1;
-            nw[3] = rr_min;
-            nw[4] = stall;
-            S->rr = gamma;
-            S->iter = done ? iter : iter + 1;
-            if (done == 3) S->breakdown = 1;
-            if (done) S->done = done;
-        }
-    }
-    __syncthreads();
-    if (sc[2] != 0.0) return;
-    const float alpha = (float)sc[0], beta = (float)sc[1];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float ri = r[i], wi = w[i];
-        const float pi = first ? ri : ri + beta * p[i];
-        const float si = first ? wi : wi + beta * s[i];
-        p[i] = pi;
-        s[i] = si;
-        x[i] += alpha * pi;
-        r[i] = ri - alpha * si;
-    }
-}
-
-// generic residual in VT: r = b - A x  (used by the FP32 inner solve with x = 0 -> r = b)
-template <class VT>
-__global__ void __launch_bounds__(kVecThreads) k_copy(int n, const VT* __restrict__ a, VT* __restrict__ b)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        b[i] = a[i];
-}
-
 // FP32-IR helpers
 // r32 = D^-1/2 r / ||r||  (the scaled system's right-hand side), d32 = 0
 __global__ void __launch_bounds__(kVecThreads) k_scale_to32(int n, const double* __restrict__ r, const double* rr,
@@ -685,59 +402,8 @@ std::string graph_key(const char* tag, std::initializer_list<const void*> ptrs, 
     return k + buf;
 }
 
-template <class VT>
-struct PcgVectors {
-    VT *x, *r, *z, *p, *q;  // z == r without a preconditioner
-    const VT* dinv;
-};
-
-// r holds the initial residual on entry; x is updated in place
-template <class VT, bool JAC>
-int pcg_run(System& s, PcgVectors<VT> v, int maxiter)
-{
-    const int n = s.n_rows;
-    KState* S = s.kstate.p;
-    double* part = s.partial.p;
-    k_pcg_init<VT, JAC><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, v.r, v.dinv, v.z, v.p, S, part);
-    MSFEM_CK(cudaGetLastError());
-    s.launches += 1;
-    const SellView<VT> A = sell_view<VT>(s);
-    const unsigned g = spmv_grid_of((const void*)k_pcg_spmv<VT>, s);
-    auto iteration = [&]() {
-        k_pcg_spmv<VT><<<g, 256, 0, s.stream>>>(A, v.p, v.q, S, part);
-        k_pcg_update<VT, JAC><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, v.x, v.r, v.z, v.p, v.q, v.dinv, S, part);
-        k_pcg_p<VT><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, v.z, v.p, S);
-    };
-    const std::string key = graph_key(sizeof(VT) == 8 ? (JAC ? "pcg64j" : "pcg64") : (JAC ? "pcg32j" : "pcg32"),
-                                      {v.x, v.r, v.z, v.p, v.q, v.dinv, A.val, A.col, (const void*)S, part}, n);
-    return run_chunks(s, key, iteration, 3, maxiter);
-}
-
-// FP32 CG (Chronopoulos-Gear, two kernels per iteration) on the Jacobi-scaled FP32 matrix from
-// x = 0: r holds the right-hand side on entry; S->tol2 / maxiter / stall_limit set by the caller.
-// Vectors: x, r, w, p, s (n floats each).
-int cg2_run(System& s, float* x, float* r, float* w, float* p, float* sv, int maxiter)
-{
-    const int n = s.n_rows;
-    KState* S = s.kstate.p;
-    double* part = s.partial.p;
-    const SellView<float> A = sell_view<float>(s);
-    const unsigned g = spmv_grid_of((const void*)k_cg2_spmv, s);
-    MSFEM_CK(cudaMemsetAsync(x, 0, sizeof(float) * n, s.stream));
-    k_cg2_spmv<<<g, 256, 0, s.stream>>>(A, r, w, S, part);
-    k_cg2_update<<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, x, r, w, p, sv, S, part, (int)g, 1, 1);
-    MSFEM_CK(cudaGetLastError());
-    s.launches += 2;
-    int parity = 0;  // slot of the scalars the next update reads: the first update wrote slot 0
-    auto iteration = [&]() {
-        k_cg2_spmv<<<g, 256, 0, s.stream>>>(A, r, w, S, part);
-        k_cg2_update<<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, x, r, w, p, sv, S, part, (int)g, parity, 0);
-        parity ^= 1;
-    };
-    // every captured chunk holds an even number of iterations, so each replay starts on slot 0
-    const std::string key = graph_key("cg2_32", {x, r, w, p, sv, A.val, A.col, (const void*)S, part}, n);
-    return run_chunks(s, key, iteration, 2, maxiter);
-}
+// vector stride of the one-launch solvers: 16-byte rows, readable past the end by a vector load
+size_t padded(int n) { return ((size_t)n + 63) / 32 * 32; }
 
 int true_residual(System& s, double* relres)
 {
@@ -753,20 +419,18 @@ int true_residual(System& s, double* relres)
 int solve_pcg64(System& s, bool jacobi, int maxiter, double tol, int* iters)
 {
     const int n = s.n_rows;
-    MSFEM_TRY(s.work64.alloc(4 * (size_t)n));
+    const size_t ld = padded(n);
+    MSFEM_TRY(s.work64.alloc(4 * ld));
     double* r = s.work64.p;
-    double* z = r + n;
-    double* p = z + n;
-    double* q = p + n;
+    double* p = r + ld;
+    double* q = p + ld;
     KState* S = s.kstate.p;
     // ff = (F, F); r = F - A X
     k_dot_self<double><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, s.F.p, s.partial.p, &S->ticket[1], &S->ff);
     MSFEM_TRY(residual64(s, s.X.p, s.F.p, r, &S->rr));
     k_set_limits<<<1, 32, 0, s.stream>>>(S, tol, maxiter, 0, kNoStall);
     s.launches += 3;
-    PcgVectors<double> v{s.X.p, r, jacobi ? z : r, p, q, s.dinv64.p};  // no preconditioner: z is r
-    MSFEM_TRY((jacobi ? pcg_run<double, true>(s, v, maxiter) : pcg_run<double, false>(s, v, maxiter)));
-    MSFEM_TRY(read_state(s));
+    MSFEM_TRY(pcg64_coop(s, jacobi, s.X.p, r, p, q, q + ld, maxiter));
     *iters = s.h_kstate->iter;
     return s.h_kstate->done == 1 ? MSFEM_OK : MSFEM_NOT_CONVERGED;
 }
@@ -793,11 +457,12 @@ int solve_refined(System& s, Inner inner, int maxiter, double tol, int* iters, i
     }
     if (inner != INNER_MINRES64) {
         // GMRES: d, r, then the (m+1) basis vectors and two gathered ones
-        MSFEM_TRY(s.work32.alloc((inner == INNER_GMRES32 ? (size_t)restart_m + 5 : 5) * (size_t)n));
+        const size_t ld = padded(n);
+        MSFEM_TRY(s.work32.alloc((inner == INNER_GMRES32 ? (size_t)restart_m + 5 : 5) * ld));
         d32 = s.work32.p;
-        r32 = d32 + n;
-        p32 = r32 + n;
-        q32 = p32 + n;
+        r32 = d32 + ld;
+        p32 = r32 + ld;
+        q32 = p32 + ld;
     }
     KState* S = s.kstate.p;
     DBuf<double>& rr_dev = s.sc_f64[1];
@@ -841,16 +506,12 @@ int solve_refined(System& s, Inner inner, int maxiter, double tol, int* iters, i
             k_scale_to32<<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, r64, rr_dev.p, s.dscale.p, r32, d32);
             s.launches += 1;
             if (inner == INNER_CG32) {
-                k_dot_self<float><<<kReduceBlocks, kVecThreads, 0, s.stream>>>(n, r32, s.partial.p, &S->ticket[1], &S->rr);
-                k_set_limits<<<1, 32, 0, s.stream>>>(S, tau, maxiter - total_inner, 1, kInnerStall);
-                s.launches += 2;
                 // d = x (from 0), r32 = the scaled right-hand side, then w, p, s
-                MSFEM_TRY(cg2_run(s, d32, r32, p32, q32, q32 + n, maxiter - total_inner));
-                MSFEM_TRY(read_state(s));
+                MSFEM_TRY(cg32_coop(s, d32, r32, p32, q32, q32 + padded(n), tau, maxiter - total_inner, kInnerStall));
                 it = s.h_kstate->iter;
                 if (s.h_kstate->breakdown) rc = MSFEM_ERR_NUMERIC;
             } else if (inner == INNER_GMRES32) {
-                float* V = r32 + n;
+                float* V = r32 + padded(n);
                 rc = gmres32_inner(s, restart_m, d32, r32, V, V + (size_t)(restart_m + 1) * n, maxiter - total_inner, tau,
                                    &it);
             } else {

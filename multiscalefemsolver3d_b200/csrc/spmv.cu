@@ -16,6 +16,8 @@
 // in column order.
 #include <cub/cub.cuh>
 
+#include <climits>
+
 #include "devutil.cuh"
 #include "internal.cuh"
 #include "spmv.cuh"
@@ -26,7 +28,8 @@ namespace {
 inline unsigned grid_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 // slice widths: entries per lane (scalar, rounded up to kChunk) or blocks per lane
-__global__ void k_slice_width(int n_rows, int n_slices, const int32_t* __restrict__ rp, int round_to, int64_t* w_out)
+__global__ void k_slice_width(int n_rows, int n_slices, const int32_t* __restrict__ rp, int round_to, int64_t* w_out,
+                              int* __restrict__ widest)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n_slices) return;
@@ -37,6 +40,42 @@ __global__ void k_slice_width(int n_rows, int n_slices, const int32_t* __restric
     if (lane == 0) {
         int w = (len + round_to - 1) / round_to * round_to;
         w_out[warp] = (int64_t)w * kSlice;
+        atomicMax(widest, w);
+    }
+}
+
+// lowest and highest column (node) of each slice
+__global__ void k_slice_span(int n_rows, int n_slices, const int32_t* __restrict__ rp, const int32_t* __restrict__ ncol,
+                             int2* __restrict__ span)
+{
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (warp >= n_slices) return;
+    const int row = warp * kSlice + lane;
+    int lo = min(row, n_rows - 1), hi = lo;  // padding entries name the row itself
+    if (row < n_rows)
+        for (int k = rp[row]; k < rp[row + 1]; k++) {
+            lo = min(lo, ncol[k]);
+            hi = max(hi, ncol[k]);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) span[warp] = make_int2(lo, hi);
+}
+
+// the widest span of G equal shares of the slices
+__global__ void k_share_span(int n_slices, int G, const int2* __restrict__ span, int* __restrict__ widest)
+{
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < G; c += gridDim.x * blockDim.x) {
+        const int s0 = (int)((int64_t)n_slices * c / G), s1 = (int)((int64_t)n_slices * (c + 1) / G);
+        int lo = INT_MAX, hi = -1;
+        for (int k = s0; k < s1; k++) {
+            lo = min(lo, span[k].x);
+            hi = max(hi, span[k].y);
+        }
+        if (hi >= lo) atomicMax(widest, hi - lo + 1);
     }
 }
 
@@ -49,7 +88,7 @@ __global__ void k_sell_pattern_scalar(int n_rows, const int32_t* __restrict__ rp
     const int64_t base = sp[slice];
     const int w = (int)((sp[slice + 1] - base) / kSlice);
     const int b = row < n_rows ? rp[row] : 0, len = row < n_rows ? rp[row + 1] - b : 0;
-    const int pad = row < n_rows ? row : 0;
+    const int pad = min(row, n_rows - 1);
     for (int k = 0; k < w; k++) {
         const int64_t pos = base + (int64_t)(k / kChunk) * (kSlice * kChunk) + lane * kChunk + (k % kChunk);
         col[pos] = k < len ? ncol[b + k] : pad;
@@ -104,7 +143,7 @@ __global__ void k_sell_pattern_block(int n_brows, const int32_t* __restrict__ rp
     const int64_t base = sp[slice];
     const int w = (int)((sp[slice + 1] - base) / kSlice);
     const int b = row < n_brows ? rp[row] : 0, len = row < n_brows ? rp[row + 1] - b : 0;
-    const int pad = row < n_brows ? row : 0;
+    const int pad = min(row, n_brows - 1);
     for (int k = 0; k < w; k++) col[base + (int64_t)k * kSlice + lane] = k < len ? ncol[b + k] : pad;
 }
 
@@ -265,8 +304,16 @@ int prepare_sell(System& s)
         MSFEM_TRY(w.alloc((size_t)S.n_slices + 1));
         MSFEM_TRY(S.slice_ptr.alloc((size_t)S.n_slices + 1));
         MSFEM_CK(cudaMemsetAsync(w.p + S.n_slices, 0, sizeof(int64_t), st));
+        DBuf<int> widest;
+        MSFEM_TRY(widest.alloc(2));
+        MSFEM_CK(cudaMemsetAsync(widest.p, 0, 2 * sizeof(int), st));
+        int sms = 0;
+        MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
+        MSFEM_TRY(S.span.alloc((size_t)S.n_slices));
+        k_slice_span<<<grid_for((int64_t)S.n_slices * 32, 256), 256, 0, st>>>(nbr, S.n_slices, s.nrp.p, s.ncol.p, S.span.p);
+        k_share_span<<<1, 256, 0, st>>>(S.n_slices, std::min(sms, S.n_slices), S.span.p, widest.p + 1);
         k_slice_width<<<grid_for((int64_t)S.n_slices * 32, 256), 256, 0, st>>>(nbr, S.n_slices, s.nrp.p,
-                                                                               s.bs == 1 ? kChunk : 1, w.p);
+                                                                               s.bs == 1 ? kChunk : 1, w.p, widest.p);
         MSFEM_CK(cudaGetLastError());
         size_t tmp_bytes = 0;
         DBuf<unsigned char> tmp;
@@ -275,7 +322,11 @@ int prepare_sell(System& s)
         MSFEM_CK(cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, w.p, S.slice_ptr.p, S.n_slices + 1, st));
         int64_t stored = 0;
         MSFEM_CK(cudaMemcpyAsync(&stored, S.slice_ptr.p + S.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        int wide[2] = {0, 0};
+        MSFEM_CK(cudaMemcpyAsync(wide, widest.p, sizeof(wide), cudaMemcpyDeviceToHost, st));
         MSFEM_CK(cudaStreamSynchronize(st));
+        S.max_width = wide[0];
+        S.max_span = wide[1];
         S.stored = stored;
         MSFEM_TRY(S.col.alloc((size_t)stored));
         const size_t nv = (size_t)stored * (s.bs == 1 ? 1 : 9);
@@ -335,13 +386,23 @@ int prepare_sell(System& s)
         s.zero_diag = h_bad != 0;  // only the Jacobi-preconditioned methods care; they check it
         s.total_launches += 2;
     }
-    if (S.fp32_col16 < 0) MSFEM_TRY(tune_fp32_columns(s));
     return MSFEM_OK;
+}
+
+int keep_share(const System& s, size_t width)
+{
+    int l2 = 0;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, s.device) != cudaSuccess) return 0;
+    const double bytes = (double)s.sell.stored * (s.bs == 1 ? width + (s.sell.col16.p ? 2 : 4) : 9 * width + 4);
+    if (bytes > 1.5 * l2) return 0;
+    return (int)std::min(1024.0, 1024.0 * 0.45 * l2 / std::max(bytes, 1.0));
 }
 
 template <class VT>
 SellView<VT> sell_view(System& s)
 {
+    // timed on the first FP32 product kernel of its own; the one-launch CG always takes the deltas
+    if (sizeof(VT) == 4 && s.sell.fp32_col16 < 0 && tune_fp32_columns(s) < 0) s.sell.fp32_col16 = 0;
     SellView<VT> v;
     v.n_slices = s.sell.n_slices;
     v.bs = s.bs;
