@@ -99,7 +99,8 @@ typedef struct {
     double ms_dirichlet;     /* device time of the last Dirichlet application                       */
     double ms_solve;         /* device time of the last solve                                       */
     double ms_spmv;          /* mean device time of one SpMV of the solve's working precision       */
-    int n_colors;            /* element colour classes used by the assembly                         */
+    int n_colors;            /* element classes the assembly launches one after the other: 1 (it gathers
+                                by rows), 0 for systems without a mesh                               */
     int kernel_launches;     /* kernels of this library launched by the last solve                  */
     int64_t total_launches;  /* kernels of this library launched on this handle since creation      */
 } msfem_stats;
@@ -111,7 +112,7 @@ int msfem_version(void);
  * (FEM/FEM_Grid.h:575-663, :3017-3102; :665-716, :3236-3287; Library/CSSD_Matrix.h:79-99):
  * uploads the mesh (nvtr = tets[4*n_tets], nvkat = material[n_tets], xyz[3*n_nodes]),
  * builds the node-level portrait (every pair of nodes of an element couples), the
- * element -> matrix-slot map and the element colouring, and allocates the zeroed
+ * row positions of every element's nodes, and allocates the zeroed
  * matrix, F and X.  kind = MSFEM_SCALAR (n rows = n_nodes) or MSFEM_ELASTIC
  * (n rows = 3*n_nodes, 3x3 blocks).  material may be NULL (all zero). */
 int msfem_system_create(int kind, int n_nodes, const double* xyz, int n_tets, const int32_t* tets,
@@ -143,7 +144,7 @@ int msfem_system_from_cssd(int n, const double* diag, const int64_t* down_ptr, c
 int msfem_xfem_system(int n_nodes, const double* xyz, int n_tets, const int32_t* tets, const double* sigma,
                       int n_cracks, const double* centre, const double* normal, const int32_t* crack_of_tet,
                       const int32_t* enr_dof, int n_dofs, msfem_system_t* out);
-/* n_rows, scalar nnz of the CSR export (diagonal included), element colour count */
+/* n_rows, scalar nnz of the CSR export (diagonal included), n_colors of msfem_stats */
 int msfem_system_info(msfem_system_t h, int* n_rows, int64_t* nnz, int* n_colors);
 int msfem_get_stats(msfem_system_t h, msfem_stats* out);
 /* the handle's CUDA stream (cudaStream_t) */

@@ -1,14 +1,23 @@
-// Coloured, deterministic element assembly into the node-level portrait.
+// Deterministic element assembly into the node-level portrait, one warp per row.
 //
 // The reference computes every element matrix in an OpenMP loop and then adds
 // them into CSSD_Matrix serially, element by element, finding each target entry
 // by a linear search of the row (FEM/FEM.h:1349-1384, CSSD_Matrix.h:307-363).
-// Here one launch per element colour class computes the element matrices and
-// adds them straight into the matrix through the precomputed element -> slot
-// map: elements of one colour share no node, so no two threads touch the same
-// entry, no atomics are needed and every entry receives its contributions in
-// the same (colour) order on every run.
+// Here a warp owns a node's row: its lanes form the geometry of the node's
+// elements (one each), then every lane owns a row entry and adds the
+// contributions of the elements that hold its column, in ascending element
+// order -- the reference's order, no atomics, one launch, the same bits on every run.
+//
+// What bounds it: the FP64 adds and the shuffles over a row's elements (24 in a Kuhn
+// grid); each element's geometry is formed four times, once per node, which is less
+// than the launches cost that it replaces: one per element colour (38 on a Kuhn grid),
+// each writing 16 entries per element back to memory, after a colouring whose 39 rounds
+// over all elements took nine tenths of the time to build a system.  Assembly at 20^3 /
+// 60^3 / 100^3, ms: elasticity 1.07 / 5.86 / 15.7 -> 0.055 / 0.70 / 3.1, scalar 0.42 / 0.63 / 2.3 ->
+// 0.043 / 0.43 / 1.9; building the system 3.2 / 13.4 / 53 -> 0.33 / 1.4 / 5.6.
 #include <cub/cub.cuh>
+
+#include <algorithm>
 
 #include "devutil.cuh"
 #include "element.cuh"
@@ -17,135 +26,151 @@
 namespace msfem {
 namespace {
 
-__device__ __forceinline__ void load_tet(const int32_t* __restrict__ tets, int e, int v[4])
-{
-    const int4 q = __ldg(reinterpret_cast<const int4*>(tets) + e);
-    v[0] = q.x;
-    v[1] = q.y;
-    v[2] = q.z;
-    v[3] = q.w;
-}
+enum RowKind { kScalar = 0, kScalar3 = 1, kElastic = 2, kTextbook = 3 };
 
-__device__ __forceinline__ void load_slots(const int32_t* __restrict__ eslot, int e, int s[16])
-{
-    const int4* p = reinterpret_cast<const int4*>(eslot) + 4 * (int64_t)e;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        int4 v = __ldg(p + q);
-        s[4 * q] = v.x;
-        s[4 * q + 1] = v.y;
-        s[4 * q + 2] = v.z;
-        s[4 * q + 3] = v.w;
-    }
-}
+struct RowMesh {
+    int n_nodes;
+    const int32_t* inc_ptr;
+    const int32_t* inc_elem;
+    const uint32_t* inc_slot;
+    const int32_t* nrp;
+    const int32_t* tets;
+    const double* xyz;
+    const int32_t* mat;
+};
 
-// FEM_Grid.h:103-152: K_IJ = sigma * grad(phi_I).grad(phi_J) * V (1-point rule, weight V)
-__global__ void k_assemble_scalar(int count, const int32_t* __restrict__ elems, const int32_t* __restrict__ tets,
-                                  const double* __restrict__ xyz, const int32_t* __restrict__ mat,
-                                  const double* __restrict__ sigma, int n_mat, const int32_t* __restrict__ eslot,
-                                  double* __restrict__ val, int* bad)
-{
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int e = elems[t];
-    const int m = mat ? mat[e] : 0;
-    if (m < 0 || m >= n_mat) {
-        atomicExch(bad, 1);
-        return;
-    }
-    int v[4], s[16];
-    load_tet(tets, e, v);
-    load_slots(eslot, e, s);
-    TetGeom G;
-    tet_geometry(xyz, v, G);
-    const double sv = sigma[m];
-#pragma unroll
-    for (int I = 0; I < 4; I++)
-#pragma unroll
-        for (int J = 0; J < 4; J++) {
-            double k = sv * (G.g[I][0] * G.g[J][0] + G.g[I][1] * G.g[J][1] + G.g[I][2] * G.g[J][2]) * G.vol;
-            val[s[4 * I + J]] += k;
-        }
-}
-
-// FEM_Grid.h:25-102, the three-coefficient element with the one-point rule (centroid, weight V):
-// A_IJ = V (S g_I.g_J + M / 16), F_I += V f / 4, with the element's coefficients S, M, f (the
-// reference's koef(elem, X) at the centroid).  Elements of one colour share no node, so the F
-// updates do not race.
-__global__ void k_assemble_scalar3(int count, const int32_t* __restrict__ elems, const int32_t* __restrict__ tets,
-                                   const double* __restrict__ xyz, const double* __restrict__ S,
-                                   const double* __restrict__ M, const double* __restrict__ f,
-                                   const int32_t* __restrict__ eslot, double* __restrict__ val, double* __restrict__ F)
-{
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int e = elems[t];
-    int v[4], sl[16];
-    load_tet(tets, e, v);
-    load_slots(eslot, e, sl);
-    TetGeom G;
-    tet_geometry(xyz, v, G);
-    const double se = S[e], m16 = M[e] / 16.0;
-#pragma unroll
-    for (int I = 0; I < 4; I++)
-#pragma unroll
-        for (int J = 0; J < 4; J++) {
-            const double k = se * (G.g[I][0] * G.g[J][0] + G.g[I][1] * G.g[J][1] + G.g[I][2] * G.g[J][2]) + m16;
-            val[sl[4 * I + J]] += k * G.vol;
-        }
-    const double fe = f[e] * G.vol / 4.0;
-#pragma unroll
-    for (int I = 0; I < 4; I++) F[v[I]] += fe;
-}
-
-// FEM_Grid.h:2125-2192.  The reference forms B_J^T D B_I (3x6 * 6x6 * 6x3) at
-// each of the 4 quadrature points; for the isotropic D of Domain.h:53-78 with
-// lambda = k*a and mu = k*b that product is, entry by entry,
+// kScalar (FEM_Grid.h:103-152, the one-point rule with weight V): A_IJ = V sigma g_I.g_J.
+// kScalar3 (FEM_Grid.h:25-102, three coefficients at the centroid): A_IJ = V (S g_I.g_J + M / 16),
+// F_I += V f / 4.
+// kElastic (FEM_Grid.h:2125-2192): the reference forms B_J^T D B_I (3x6 * 6x6 * 6x3) at each of the 4
+// quadrature points; for the isotropic D of Domain.h:53-78 with lambda = k*a and mu = k*b that product
+// is, entry by entry,
 //   A[I][J][a][b] = V * (lambda * gJ_a * gI_b + mu * gI_a * gJ_b + mu * delta_ab * gI.gJ)
-// (g = basis gradient), which also equals the reference's mirrored blocks
-// A[J][I] = A[I][J]^T, so all 16 blocks come from this one expression.
-// TEXTBOOK: the textbook orientation lambda gI_a gJ_b + mu gJ_a gI_b (the transpose of every
-// block), symmetric positive semi-definite; used to build preconditioners, not by the reference.
-template <bool TEXTBOOK>
-__global__ void k_assemble_elastic(int count, const int32_t* __restrict__ elems, const int32_t* __restrict__ tets,
-                                   const double* __restrict__ xyz, const int32_t* __restrict__ mat,
-                                   const double* __restrict__ lame /* [n_mat][2] */, int n_mat,
-                                   const int32_t* __restrict__ eslot, double* __restrict__ val, int* bad)
+// (g = basis gradient), which also equals the reference's mirrored blocks A[J][I] = A[I][J]^T, so all
+// 16 blocks come from this one expression.
+// kTextbook: the textbook orientation lambda gI_a gJ_b + mu gJ_a gI_b (the transpose of every block),
+// symmetric positive semi-definite; used to build preconditioners, not by the reference.
+// c0, c1, c2: kScalar sigma per material; kScalar3 S, M, f per element; elasticity lambda, mu per
+// material ([n_mat][2]).
+template <int KIND>
+__global__ void __launch_bounds__(128) k_assemble_rows(RowMesh G, const double* __restrict__ c0,
+                                                       const double* __restrict__ c1, const double* __restrict__ c2,
+                                                       int n_mat, double* __restrict__ val, double* __restrict__ F,
+                                                       int* __restrict__ bad)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int e = elems[t];
-    const int m = mat ? mat[e] : 0;
-    if (m < 0 || m >= n_mat) {
-        atomicExch(bad, 1);
-        return;
-    }
-    const double lam = lame[2 * m], mu = lame[2 * m + 1];
-    if (lam == 0.0 && mu == 0.0) return;  // E <= 0: the element contributes nothing (FEM/FEM.h:1355-1363)
-    int v[4], s[16];
-    load_tet(tets, e, v);
-    load_slots(eslot, e, s);
-    TetGeom G;
-    tet_geometry(xyz, v, G);
-    const double V = G.vol;
+    constexpr bool EL = KIND == kElastic || KIND == kTextbook;
+    constexpr int NQ = EL ? 15 : 5;  // per element: gradients, lambda, mu, V / the four entries, the load
+    constexpr int W = EL ? 9 : 1;
+    __shared__ double sh[4][NQ * 32];
+    const int lane = threadIdx.x & 31;
+    double* q = sh[threadIdx.x >> 5];
+    const int nw = gridDim.x * 4;
+    for (int node = blockIdx.x * 4 + (threadIdx.x >> 5); node < G.n_nodes; node += nw) {
+        const int b = G.inc_ptr[node], deg = G.inc_ptr[node + 1] - b;
+        const int row = G.nrp[node], len = G.nrp[node + 1] - row;
+        for (int s0 = 0; s0 < len || s0 == 0; s0 += 32) {  // 32 entries of the row at a time
+            double acc[W];
 #pragma unroll
-    for (int I = 0; I < 4; I++)
+            for (int k = 0; k < W; k++) acc[k] = 0.0;
+            double load = 0.0;
+            for (int e0 = 0; e0 < deg; e0 += 32) {
+                uint32_t slots = 0xffffffffu;  // no entry: the row is shorter than 255
+                int own = 0;
+                if (e0 + lane < deg) {
+                    const int e = G.inc_elem[b + e0 + lane];
+                    const int m = KIND == kScalar3 ? 0 : (G.mat ? G.mat[e] : 0);
+                    const bool known = KIND == kScalar3 || (m >= 0 && m < n_mat);
+                    if (!known) atomicExch(bad, 1);
+                    double lam = 0.0, mu = 0.0;
+                    if (EL && known) {
+                        lam = c0[2 * m];
+                        mu = c0[2 * m + 1];
+                    }
+                    // E <= 0: the element contributes nothing (FEM/FEM.h:1355-1363)
+                    if (known && (!EL || lam != 0.0 || mu != 0.0)) {
+                        const int4 t = __ldg(reinterpret_cast<const int4*>(G.tets) + e);
+                        const int v[4] = {t.x, t.y, t.z, t.w};
+                        own = node == v[0] ? 0 : node == v[1] ? 1 : node == v[2] ? 2 : 3;
+                        slots = G.inc_slot[b + e0 + lane];
+                        TetGeom T;
+                        tet_geometry(G.xyz, v, T);
+                        if constexpr (EL) {
 #pragma unroll
-        for (int J = 0; J < 4; J++) {
-            const double* gi = G.g[I];
-            const double* gj = G.g[J];
-            const double dd = mu * (gi[0] * gj[0] + gi[1] * gj[1] + gi[2] * gj[2]);
-            double* out = val + 9 * (int64_t)s[4 * I + J];
+                            for (int J = 0; J < 4; J++)
 #pragma unroll
-            for (int a = 0; a < 3; a++)
+                                for (int a = 0; a < 3; a++) q[(3 * J + a) * 32 + lane] = T.g[J][a];
+                            q[12 * 32 + lane] = lam;
+                            q[13 * 32 + lane] = mu;
+                            q[14 * 32 + lane] = T.vol;
+                        } else {
+                            double gi[3];
 #pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    double k = TEXTBOOK ? lam * gi[a] * gj[b] + mu * gj[a] * gi[b]
-                                        : lam * gj[a] * gi[b] + mu * gi[a] * gj[b];
-                    if (a == b) k += dd;
-                    out[3 * a + b] += V * k;
+                            for (int a = 0; a < 3; a++)
+                                gi[a] = own == 0 ? T.g[0][a] : own == 1 ? T.g[1][a] : own == 2 ? T.g[2][a] : T.g[3][a];
+                            const double k0 = KIND == kScalar ? c0[m] : c0[e], m16 = KIND == kScalar3 ? c1[e] / 16.0 : 0.0;
+#pragma unroll
+                            for (int J = 0; J < 4; J++) {
+                                double k = k0 * (gi[0] * T.g[J][0] + gi[1] * T.g[J][1] + gi[2] * T.g[J][2]);
+                                if (KIND == kScalar3) k += m16;
+                                q[J * 32 + lane] = k * T.vol;
+                            }
+                            if (KIND == kScalar3) q[4 * 32 + lane] = c2[e] * T.vol / 4.0;
+                        }
+                    }
                 }
+                __syncwarp();
+                const int n = min(32, deg - e0);
+                for (int e = 0; e < n; e++) {
+                    const uint32_t at = __shfl_sync(0xffffffffu, slots, e);
+                    const int I = EL ? __shfl_sync(0xffffffffu, own, e) : 0;
+                    if (KIND == kScalar3) load += q[4 * 32 + e];
+                    if (at == 0xffffffffu) continue;
+                    const uint32_t d = at ^ ((uint32_t)(s0 + lane) * 0x01010101u);
+                    const int J = (d & 0xffu) == 0 ? 0 : (d & 0xff00u) == 0 ? 1 : (d & 0xff0000u) == 0 ? 2 : (d >> 24) == 0 ? 3 : -1;
+                    if (J < 0) continue;
+                    if constexpr (EL) {
+                        double gi[3], gj[3];
+#pragma unroll
+                        for (int a = 0; a < 3; a++) {
+                            gi[a] = q[(3 * I + a) * 32 + e];
+                            gj[a] = q[(3 * J + a) * 32 + e];
+                        }
+                        const double lam = q[12 * 32 + e], mu = q[13 * 32 + e], V = q[14 * 32 + e];
+                        const double dd = mu * (gi[0] * gj[0] + gi[1] * gj[1] + gi[2] * gj[2]);
+#pragma unroll
+                        for (int a = 0; a < 3; a++)
+#pragma unroll
+                            for (int c = 0; c < 3; c++) {
+                                double k = KIND == kTextbook ? lam * gi[a] * gj[c] + mu * gj[a] * gi[c]
+                                                             : lam * gj[a] * gi[c] + mu * gi[a] * gj[c];
+                                if (a == c) k += dd;
+                                acc[3 * a + c] += V * k;
+                            }
+                    } else {
+                        acc[0] += q[J * 32 + e];
+                    }
+                }
+                __syncwarp();
+            }
+            if (s0 + lane < len) {
+                double* out = val + (int64_t)W * (row + s0 + lane);
+#pragma unroll
+                for (int k = 0; k < W; k++) out[k] += acc[k];
+            }
+            if (KIND == kScalar3 && s0 == 0 && lane == 0) F[node] += load;
         }
+    }
+}
+
+template <int KIND>
+int launch_rows(System& s, const double* c0, const double* c1, const double* c2, int n_mat, int* bad)
+{
+    const RowMesh G{s.n_nodes, s.inc_ptr.p, s.inc_elem.p, s.inc_slot.p, s.nrp.p, s.tets.p, s.xyz.p, s.mat.p};
+    const int blocks = (int)std::min<int64_t>(((int64_t)s.n_nodes + 3) / 4, 148 * 64);
+    k_assemble_rows<KIND><<<blocks, 128, 0, s.stream>>>(G, c0, c1, c2, n_mat, s.val.p, s.F.p, bad);
+    MSFEM_CK(cudaGetLastError());
+    s.total_launches += 1;
+    return MSFEM_OK;
 }
 
 // ---- traction: per (face, vertex) contribution, then a per-node sum in face order
@@ -237,15 +262,7 @@ int assemble_scalar(System& s, const double* sigma, int n_mat)
     MSFEM_CK(cudaEventRecord(s.ev0, s.stream));
     MSFEM_CK(cudaMemcpyAsync(d_sig.p, sigma, sizeof(double) * n_mat, cudaMemcpyHostToDevice, s.stream));
     MSFEM_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), s.stream));
-    const int nc = (int)s.color_off.size() - 1;
-    for (int c = 0; c < nc; c++) {
-        int cnt = s.color_off[c + 1] - s.color_off[c];
-        k_assemble_scalar<<<grid_for(cnt, 128), 128, 0, s.stream>>>(cnt, s.color_elems.p + s.color_off[c], s.tets.p,
-                                                                    s.xyz.p, s.mat.p, d_sig.p, n_mat, s.eslot.p,
-                                                                    s.val.p, bad.p);
-    }
-    MSFEM_CK(cudaGetLastError());
-    s.total_launches += nc;
+    MSFEM_TRY(launch_rows<kScalar>(s, d_sig.p, nullptr, nullptr, n_mat, bad.p));
     return finish_assembly(s, bad);
 }
 
@@ -270,15 +287,7 @@ int assemble_scalar3(System& s, const double* S, const double* M, const double* 
     MSFEM_CK(cudaMemcpyAsync(coef.p + ne, M, sizeof(double) * ne, kind, s.stream));
     MSFEM_CK(cudaMemcpyAsync(coef.p + 2 * ne, f, sizeof(double) * ne, kind, s.stream));
     MSFEM_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), s.stream));
-    const int nc = (int)s.color_off.size() - 1;
-    for (int c = 0; c < nc; c++) {
-        int cnt = s.color_off[c + 1] - s.color_off[c];
-        k_assemble_scalar3<<<grid_for(cnt, 128), 128, 0, s.stream>>>(cnt, s.color_elems.p + s.color_off[c], s.tets.p,
-                                                                     s.xyz.p, coef.p, coef.p + ne, coef.p + 2 * ne,
-                                                                     s.eslot.p, s.val.p, s.F.p);
-    }
-    MSFEM_CK(cudaGetLastError());
-    s.total_launches += nc;
+    MSFEM_TRY(launch_rows<kScalar3>(s, coef.p, coef.p + ne, coef.p + 2 * ne, 0, bad.p));
     return finish_assembly(s, bad);
 }
 
@@ -320,16 +329,8 @@ int assemble_elastic(System& s, const double* E, const double* nu, int n_mat, bo
     MSFEM_CK(cudaEventRecord(s.ev0, s.stream));
     MSFEM_CK(cudaMemcpyAsync(d_lame.p, lame.data(), sizeof(double) * 2 * n_mat, cudaMemcpyHostToDevice, s.stream));
     MSFEM_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), s.stream));
-    const int nc = (int)s.color_off.size() - 1;
-    for (int c = 0; c < nc; c++) {
-        int cnt = s.color_off[c + 1] - s.color_off[c];
-        auto kern = textbook ? k_assemble_elastic<true> : k_assemble_elastic<false>;
-        kern<<<grid_for(cnt, 128), 128, 0, s.stream>>>(cnt, s.color_elems.p + s.color_off[c], s.tets.p,
-                                                                     s.xyz.p, s.mat.p, d_lame.p, n_mat, s.eslot.p,
-                                                                     s.val.p, bad.p);
-    }
-    MSFEM_CK(cudaGetLastError());
-    s.total_launches += nc;
+    MSFEM_TRY((textbook ? launch_rows<kTextbook>(s, d_lame.p, nullptr, nullptr, n_mat, bad.p)
+                        : launch_rows<kElastic>(s, d_lame.p, nullptr, nullptr, n_mat, bad.p)));
     // a matrix-free operator (kuhn.cu) can stand for the values only while they hold one assembly
     if (s.elastic_form == 0) {
         s.elastic_form = textbook ? 2 : 1;

@@ -130,7 +130,6 @@ int system_adopt_csr(int n, DBuf<int32_t>& row_ptr, DBuf<int32_t>& col, DBuf<dou
     s->n_tets = 0;
     s->n_rows = n;
     s->nnzb = nnz;
-    s->color_off = {0};
     MSFEM_CK(cudaGetDevice(&s->device));
     MSFEM_CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     MSFEM_CK(cudaEventCreate(&s->ev0));
@@ -287,7 +286,6 @@ int msfem_system_from_cssd(int n, const double* diag, const int64_t* down_ptr, c
     s->n_tets = 0;
     s->n_rows = n;
     s->nnzb = (int64_t)col.size();
-    s->color_off = {0};
     MSFEM_CK(cudaGetDevice(&s->device));
     MSFEM_CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     MSFEM_CK(cudaEventCreate(&s->ev0));
@@ -334,7 +332,7 @@ int msfem_system_info(msfem_system_t h, int* n_rows, int64_t* nnz, int* n_colors
     System* s = as_sys(h);
     if (n_rows) *n_rows = s->n_rows;
     if (nnz) *nnz = s->nnzb * s->bs * s->bs;
-    if (n_colors) *n_colors = (int)s->color_off.size() - 1;
+    if (n_colors) *n_colors = s->stats.n_colors;
     return MSFEM_OK;
 }
 

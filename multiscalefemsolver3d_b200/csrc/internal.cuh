@@ -126,11 +126,8 @@ struct System {
     // node-level portrait, diagonal included, rows sorted
     DBuf<int32_t> nrp, ncol;
     int64_t nnzb = 0;
-    // element (e, I, J) -> node-portrait slot, e*16 + 4*I + J
-    DBuf<int32_t> eslot;
-    // element colouring: elements listed colour by colour
-    DBuf<int32_t> color_elems;
-    std::vector<int> color_off;  // host copy, size n_colors + 1
+    // per incidence (same order as inc_elem): the positions of the element's nodes in the node's row
+    DBuf<uint32_t> inc_slot;
 
     // values: scalar val[slot]; elasticity val[9*slot + 3*a + b]
     DBuf<double> val;

@@ -1,7 +1,7 @@
 // Mesh topology on the GPU: node -> element incidence, the node-level portrait
-// (the reference's CreationPortrait, FEM/FEM_Grid.h:665-716 and :3236-3287),
-// the element -> matrix-slot map used by the scatter, and the element colouring
-// that makes the scatter race-free and deterministic.
+// (the reference's CreationPortrait, FEM/FEM_Grid.h:665-716 and :3236-3287), and for
+// every incidence the positions of the element's four nodes in the node's row,
+// which the assembly (one warp per row, assemble.cu) gathers by.
 #include <cub/cub.cuh>
 
 #include <climits>
@@ -53,14 +53,17 @@ __global__ void k_sort_incidence(int n_nodes, const int32_t* __restrict__ ptr, i
 
 // One warp per node row: gather the nodes of all incident elements (self
 // included) into shared memory, bitonic-sort them, drop duplicates.  Pass 0
-// stores the unique count, pass 1 writes the sorted columns.
+// stores the unique count, pass 1 writes the sorted columns and, per incidence,
+// the row positions of the element's nodes in four bytes (a row has at most
+// kMaxCandidates - kMaxCandidates / 4 + 1 < 255 entries).
 template <int PASS>
 __global__ void k_portrait_rows(int n_nodes, const int32_t* __restrict__ tets, const int32_t* __restrict__ inc_ptr,
                                 const int32_t* __restrict__ inc, int32_t* count, const int32_t* __restrict__ rp,
-                                int32_t* col, int* overflow)
+                                int32_t* col, uint32_t* inc_slot, int* overflow)
 {
     constexpr int WPB = 4;
     __shared__ int buf[WPB][kMaxCandidates];
+    __shared__ int uniq[PASS ? WPB : 1][PASS ? kMaxCandidates : 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int row = blockIdx.x * WPB + w;
     if (row >= n_nodes) return;
@@ -101,139 +104,33 @@ __global__ void k_portrait_rows(int n_nodes, const int32_t* __restrict__ tets, c
         int v = s[i];
         bool keep = (v != INT_MAX) && (i == 0 || s[i - 1] != v);
         unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (PASS && keep) col[out0 + total + __popc(m & ((1u << lane) - 1u))] = v;
+        if (PASS && keep) {
+            const int at = total + __popc(m & ((1u << lane) - 1u));
+            col[out0 + at] = v;
+            uniq[w][at] = v;
+        }
         total += __popc(m);
     }
     if (!PASS && lane == 0) count[row] = total;
-}
-
-__device__ __forceinline__ int find_slot(const int32_t* __restrict__ col, int lo, int hi, int c)
-{
-    hi -= 1;
-    while (lo <= hi) {
-        int mid = (lo + hi) >> 1;
-        int v = col[mid];
-        if (v == c) return mid;
-        if (v < c) lo = mid + 1;
-        else hi = mid - 1;
-    }
-    return -1;
-}
-
-__global__ void k_element_slots(int n_tets, const int32_t* __restrict__ tets, const int32_t* __restrict__ rp,
-                                const int32_t* __restrict__ col, int32_t* eslot, int* bad)
-{
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_tets) return;
-    int v[4];
+    if (PASS) {
+        __syncwarp();
+        for (int i = lane; i < deg; i += 32) {
+            const int4 t = reinterpret_cast<const int4*>(tets)[inc[b + i]];
+            const int node[4] = {t.x, t.y, t.z, t.w};
+            uint32_t packed = 0;
 #pragma unroll
-    for (int a = 0; a < 4; a++) v[a] = tets[4 * (int64_t)e + a];
-#pragma unroll
-    for (int I = 0; I < 4; I++)
-#pragma unroll
-        for (int J = 0; J < 4; J++) {
-            int s = find_slot(col, rp[v[I]], rp[v[I] + 1], v[J]);
-            if (s < 0) atomicExch(bad, 1);
-            eslot[16 * (int64_t)e + 4 * I + J] = s;
-        }
-}
-
-// Speculative greedy colouring of the element conflict graph (elements
-// conflict when they share a node), deterministic by construction:
-//  1. every uncoloured element proposes the smallest colour that none of its
-//     already-coloured neighbours holds (reads only colours committed in
-//     earlier rounds);
-//  2. among neighbours that proposed the same colour in this round, the one
-//     with the highest priority (hash of the id, ties by id) keeps it;
-//  3. winners are committed, losers try again in the next round.
-// Each kernel only reads arrays that no thread of the same kernel writes, so
-// the colouring -- and with it the order in which the assembly adds element
-// contributions -- is identical on every run.
-constexpr int kMaxColors = 256;
-
-__global__ void k_color_propose(int n_tets, const int32_t* __restrict__ tets, const int32_t* __restrict__ inc_ptr,
-                                const int32_t* __restrict__ inc, const int32_t* __restrict__ color,
-                                int32_t* __restrict__ tent, int* overflow)
-{
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_tets) return;
-    if (color[e] >= 0) {
-        tent[e] = -1;
-        return;
-    }
-    unsigned used[kMaxColors / 32];
-#pragma unroll
-    for (int w = 0; w < kMaxColors / 32; w++) used[w] = 0u;
-    for (int a = 0; a < 4; a++) {
-        const int v = tets[4 * (int64_t)e + a];
-        for (int k = inc_ptr[v]; k < inc_ptr[v + 1]; k++) {
-            const int c = color[inc[k]];
-            if (c >= 0) used[c >> 5] |= 1u << (c & 31);
-        }
-    }
-    int pick = -1;
-#pragma unroll
-    for (int w = 0; w < kMaxColors / 32; w++)
-        if (pick < 0 && used[w] != 0xffffffffu) pick = 32 * w + __ffs(~used[w]) - 1;
-    if (pick < 0) atomicExch(overflow, 1);
-    tent[e] = pick;
-}
-
-__global__ void k_color_resolve(int n_tets, const int32_t* __restrict__ tets, const int32_t* __restrict__ inc_ptr,
-                                const int32_t* __restrict__ inc, const int32_t* __restrict__ tent,
-                                int32_t* __restrict__ win)
-{
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_tets) return;
-    const int c = tent[e];
-    if (c < 0) {
-        win[e] = 0;
-        return;
-    }
-    const unsigned pe = hash32((unsigned)e);
-    bool best = true;
-    for (int a = 0; a < 4 && best; a++) {
-        const int v = tets[4 * (int64_t)e + a];
-        for (int k = inc_ptr[v]; k < inc_ptr[v + 1]; k++) {
-            const int f = inc[k];
-            if (f == e || tent[f] != c) continue;
-            const unsigned pf = hash32((unsigned)f);
-            if (pf > pe || (pf == pe && f > e)) {
-                best = false;
-                break;
+            for (int a = 0; a < 4; a++) {
+                int lo = 0, hi = total - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (uniq[w][mid] < node[a]) lo = mid + 1;
+                    else hi = mid;
+                }
+                packed |= (uint32_t)lo << (8 * a);
             }
+            inc_slot[b + i] = packed;
         }
     }
-    win[e] = best ? 1 : 0;
-}
-
-__global__ void k_color_commit(int n_tets, const int32_t* __restrict__ tent, const int32_t* __restrict__ win,
-                               int32_t* __restrict__ color, unsigned int* remaining)
-{
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_tets) return;
-    if (win[e]) color[e] = tent[e];
-    else if (color[e] < 0) atomicAdd(remaining, 1u);
-}
-
-// off[c] = first position of colour c in the sorted key array
-__global__ void k_color_starts(int n, const int32_t* __restrict__ keys, int32_t* off)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (i == 0 || keys[i] != keys[i - 1]) off[keys[i]] = i;
-}
-
-__global__ void k_max(int n, const int32_t* __restrict__ a, int32_t* mx)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) atomicMax(mx, a[i]);
-}
-
-__global__ void k_iota(int n, int32_t* a)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = i;
 }
 
 inline unsigned grid_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
@@ -244,7 +141,7 @@ int build_topology(System& s)
 {
     cudaStream_t st = s.stream;
     const int N = s.n_nodes, E = s.n_tets;
-    DBuf<int> flags;  // [0] bad node id, [1] overflow, [2] bad slot, [3] uncoloured count, [4] max colour
+    DBuf<int> flags;  // [0] bad node id, [1] overflow
     MSFEM_TRY(flags.alloc(8));
     MSFEM_CK(cudaMemsetAsync(flags.p, 0, 8 * sizeof(int), st));
 
@@ -277,7 +174,7 @@ int build_topology(System& s)
     // ---- node-level portrait
     MSFEM_TRY(s.nrp.alloc((size_t)N + 1));
     k_portrait_rows<0><<<grid_for(N, 4), 128, 0, st>>>(N, s.tets.p, s.inc_ptr.p, s.inc_elem.p, cnt.p, nullptr,
-                                                       nullptr, flags.p + 1);
+                                                       nullptr, nullptr, flags.p + 1);
     MSFEM_CK(cudaGetLastError());
     MSFEM_CK(cudaMemsetAsync(cnt.p + N, 0, sizeof(int32_t), st));
     tmp_bytes = 0;
@@ -295,97 +192,15 @@ int build_topology(System& s)
     }
     s.nnzb = nnzb;
     MSFEM_TRY(s.ncol.alloc((size_t)nnzb));
+    MSFEM_TRY(s.inc_slot.alloc((size_t)E * 4));
     k_portrait_rows<1><<<grid_for(N, 4), 128, 0, st>>>(N, s.tets.p, s.inc_ptr.p, s.inc_elem.p, nullptr, s.nrp.p,
-                                                       s.ncol.p, flags.p + 1);
+                                                       s.ncol.p, s.inc_slot.p, flags.p + 1);
     MSFEM_CK(cudaGetLastError());
-
-    // ---- element -> slot map
-    MSFEM_TRY(s.eslot.alloc((size_t)E * 16));
-    k_element_slots<<<grid_for(E, 128), 128, 0, st>>>(E, s.tets.p, s.nrp.p, s.ncol.p, s.eslot.p, flags.p + 2);
-    MSFEM_CK(cudaGetLastError());
-
-    // ---- colouring
-    DBuf<int32_t> color, tent, win;
-    MSFEM_TRY(color.alloc((size_t)E));
-    MSFEM_TRY(tent.alloc((size_t)E));
-    MSFEM_TRY(win.alloc((size_t)E));
-    MSFEM_CK(cudaMemsetAsync(color.p, 0xff, sizeof(int32_t) * (size_t)E, st));
-    unsigned int* remaining = reinterpret_cast<unsigned int*>(flags.p + 3);
-    int rounds = 0;
-    for (;;) {
-        if (rounds >= 1024) {
-            set_error("element colouring did not finish in 1024 rounds");
-            return MSFEM_ERR_LIMIT;
-        }
-        MSFEM_CK(cudaMemsetAsync(remaining, 0, sizeof(unsigned int), st));
-        k_color_propose<<<grid_for(E, 256), 256, 0, st>>>(E, s.tets.p, s.inc_ptr.p, s.inc_elem.p, color.p, tent.p,
-                                                          flags.p + 1);
-        k_color_resolve<<<grid_for(E, 256), 256, 0, st>>>(E, s.tets.p, s.inc_ptr.p, s.inc_elem.p, tent.p, win.p);
-        k_color_commit<<<grid_for(E, 256), 256, 0, st>>>(E, tent.p, win.p, color.p, remaining);
-        MSFEM_CK(cudaGetLastError());
-        rounds++;
-        unsigned int h_rem = 0;
-        MSFEM_CK(cudaMemcpyAsync(&h_rem, remaining, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-        MSFEM_CK(cudaMemcpyAsync(h_flags, flags.p, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
-        MSFEM_CK(cudaStreamSynchronize(st));
-        if (h_flags[1]) {
-            set_error("element colouring needs more than %d colours", kMaxColors);
-            return MSFEM_ERR_LIMIT;
-        }
-        if (h_rem == 0) break;
-    }
-    int n_colors = 0;
-    {
-        // number of colours = 1 + max colour
-        int32_t* mx = flags.p + 4;
-        MSFEM_CK(cudaMemsetAsync(mx, 0, sizeof(int32_t), st));
-        k_max<<<grid_for(E, 256), 256, 0, st>>>(E, color.p, mx);
-        int32_t h_mx = 0;
-        MSFEM_CK(cudaMemcpyAsync(&h_mx, mx, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        MSFEM_CK(cudaStreamSynchronize(st));
-        n_colors = h_mx + 1;
-        MSFEM_CK(cudaMemsetAsync(mx, 0, sizeof(int32_t), st));
-    }
-    // elements grouped by colour, ascending element id inside a colour (stable radix sort)
-    DBuf<int32_t> ids, keys_out;
-    MSFEM_TRY(ids.alloc((size_t)E));
-    MSFEM_TRY(keys_out.alloc((size_t)E));
-    MSFEM_TRY(s.color_elems.alloc((size_t)E));
-    k_iota<<<grid_for(E, 256), 256, 0, st>>>(E, ids.p);
-    int end_bit = 1;
-    while ((1 << end_bit) <= n_colors) end_bit++;
-    tmp_bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, color.p, keys_out.p, ids.p, s.color_elems.p, E, 0, end_bit, st);
-    MSFEM_TRY(tmp.alloc(tmp_bytes + 1));
-    MSFEM_CK(cub::DeviceRadixSort::SortPairs(tmp.p, tmp_bytes, color.p, keys_out.p, ids.p, s.color_elems.p, E, 0,
-                                             end_bit, st));
-    // greedy colours are dense: every colour below the maximum is used
-    DBuf<int32_t> starts;
-    MSFEM_TRY(starts.alloc((size_t)n_colors));
-    k_color_starts<<<grid_for(E, 256), 256, 0, st>>>(E, keys_out.p, starts.p);
-    MSFEM_CK(cudaGetLastError());
-    s.color_off.assign(n_colors + 1, 0);
-    MSFEM_CK(cudaMemcpyAsync(s.color_off.data(), starts.p, sizeof(int32_t) * n_colors, cudaMemcpyDeviceToHost, st));
-    MSFEM_CK(cudaMemcpyAsync(h_flags, flags.p, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
     MSFEM_CK(cudaStreamSynchronize(st));
-    s.color_off[n_colors] = E;
-    starts.release();
-    if (h_flags[2]) {
-        set_error("element slot lookup failed (inconsistent portrait)");
-        return MSFEM_ERR_STATE;
-    }
-    s.stats.n_colors = n_colors;
-    // incidence count/fill/sort, portrait count/fill, slots, max, iota, colour starts, 3 launches per round
-    s.total_launches += 9 + 3 * rounds;
+    s.stats.n_colors = 1;  // the assembly is one launch over the rows
+    // incidence count / fill / sort, portrait count / fill
+    s.total_launches += 5;
 
-    cnt.release();
-    tmp.release();
-    flags.release();
-    color.release();
-    tent.release();
-    win.release();
-    ids.release();
-    keys_out.release();
     return MSFEM_OK;
 }
 

@@ -160,7 +160,6 @@ extern "C" int msfem_xfem_system(int n_nodes, const double* xyz, int n_tets, con
     s->n_nodes = n_dofs;
     s->n_tets = 0;
     s->n_rows = n_dofs;
-    s->color_off = {0};
     MSFEM_CK(cudaGetDevice(&s->device));
     MSFEM_CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     MSFEM_CK(cudaEventCreate(&s->ev0));
