@@ -7,6 +7,32 @@
 
 namespace msfem {
 
+// Programmatic dependent launch (a chain of short kernels): a kernel launched with launch_chained may
+// start while its predecessor in the stream still runs.  chain_next lets the successor start as soon
+// as every block of this kernel is resident; chain_wait holds until the predecessor has completed and
+// its writes are visible, and comes before the first access to anything an earlier kernel of the
+// chain reads or writes; what was complete before the chain began may be read ahead of it.  Every block
+// waits (or has nothing to do), so that a kernel's completion implies that of all before it.  In a
+// kernel launched the plain way both do nothing.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll

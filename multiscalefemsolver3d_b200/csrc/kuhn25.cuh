@@ -23,6 +23,7 @@
 
 #include <cstdint>
 
+#include "devutil.cuh"
 #include "kuhn.cuh"
 
 namespace msfem {
@@ -194,7 +195,6 @@ template <int FORM, bool ISO, bool SC, class T, int TX, int TY, int MINB, class 
 __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_z(KzArgs<T> A, Epi epi)
 {
     using L = KzLayout<T, TX, TY, Epi::NE, SC>;
-    if (epi.skip()) return;
     extern __shared__ __align__(128) unsigned char kz_smem[];
     const KuhnView<T>& K = A.K;
     T* U = reinterpret_cast<T*>(kz_smem + L::U_OFF);
@@ -263,6 +263,8 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_z(KzArgs<T> A, Epi epi)
     // prologue: stages first .. first+2 in flight.  A wait's outcome is made block-wide at the
     // next barrier (__syncthreads_and), so every thread takes the same path.
     const KzCopy cp = kz_copy_of<L>(K, i0, j0);
+    chain_wait();  // everything above reads only what the operator keeps
+    if (epi.skip()) return;
     const int64_t Q = (int64_t)K.nx * K.ny;
     kz_issue<L>(A, cp, P, Q, first, stage_of(first), bar0 + 8 * slot(first));
     kz_issue<L>(A, cp, P, Q, first + 1, stage_of(first + 1), bar0 + 8 * slot(first + 1));
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_z(KzArgs<T> A, Epi epi)
     const int64_t g0 = gi + (int64_t)nnx * gj;
     const int wrow = gi_lo + nnx * gj;
     for (int kz = first; kz < k1; kz++) {
+        if (kz == k1 - 1) chain_next();  // earlier, the successor's blocks would take the SM's memory
         // stage kz+1 (issued two steps ago): wait, convert; the barrier then also frees stage kz-1's
         // ring slot (every thread is past step kz-1) for stage kz+3
         ok = kz_wait(bar0 + 8 * slot(kz + 1), parity(kz + 1)) && ok;
@@ -417,7 +420,6 @@ template <int FORM, bool ISO, class T, int TX, int TY, int MINB, class Epi>
 __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_zp(KzArgs<T> A, Epi epi)
 {
     using L = KzpLayout<T, TX, TY, Epi::NE>;
-    if (epi.skip()) return;
     extern __shared__ __align__(128) unsigned char kz_smem[];
     const KuhnView<T>& K = A.K;
     T* Bc = reinterpret_cast<T*>(kz_smem + L::B_OFF);
@@ -452,11 +454,17 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_zp(KzArgs<T> A, Epi epi)
     const int Qm2 = (int)(((int64_t)K.nx * K.ny) & 1);
     // prologue: stages first .. first+RING-2 in flight
     const KzCopy cp = kz_copy_of<L>(K, i0, j0);
+    chain_wait();  // everything above reads only what the operator keeps
+    const bool skip = epi.skip();  // in flight with the first copies
     const int64_t Q = (int64_t)K.nx * K.ny;
     int issued = first - 1;
     for (int layer = first; layer <= first + L::RING - 2 && layer <= k1; layer++) {
         kz_issue<L>(A, cp, P, Q, layer, stage_of(layer), bar0 + 8 * slot(layer));
         issued = layer;
+    }
+    if (skip) {  // the copies land before the block leaves
+        for (int layer = first; layer <= issued; layer++) kz_wait(bar0 + 8 * slot(layer), parity(layer));
+        return;
     }
     int landed = first - 1;
     bool ok = kz_wait(bar0 + 8 * slot(first), parity(first));
@@ -474,6 +482,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_zp(KzArgs<T> A, Epi epi)
     const int64_t g0 = gi + (int64_t)nnx * gj;
     const int wrow = gi_lo + nnx * gj;
     for (int kz = first; kz < k1; kz++) {
+        if (kz == k1 - 1) chain_next();  // earlier, the successor's blocks would take the SM's memory
         // stage kz+1 (the slab's top layer)
         ok = kz_wait(bar0 + 8 * slot(kz + 1), parity(kz + 1)) && ok;
         // the epilogue's per-node vectors, loaded now so the loads overlap the hexahedron

@@ -71,11 +71,7 @@ struct KzKernel {
                 A.n_seg = segs;
             }
         }
-        if (K.iso)
-            kernel_iso<<<tiles * A.n_seg, L::THREADS, L::smem, st>>>(A, epi);
-        else
-            kernel_aniso<<<tiles * A.n_seg, L::THREADS, L::smem, st>>>(A, epi);
-        return cudaGetLastError();
+        return launch_chained(K.iso ? kernel_iso : kernel_aniso, tiles * A.n_seg, L::THREADS, L::smem, st, A, epi);
     }
 };
 
@@ -138,11 +134,7 @@ struct KzpKernel {
                 A.n_seg = segs;
             }
         }
-        if (K.iso)
-            kernel_iso<<<tiles * A.n_seg, L::THREADS, L::smem, st>>>(A, epi);
-        else
-            kernel_aniso<<<tiles * A.n_seg, L::THREADS, L::smem, st>>>(A, epi);
-        return cudaGetLastError();
+        return launch_chained(K.iso ? kernel_iso : kernel_aniso, tiles * A.n_seg, L::THREADS, L::smem, st, A, epi);
     }
 };
 

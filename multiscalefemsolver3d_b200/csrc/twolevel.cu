@@ -415,7 +415,6 @@ __global__ void __launch_bounds__(256) k_tl_symv(int nb, int n_blocks, const int
                                                  const float* __restrict__ P, const float* __restrict__ x,
                                                  float* __restrict__ part, const TlState* S)
 {
-    if (S->done) return;
     __shared__ float colp[8][kSymB];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int cq = t & 15, r0 = t >> 4;
@@ -426,6 +425,8 @@ __global__ void __launch_bounds__(256) k_tl_symv(int nb, int n_blocks, const int
 #pragma unroll
         for (int k = 0; k < 4; k++) an[k] = __ldcs(blk + t + 256 * k);
     }
+    chain_wait();  // the matrix blocks above are constant
+    if (S->done) return;
     for (int b = blockIdx.x; b < n_blocks; b += gridDim.x) {
         const int I = blocks[b].x, J = blocks[b].y;
 #pragma unroll
@@ -471,12 +472,15 @@ __global__ void __launch_bounds__(256) k_tl_symv(int nb, int n_blocks, const int
         }
         __syncthreads();
     }
+    chain_next();
 }
 
 // y[i] = sum over block columns K of part[i / 64][K][i % 64], K ascending
 __global__ void k_tl_symv_sum(int n_pad, int nb, const float* __restrict__ part, float* __restrict__ y,
                               const TlState* S)
 {
+    chain_next();
+    chain_wait();
     if (S->done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
@@ -489,18 +493,23 @@ __global__ void k_tl_symv_sum(int n_pad, int nb, const float* __restrict__ part,
 
 // ---- preconditioner application kernels (FP32)
 
+// A block per cell, one pass over its nodes: a serial chain of loads per thread, so 256 threads (40^3,
+// an iteration: 136.3 us with 128, 134.9 with 256, 135.5 with 512; 128^3: 1536, 1535, 1556)
+constexpr int kRestrictThreads = 256;
+
 // per cell: restriction partials over its owned nodes, cpart[c][v a] = sum psi_hat[g][v a] q[g a],
 // q = r (scaled FP32 system) or s r (FP64 in the original unknowns, s = D^-1/2);
 // with `lanczos`, r is first formed as r_new = z - (alfa / beta) r2 and written over `out`
 template <class VT>
-__global__ void __launch_bounds__(128) k_tl_restrict(const int32_t* __restrict__ own_ptr, const int32_t* __restrict__ own,
-                                                     const float* __restrict__ psi_hat, const VT* __restrict__ z,
-                                                     const VT* __restrict__ r2, VT* __restrict__ out,
-                                                     float* __restrict__ cpart, const double* __restrict__ s,
-                                                     const TlState* S, int lanczos)
+__global__ void __launch_bounds__(kRestrictThreads)
+    k_tl_restrict(const int32_t* __restrict__ own_ptr, const int32_t* __restrict__ own,
+                  const float* __restrict__ psi_hat, const VT* __restrict__ z, const VT* __restrict__ r2,
+                  VT* __restrict__ out, float* __restrict__ cpart, const double* __restrict__ s, const TlState* S,
+                  int lanczos)
 {
+    chain_wait();
     if (S->done) return;
-    __shared__ VT red[4][24];
+    __shared__ VT red[kRestrictThreads / 32][24];
     const int c = blockIdx.x;
     const VT coef = lanczos ? (VT)(S->alfa / S->beta) : (VT)0;
     VT acc[24];
@@ -551,6 +560,8 @@ __global__ void __launch_bounds__(128) k_tl_restrict(const int32_t* __restrict__
 __global__ void k_tl_gather(int n_cf, const int32_t* __restrict__ dptr, const int32_t* __restrict__ dent,
                             const float* __restrict__ cpart, float* __restrict__ rc, const TlState* S)
 {
+    chain_next();
+    chain_wait();
     if (S->done) return;
     for (int d = blockIdx.x * blockDim.x + threadIdx.x; d < n_cf; d += gridDim.x * blockDim.x) {
         float s = 0.0f;
@@ -695,8 +706,9 @@ __global__ void __launch_bounds__(256) k_tl_spmv(SellView<VT> A, const VT* __res
 template <class VT>
 __global__ void __launch_bounds__(kVecThreads) k_tl_update(int n, const VT* __restrict__ v, VT* __restrict__ w1,
                                                           const VT* __restrict__ w2, VT* __restrict__ x,
-                                                          const TlState* S)
+                                                          TlState* S)
 {
+    chain_wait();
     if (S->done && S->applied == S->iter) return;
     if (S->done == 3) return;
     const VT oe = (VT)S->oldeps, de = (VT)S->delta, dn = (VT)S->denom, ph = (VT)S->phi;
@@ -705,11 +717,10 @@ __global__ void __launch_bounds__(kVecThreads) k_tl_update(int n, const VT* __re
         w1[i] = w;
         x[i] += ph * w;
     }
-}
-
-__global__ void k_tl_applied(TlState* S)
-{
-    if (S->done) S->applied = S->iter;
+    if (S->done && arrive_last(&S->ticket[3]) && threadIdx.x == 0) {
+        S->applied = S->iter;
+        S->ticket[3] = 0;
+    }
 }
 
 // rhs of the inner solve: b = S r / ||S r|| (scaled FP32 system) or r / ||r|| (FP64), and the
@@ -880,6 +891,7 @@ __global__ void __launch_bounds__(kVecThreads) k_mg_in(int n, const double* __re
                                                       const TlState* S, int lanczos, const float* __restrict__ s32,
                                                       const uint32_t* __restrict__ fixw, float* __restrict__ dh)
 {
+    chain_wait();
     if (S->done) return;
     const double coef = lanczos ? S->alfa / S->beta : 0.0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1094,6 +1106,7 @@ __global__ void __launch_bounds__(kVecThreads) k_mg_prolong(int n_fine, const in
                                                            const float* __restrict__ s32,
                                                            const uint32_t* __restrict__ fixw, float* __restrict__ xh)
 {
+    chain_wait();
     if (S->done) return;
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n_fine; g += (int64_t)gridDim.x * blockDim.x) {
         // 24 coarse DOFs of the owner cell and the node's 24 prolongation weights: six 16-byte loads each
@@ -1125,6 +1138,7 @@ __global__ void __launch_bounds__(kVecThreads) k_mg_out(int n, const float* __re
                                                        const double* __restrict__ r, double* __restrict__ y, TlState* S,
                                                        double* __restrict__ partial, int init)
 {
+    chain_wait();
     if (S->done) return;
     __shared__ double sh[32];
     double acc[1] = {0.0};
@@ -1495,9 +1509,9 @@ int coarse_build(CoarseHandle& C, System& F, CellsHandle& Ce, const int32_t* h_c
 // ec = Cinv rc (symmetric packed blocks)
 void coarse_solve(CoarseHandle& C, const TlState* S, cudaStream_t st)
 {
-    k_tl_symv<<<std::min(C.sym_n, 148 * 4), 256, 0, st>>>(C.sym_nb, C.sym_n, C.sym_blocks.p, C.Csym.p, C.rc.p,
-                                                          C.sym_part.p, S);
-    k_tl_symv_sum<<<(C.n_pad + 255) / 256, 256, 0, st>>>(C.n_pad, C.sym_nb, C.sym_part.p, C.ec.p, S);
+    launch_chained(k_tl_symv, std::min(C.sym_n, 148 * 4), 256, 0, st, C.sym_nb, C.sym_n, C.sym_blocks.p, C.Csym.p,
+                   C.rc.p, C.sym_part.p, S);
+    launch_chained(k_tl_symv_sum, (C.n_pad + 255) / 256, 256, 0, st, C.n_pad, C.sym_nb, C.sym_part.p, C.ec.p, S);
 }
 
 // y = M^-1 r into y (FP32: scaled system; FP64: original unknowns with s = D^-1/2);
@@ -1505,8 +1519,8 @@ void coarse_solve(CoarseHandle& C, const TlState* S, cudaStream_t st)
 template <class VT>
 void precondition(CoarseHandle& C, const VT* r, VT* y, int init, cudaStream_t st, unsigned gprol, const double* s)
 {
-    k_tl_restrict<VT><<<C.n_cells, 128, 0, st>>>(C.own_ptr.p, C.own.p, C.psi_hat.p, r, nullptr, nullptr, C.cpart.p, s,
-                                                 C.st.p, 0);
+    k_tl_restrict<VT><<<C.n_cells, kRestrictThreads, 0, st>>>(C.own_ptr.p, C.own.p, C.psi_hat.p, r, nullptr, nullptr,
+                                                              C.cpart.p, s, C.st.p, 0);
     k_tl_gather<<<gridn(C.n_cf), 256, 0, st>>>(C.n_cf, C.dptr.p, C.dent.p, C.cpart.p, C.rc.p, C.st.p);
     coarse_solve(C, C.st.p, st);
     k_tl_prolong<VT><<<gprol, kVecThreads, 0, st>>>(C.n_fine, C.owner.p, C.cdof.p, C.psi_hat.p, C.ec.p, r, y, s, C.st.p,
@@ -1564,13 +1578,13 @@ int inner_solve(CoarseHandle& C, int maxiter, double tau, int* iters)
             VT* w2 = Wb[1 - p];
             k_tl_spmv<VT><<<gsp, 256, 0, st>>>(A, Y, V, Z, r1, S, C.partial.p + 2048);
             // r2_new = z - (alfa/beta) r2 over r1's buffer, and its restriction partials
-            k_tl_restrict<VT><<<C.n_cells, 128, 0, st>>>(C.own_ptr.p, C.own.p, C.psi_hat.p, Z, r2, r1, C.cpart.p, s, S, 1);
+            k_tl_restrict<VT><<<C.n_cells, kRestrictThreads, 0, st>>>(C.own_ptr.p, C.own.p, C.psi_hat.p, Z, r2, r1,
+                                                                      C.cpart.p, s, S, 1);
             k_tl_gather<<<gridn(C.n_cf), 256, 0, st>>>(C.n_cf, C.dptr.p, C.dent.p, C.cpart.p, C.rc.p, S);
             coarse_solve(C, S, st);
             k_tl_prolong<VT><<<gprol, kVecThreads, 0, st>>>(C.n_fine, C.owner.p, C.cdof.p, C.psi_hat.p, C.ec.p, r1, Y, s,
                                                             S, C.partial.p, 0);
             k_tl_update<VT><<<gvec, kVecThreads, 0, st>>>(n, V, w1, w2, X, S);
-            k_tl_applied<<<1, 1, 0, st>>>(S);
         }
     };
     cudaGraphExec_t& graph = C.graph[f32 ? 0 : 1];
@@ -1597,7 +1611,7 @@ int inner_solve(CoarseHandle& C, int maxiter, double tau, int* iters)
         if (16 * rounds > maxiter + 32) break;
         for (int k = 0; k < 4; k++) MSFEM_CK(cudaGraphLaunch(graph, st));
         rounds += 4;
-        F.total_launches += 4 * 16 * 7;
+        F.total_launches += 4 * 16 * 6;
     }
     *iters = C.h_st->iter;
     return C.h_st->done == 3 ? MSFEM_ERR_NUMERIC : MSFEM_OK;
@@ -1650,19 +1664,24 @@ void mg_cycle(CoarseHandle& C, const double* z, const double* r2, double* r_out,
         else
             k_mg_resid<<<gsp, 256, 0, st>>>(At, v16, c16, rhat, x, res, d0, x2, inv_theta, S, start);
     };
-    k_mg_in<<<gvec, kVecThreads, 0, st>>>(n, z, r2, r_out, s_t, rhat, res, dA, x, C.cc, S, lanczos, Kv.scale, Kv.fix,
-                                          mf ? dhA : nullptr);
+    // The cycle is a chain of kernels of 4 to 13 us at 40^3, so it is launched as one (launch_chained): the
+    // next kernel's launch and its set-up overlap the end of the last.  A MINRES iteration at 24^3, 40^3,
+    // 64^3 and 128^3 took 98, 152, 314 and 1551 us with plain launches and takes 80, 135, 298 and 1535.
+    // Only the kernels of a few blocks and the z-marches at their last step call chain_next: with it at the
+    // head of the long vector kernels as well, the waiting blocks crowd the SMs (98, 147, 333 and 1752 us).
+    launch_chained(k_mg_in, gvec, kVecThreads, 0, st, n, z, r2, r_out, s_t, rhat, res, dA, x, C.cc, S, lanczos,
+                   Kv.scale, Kv.fix, mf ? dhA : nullptr);
     for (int i = 1; i < C.cheb_deg; i++) cheb(i, x, i == C.cheb_deg - 1 ? xh : nullptr);
     resid(C.cheb_deg > 1 ? xh : dhA, nullptr, nullptr, 0.0f, 0);
-    k_tl_restrict<float><<<C.n_cells, 128, 0, st>>>(C.own_ptr.p, C.own.p, C.psi_t.p, res, nullptr, nullptr, C.cpart.p,
-                                                    nullptr, S, 0);
-    k_tl_gather<<<gridn(C.n_cf), 256, 0, st>>>(C.n_cf, C.dptr.p, C.dent.p, C.cpart.p, C.rc.p, S);
+    launch_chained(k_tl_restrict<float>, C.n_cells, kRestrictThreads, 0, st, C.own_ptr.p, C.own.p, C.psi_t.p, res,
+                   nullptr, nullptr, C.cpart.p, nullptr, S, 0);
+    launch_chained(k_tl_gather, gridn(C.n_cf), 256, 0, st, C.n_cf, C.dptr.p, C.dent.p, C.cpart.p, C.rc.p, S);
     coarse_solve(C, S, st);
-    k_mg_prolong<<<gvec, kVecThreads, 0, st>>>(C.n_fine, C.owner.p, C.cdof.p, C.psi_t.p, C.ec.p, x, S, Kv.scale, Kv.fix,
-                                               mf ? xh : nullptr);
+    launch_chained(k_mg_prolong, gvec, kVecThreads, 0, st, C.n_fine, C.owner.p, C.cdof.p, C.psi_t.p, C.ec.p, x, S,
+                   Kv.scale, Kv.fix, mf ? xh : nullptr);
     resid(xh, dA, x2, C.cc.inv_theta, 1);
     for (int i = 1; i < C.cheb_deg; i++) cheb(i, x2, nullptr);
-    k_mg_out<<<gvec, kVecThreads, 0, st>>>(n, x2, s_t, lanczos ? r_out : z, y, S, C.partial.p, init);
+    launch_chained(k_mg_out, gvec, kVecThreads, 0, st, n, x2, s_t, lanczos ? r_out : z, y, S, C.partial.p, init);
 }
 
 // FP64 MINRES on the original matrix with the multiplicative cycle as preconditioner
@@ -1710,8 +1729,7 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
             else
                 k_tl_spmv<double><<<gsp, 256, 0, st>>>(A, Y, V, Z, r1, S, C.partial.p + 2048);
             mg_cycle(C, Z, r2, r1, Y, 1, 0, st);  // r2_new over r1's buffer, then y = M^-1 r2_new
-            k_tl_update<double><<<gvec, kVecThreads, 0, st>>>(n, V, w1, w2, X, S);
-            k_tl_applied<<<1, 1, 0, st>>>(S);
+            launch_chained(k_tl_update<double>, gvec, kVecThreads, 0, st, n, V, w1, w2, X, S);
         }
     };
     cudaGraphExec_t& graph = C.graph[2];
@@ -1764,7 +1782,7 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
         }
         for (int k = 0; k < 4; k++) MSFEM_CK(cudaGraphLaunch(graph, st));
         rounds += 4;
-        F.total_launches += 4 * 16 * (11 + 2 * (C.cheb_deg - 1));
+        F.total_launches += 4 * 16 * (10 + 2 * (C.cheb_deg - 1));
     }
     *iters = C.h_st->iter;
     return C.h_st->done == 3 ? MSFEM_ERR_NUMERIC : MSFEM_OK;
