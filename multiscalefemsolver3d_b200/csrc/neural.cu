@@ -57,9 +57,8 @@ constexpr int kLayerW = kTaps * kCh * kCh;               // [27][32 co][32 ci]
 constexpr int kLayer = kLayerW + kCh;                    // weights + bias
 constexpr int kParams = kL1 + 3 * kLayer;
 constexpr int kPart0 = kL1;                              // first-layer weight-gradient partial
-// conv kernel shared memory: a 4-plane halo of 18 x 18 voxel records (64 B) + the weights
+// weight-gradient kernel shared memory: a 4-plane halo of 18 x 18 voxel records (64 B) + 512 records of dZ
 constexpr int kHaloRec = 4 * 18 * 18;
-constexpr int kConvSmem = kHaloRec * 64 + kTaps * kCh * 64;
 constexpr int kWgradSmem = kHaloRec * 64 + 512 * 64;
 
 __host__ __device__ constexpr int layer_base(int l) { return kL1 + (l - 1) * kLayer; }
@@ -102,6 +101,33 @@ __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.commit_group;\n" ::);
     asm volatile("cp.async.wait_group 0;\n" ::);
+}
+
+__device__ __forceinline__ void mb_init(uint32_t bar, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
+}
+
+__device__ __forceinline__ void mb_arrive(uint32_t bar)
+{
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}\n" ::"r"(bar) : "memory");
+}
+
+// bounded wait on phase `parity` of a shared-memory barrier
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
+{
+    for (int i = 0; i < (1 << 22); i++) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
 }
 
 // the halo of planes z0-1 .. z0+2 of one cell: 18 x 18 records per plane, zero outside the cell
@@ -221,98 +247,213 @@ __global__ void __launch_bounds__(256) k_first_wgrad(int n_cells, int cells_per_
 
 enum { kEpiRelu = 0, kEpiF32 = 1, kEpiMask = 2 };
 
-// One CTA = two z-planes (512 voxels) of one cell; warp w owns the x-rows 4w .. 4w+3 (16 voxels
+// One step = two z-planes (512 voxels) of one cell; warp w owns the x-rows 4w .. 4w+3 (16 voxels
 // each, one m16 tile) and all 32 output channels (four n8 tiles).  K = 27 taps x 32 input
 // channels, walked as 54 k16 steps over the shared-memory halo (implicit GEMM).
 //   kEpiRelu: out = bf16(relu(acc + bias))           (forward, hidden layers)
 //   kEpiF32:  outf = acc + bias                      (forward, last layer)
 //   kEpiMask: out = bf16(acc * (mask > 0))           (backward data: w holds the flipped,
 //             transposed weights and mask the activations of the layer below)
+// A CTA walks a contiguous range of steps with the weights loaded once.  Its planes go through a ring
+// of eight slots: the two new planes of the next step (four at the start of a cell) land while this
+// step's products run, behind one barrier a step.  A plane is [16-byte channel chunk][18 y][18 x], so
+// the eight rows of a matrix are 128 contiguous bytes (no bank conflicts) and every ldmatrix is one
+// lane address plus a constant.
+// Bound by the rate of mma.sync (a loop of these alone: 550 TFLOP/s, 7.6 us a step): a step takes
+// 9.9 us, 8.5 of which the products alone in this order.  A layer of 512 cells: 290 us; with a CTA a
+// step, loads before products, 367.
+constexpr int kCvRec = 18 * 18;
+constexpr int kCvChunk = kCvRec * 16;                      // 5,184 B
+constexpr int kCvPlane = 4 * kCvChunk;                     // 20,736 B
+constexpr int kCvSlots = 8;
+constexpr int kCvWChunk = kTaps * kCh * 16;                // 13,824 B: one channel chunk of the weights
+constexpr int kCvBar = kCvSlots * kCvPlane + 4 * kCvWChunk;
+constexpr int kCvSmem = kCvBar + 16;                       // 221,200 B
+
+// the 256 voxels of plane p (zero outside the cell) into a slot whose border is zero; 256 threads
+__device__ __forceinline__ void cv_load_plane(unsigned char* slot, const __nv_bfloat16* cell_base, int p)
+{
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int v = (threadIdx.x >> 2) + 64 * i, c = threadIdx.x & 3;
+        const uint32_t off = c * kCvChunk + (((v >> 4) + 1) * 18 + (v & 15) + 1) * 16;
+        if (p >= 0 && p < kV)
+            cp_async16(smem_u32(slot) + off, cell_base + ((size_t)(p * 256 + v) * kCh + c * 8));
+        else
+            *reinterpret_cast<uint4*>(slot + off) = make_uint4(0, 0, 0, 0);
+    }
+}
+
+// lane t of a quad holds word t of four groups; afterwards it holds the four words of group t
+__device__ __forceinline__ uint4 quad_transpose(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int t)
+{
+    const bool odd = t & 1, up = t & 2;
+    const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1), b = __shfl_xor_sync(0xffffffffu, odd ? w2 : w3, 1);
+    const uint32_t l0 = odd ? a : w0, l1 = odd ? w1 : a;  // group 0 or 1, words of the lane pair
+    const uint32_t h0 = odd ? b : w2, h1 = odd ? w3 : b;  // group 2 or 3
+    const uint32_t c = __shfl_xor_sync(0xffffffffu, up ? l0 : h0, 2), d = __shfl_xor_sync(0xffffffffu, up ? l1 : h1, 2);
+    return up ? make_uint4(c, d, h0, h1) : make_uint4(l0, l1, c, d);
+}
+
+// the two BF16 values of v where m's are positive, zero elsewhere
+__device__ __forceinline__ uint32_t positive_only(uint32_t v, uint32_t m)
+{
+    const __nv_bfloat162 mm = *reinterpret_cast<const __nv_bfloat162*>(&m);
+    return (__low2float(mm) > 0.f ? v & 0xffffu : 0u) | (__high2float(mm) > 0.f ? v & 0xffff0000u : 0u);
+}
+
 template <int EPI>
-__global__ void __launch_bounds__(256, 1) k_conv32(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ w,
-                                                   const float* __restrict__ bias, const __nv_bfloat16* __restrict__ mask,
-                                                   __nv_bfloat16* __restrict__ out, float* __restrict__ outf)
+__global__ void __launch_bounds__(256, 1) k_conv32(int n_cells, const __nv_bfloat16* __restrict__ in,
+                                                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
+                                                   const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* __restrict__ out,
+                                                   float* __restrict__ outf, int* err)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    unsigned char* halo = sm;
-    unsigned char* ws = sm + kHaloRec * 64;
-    const int slab = blockIdx.x, cell = blockIdx.y, tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    load_halo(halo, in + (size_t)cell * kVox * kCh, 2 * slab);
+    unsigned char* ws = sm + kCvSlots * kCvPlane;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int s0 = (int)((int64_t)8 * n_cells * blockIdx.x / gridDim.x);
+    const int s1 = (int)((int64_t)8 * n_cells * (blockIdx.x + 1) / gridDim.x);
+    if (s0 >= s1) return;
+    auto cell_of = [&](int step) { return in + (size_t)(step >> 3) * kVox * kCh; };
+    auto slot_of = [&](int g) { return sm + (g & (kCvSlots - 1)) * kCvPlane; };
     for (int q = tid; q < kTaps * kCh * 4; q += blockDim.x) {
         const int row = q >> 2, c = q & 3;
-        cp_async16(smem_u32(ws) + swz(row, c), w + (size_t)row * kCh + c * 8);
+        cp_async16(smem_u32(ws) + c * kCvWChunk + row * 16, w + (size_t)row * kCh + c * 8);
+    }
+    // the 68 border records of every slot and chunk that a plane will use
+    for (int q = tid; q < (s1 - s0 > 1 ? kCvSlots : 4) * 4 * 68; q += blockDim.x) {
+        const int r = q % 68, k = r - 36;
+        const int rec = r < 18 ? r : r < 36 ? 17 * 18 + r - 18 : (1 + (k >> 1)) * 18 + 17 * (k & 1);
+        *reinterpret_cast<uint4*>(sm + (q / 68) * kCvChunk + rec * 16) = make_uint4(0, 0, 0, 0);
+    }
+    for (int k = 0; k < 4; k++) cv_load_plane(slot_of(k), cell_of(s0), 2 * (s0 & 7) - 1 + k);
+    const uint32_t bar = smem_u32(sm + kCvBar);
+    if (tid == 0) {
+        mb_init(bar, 8);  // an arrival per warp and step
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
     }
     cp_async_wait_all();
     __syncthreads();
 
-    float acc[4][4][4];
-#pragma unroll
-    for (int mt = 0; mt < 4; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) acc[mt][nt][q] = 0.f;
-
-    const uint32_t hb = smem_u32(halo), wb = smem_u32(ws);
     const int xa = (lane & 7) + 8 * ((lane >> 3) & 1), ka = lane >> 4;
     const int nb = lane & 7, ntoff = lane >> 4, kb = (lane >> 3) & 1;
-    for (int tap = 0; tap < kTaps; tap++) {
-        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+    const int zl = warp >> 2, y0 = 4 * (warp & 3);
+    const uint32_t la = smem_u32(sm) + ka * kCvChunk + (y0 * 18 + xa) * 16;
+    const uint32_t lb = smem_u32(ws) + kb * kCvWChunk + (8 * ntoff + nb) * 16;
+    int g0 = 0;
+    for (int step = s0; step < s1; step++) {
+        if (step > s0 && !tc_wait(bar, (step - s0 - 1) & 1)) {
+            if (lane == 0) atomicExch(err, 1);
+            break;
+        }
+        const int gn = (step & 7) == 7 ? g0 + 4 : g0 + 2;
+        if (step + 1 < s1)
+            for (int g = g0 + 4; g < gn + 4; g++)
+                cv_load_plane(slot_of(g), cell_of(step + 1), 2 * ((step + 1) & 7) - 1 + g - gn);
+        asm volatile("cp.async.commit_group;\n" ::);
+
+        float acc[4][4][4];
 #pragma unroll
-        for (int kc = 0; kc < 2; kc++) {
-            uint32_t a[4][4];
+        for (int mt = 0; mt < 4; mt++)
 #pragma unroll
-            for (int mt = 0; mt < 4; mt++) {
-                const int rr = 4 * warp + mt, zl = rr >> 4, y = rr & 15;
-                const int rec = ((zl + dz) * 18 + (y + dy)) * 18 + (xa + dx);
-                ldsm_x4(a[mt], hb + swz(rec, 2 * kc + ka));
-            }
-            uint32_t b[4][2];
+            for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[mt][nt][q] = 0.f;
+        // The k16 steps run dz, dy, dx, k half (the order of the sums on every path): with the last two fixed (i below), the x-rows of dy + 1 are
+        // those of dy moved by one, so the four fragments of each of the six (dx, half) stay in registers,
+        // the row that dy leaves behind is replaced at once (its successor is needed six steps later), and
+        // after dy = 2 the first four rows of the next plane take their places.
+        uint32_t a[6][4][4], b[2][4][2];
+        auto fetch_a = [&](uint32_t ab, int i, int row) {
+            ldsm_x4(a[i][row & 3], ab + 2 * (i & 1) * kCvChunk + (row * 18 + (i >> 1)) * 16);
+        };
+        auto fetch_b = [&](int buf, uint32_t bb, int t9, int kc) {
 #pragma unroll
             for (int pr = 0; pr < 2; pr++) {
                 uint32_t r[4];
-                const int row = tap * kCh + 8 * (2 * pr + ntoff) + nb;
-                ldsm_x4(r, wb + swz(row, 2 * kc + kb));
-                b[2 * pr][0] = r[0];
-                b[2 * pr][1] = r[1];
-                b[2 * pr + 1][0] = r[2];
-                b[2 * pr + 1][1] = r[3];
+                ldsm_x4(r, bb + 2 * kc * kCvWChunk + (t9 * kCh + 16 * pr) * 16);
+                b[buf][2 * pr][0] = r[0];
+                b[buf][2 * pr][1] = r[1];
+                b[buf][2 * pr + 1][0] = r[2];
+                b[buf][2 * pr + 1][1] = r[3];
             }
+        };
+        auto plane = [&](int dz) { return la + (uint32_t)((g0 + zl + dz) & (kCvSlots - 1)) * kCvPlane; };
+        fetch_b(0, lb, 0, 0);
 #pragma unroll
-            for (int mt = 0; mt < 4; mt++)
+        for (int i = 0; i < 6; i++)
 #pragma unroll
-                for (int nt = 0; nt < 4; nt++) mma16816(acc[mt][nt], a[mt], b[nt][0], b[nt][1]);
+            for (int row = 0; row < 4; row++) fetch_a(plane(0), i, row);
+        for (int dz = 0; dz < 3; dz++) {
+            const uint32_t ab = plane(dz), an = plane(dz + 1), bb = lb + dz * 9 * kCh * 16;
+#pragma unroll
+            for (int dy = 0; dy < 3; dy++)
+#pragma unroll
+                for (int i = 0; i < 6; i++) {
+                    const int k = 6 * dy + i;
+                    if (k < 17)
+                        fetch_b((k + 1) & 1, bb, (k + 1) / 2, (k + 1) & 1);
+                    else if (dz < 2)
+                        fetch_b(0, bb + 9 * kCh * 16, 0, 0);
+#pragma unroll
+                    for (int mt = 0; mt < 4; mt++)
+#pragma unroll
+                        for (int nt = 0; nt < 4; nt++)
+                            mma16816(acc[mt][nt], a[i][(mt + dy) & 3], b[k & 1][nt][0], b[k & 1][nt][1]);
+                    if (dy < 2)
+                        fetch_a(ab, i, dy + 4);
+                    else if (dz < 2)
+#pragma unroll
+                        for (int row = 0; row < 4; row++) fetch_a(an, i, row);
+                }
         }
-    }
 
-    const int g = lane >> 2, t = lane & 3;
+        // this thread's share of the next step's planes has landed and the warp has left this step's: the
+        // arrival comes before the epilogue, which so runs under the products of the other warps
+        cp_async_wait_all();
+        __syncwarp();
+        if (lane == 0) mb_arrive(bar);
+
+        const int g = lane >> 2, t = lane & 3;
+        const size_t vox0 = (size_t)(step >> 3) * kVox + (2 * (step & 7) + zl) * 256;
 #pragma unroll
-    for (int mt = 0; mt < 4; mt++) {
-        const int rr = 4 * warp + mt, z = 2 * slab + (rr >> 4), y = rr & 15;
+        for (int mt = 0; mt < 4; mt++) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int xv = g + 8 * h;
-            const size_t vox = (size_t)cell * kVox + (z * kV + y) * kV + xv;
-#pragma unroll
-            for (int nt = 0; nt < 4; nt++) {
-                const int co = 8 * nt + 2 * t;
-                float v0 = acc[mt][nt][2 * h], v1 = acc[mt][nt][2 * h + 1];
+            for (int h = 0; h < 2; h++) {
+                const size_t vox = vox0 + (y0 + mt) * kV + g + 8 * h;
                 if (EPI == kEpiF32) {
-                    *reinterpret_cast<float2*>(outf + vox * kCh + co) = make_float2(v0 + bias[co], v1 + bias[co + 1]);
-                } else {
-                    if (EPI == kEpiRelu) {
-                        v0 = fmaxf(v0 + bias[co], 0.f);
-                        v1 = fmaxf(v1 + bias[co + 1], 0.f);
-                    } else {
-                        const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(mask + vox * kCh + co);
-                        v0 = __bfloat162float(m.x) > 0.f ? v0 : 0.f;
-                        v1 = __bfloat162float(m.y) > 0.f ? v1 : 0.f;
+#pragma unroll
+                    for (int nt = 0; nt < 4; nt++) {
+                        const int co = 8 * nt + 2 * t;
+                        *reinterpret_cast<float2*>(outf + vox * kCh + co) =
+                            make_float2(acc[mt][nt][2 * h] + bias[co], acc[mt][nt][2 * h + 1] + bias[co + 1]);
                     }
-                    *reinterpret_cast<__nv_bfloat162*>(out + vox * kCh + co) = __floats2bfloat162_rn(v0, v1);
+                } else {
+                    uint32_t wd[4];
+#pragma unroll
+                    for (int nt = 0; nt < 4; nt++) {
+                        const int co = 8 * nt + 2 * t;
+                        float v0 = acc[mt][nt][2 * h], v1 = acc[mt][nt][2 * h + 1];
+                        if (EPI == kEpiRelu) {
+                            v0 = fmaxf(v0 + bias[co], 0.f);
+                            v1 = fmaxf(v1 + bias[co + 1], 0.f);
+                        }
+                        const __nv_bfloat162 r = __floats2bfloat162_rn(v0, v1);
+                        wd[nt] = *reinterpret_cast<const uint32_t*>(&r);
+                    }
+                    uint4 o = quad_transpose(wd[0], wd[1], wd[2], wd[3], t);  // channels 8t .. 8t+7 of the voxel
+                    if (EPI == kEpiMask) {
+                        const uint4 m = reinterpret_cast<const uint4*>(mask + vox * kCh)[t];
+                        o.x = positive_only(o.x, m.x);
+                        o.y = positive_only(o.y, m.y);
+                        o.z = positive_only(o.z, m.z);
+                        o.w = positive_only(o.w, m.w);
+                    }
+                    reinterpret_cast<uint4*>(out + vox * kCh)[t] = o;
                 }
             }
         }
+        g0 = gn;
     }
 }
 
@@ -351,22 +492,6 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(kTcIdesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
-{
-    for (int i = 0; i < (1 << 22); i++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // plane gz of one cell into ring slot `slot`: [chunk][18 y][18 x] records, zero outside the cell
@@ -686,16 +811,6 @@ constexpr int kWsNBar = 2 * kWsSlots + 2 + 2 + 1;           // full, empty, accf
 constexpr int kWsSmem = kWsBar + 8 * kWsNBar + 16;
 constexpr int kWsThreads = 192;
 constexpr int kWsTmemCols = 128;
-
-__device__ __forceinline__ void mb_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ void mb_arrive(uint32_t bar)
-{
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}\n" ::"r"(bar) : "memory");
-}
 
 __device__ __forceinline__ void tc_commit(uint32_t bar)
 {
@@ -1308,9 +1423,9 @@ int conv_attrs()
 {
     static bool done = false;
     if (done) return 0;
-    MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
-    MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
-    MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_wgrad32, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgradSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tc<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tc<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
@@ -1337,7 +1452,7 @@ void conv(NetHandle& N, int n, const __nv_bfloat16* in, const __nv_bfloat16* w, 
     else if (N.tcgen05 == 1)
         k_conv32_tc<EPI><<<n, 128, kTcSmem, N.stream>>>(in, w, bias, mask, out, outf, N.err.p);
     else
-        k_conv32<EPI><<<dim3(8, n), 256, kConvSmem, N.stream>>>(in, w, bias, mask, out, outf);
+        k_conv32<EPI><<<std::min(8 * n, N.sms), 256, kCvSmem, N.stream>>>(n, in, w, bias, mask, out, outf, N.err.p);
 }
 
 // forward of n cells held in N.x -> N.a0, N.a1, N.a2, N.o
