@@ -56,16 +56,8 @@ constexpr int kL1 = kB0 + kCh;                           // layer l >= 1 at kL1 
 constexpr int kLayerW = kTaps * kCh * kCh;               // [27][32 co][32 ci]
 constexpr int kLayer = kLayerW + kCh;                    // weights + bias
 constexpr int kParams = kL1 + 3 * kLayer;
-constexpr int kPart0 = kL1;                              // first-layer weight-gradient partial
-// weight-gradient kernel shared memory: a 4-plane halo of 18 x 18 voxel records (64 B) + 512 records of dZ
-constexpr int kHaloRec = 4 * 18 * 18;
-constexpr int kWgradSmem = kHaloRec * 64 + 512 * 64;
 
 __host__ __device__ constexpr int layer_base(int l) { return kL1 + (l - 1) * kLayer; }
-
-// 16-byte chunk c of 64-byte record r: chunks XOR-swizzled by (r >> 1) & 3 so that eight
-// consecutive records read at one chunk index hit eight different bank groups
-__device__ __forceinline__ uint32_t swz(int rec, int chunk) { return rec * 64 + ((chunk ^ ((rec >> 1) & 3)) << 4); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -130,21 +122,6 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
-// the halo of planes z0-1 .. z0+2 of one cell: 18 x 18 records per plane, zero outside the cell
-__device__ __forceinline__ void load_halo(unsigned char* sm, const __nv_bfloat16* cell_base, int z0)
-{
-    for (int q = threadIdx.x; q < kHaloRec * 4; q += blockDim.x) {
-        const int rec = q >> 2, c = q & 3;
-        const int hz = rec / 324, rem = rec - hz * 324, hy = rem / 18, hx = rem - hy * 18;
-        const int gz = z0 - 1 + hz, gy = hy - 1, gx = hx - 1;
-        const uint32_t dst = smem_u32(sm) + swz(rec, c);
-        if (gz >= 0 && gz < kV && gy >= 0 && gy < kV && gx >= 0 && gx < kV)
-            cp_async16(dst, cell_base + ((size_t)((gz * kV + gy) * kV + gx) * kCh + c * 8));
-        else
-            *reinterpret_cast<uint4*>(sm + swz(rec, c)) = make_uint4(0, 0, 0, 0);
-    }
-}
-
 // ------------------------------------------------------------------ layer 0 (4 -> 32, FP32)
 
 __device__ __forceinline__ float coord_of(int i) { return (2.0f * i + 1.0f) / kV - 1.0f; }
@@ -187,60 +164,136 @@ __global__ void __launch_bounds__(256) k_first_fwd(const float* __restrict__ x, 
 }
 
 // dW0[tap][co][c] = sum_v dZ0[v][co] I[v + tap][c], db0[co] = sum_v dZ0[v][co]; one partial per CTA
-__global__ void __launch_bounds__(256) k_first_wgrad(int n_cells, int cells_per_cta, const float* __restrict__ x,
-                                                     const __nv_bfloat16* __restrict__ dz, float* __restrict__ part)
+// over a contiguous range of units (one unit = two z-planes of one cell).  FP32 on the CUDA cores: lane
+// = co, a warp takes four x-rows of one plane.  Channel 0 is the sum over the voxels (27 products each;
+// per row of 16 voxels nine rows of inputs, read as broadcast 16-byte words).  Channels 1..3 are
+// coordinates, so they need only sums of dZ0: over a row with the x-coordinate or without it, each of the
+// three ways a tap can leave the cell at the row's ends; y and z enter once per row and plane.
+// A thread's sums go to the CTA's partial after 64 units: at most 4,096 products in one chain.
+// Bound by the FP32 pipe (0.5 GFMA for 128 cells): 40 us; a CTA a cell with a lane per tap and channel and
+// all four inputs multiplied out, 1,240.
+constexpr int kFirstFlush = 64;
+__global__ void __launch_bounds__(256, 1) k_first_wgrad(int n_cells, const float* __restrict__ x,
+                                                        const __nv_bfloat16* __restrict__ dz, float* __restrict__ part)
 {
-    __shared__ float xs[3][18][18];
-    __shared__ float ds[256][kCh + 1];
-    const int tid = threadIdx.x, co = tid & 31, tg = tid >> 5;
-    float acc[4][kCin0];
+    __shared__ __align__(16) float xs[4][18][20];
+    __shared__ float red[8][kTaps][kCh];
+    const int tid = threadIdx.x, co = tid & 31, warp = tid >> 5;
+    const int zl = warp >> 2, y0 = 4 * (warp & 3);
+    float acc[kCin0][kTaps];
     float accb = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int c = 0; c < kCin0; c++)
 #pragma unroll
-        for (int c = 0; c < kCin0; c++) acc[i][c] = 0.f;
-    const int c0 = blockIdx.x * cells_per_cta, c1 = min(n_cells, c0 + cells_per_cta);
-    for (int cell = c0; cell < c1; cell++) {
-        const float* xc = x + (size_t)cell * kVox;
-        for (int z = 0; z < kV; z++) {
-            __syncthreads();
-            for (int q = tid; q < 3 * 18 * 18; q += blockDim.x) {
-                const int hz = q / 324, rem = q % 324, hy = rem / 18, hx = rem % 18;
-                const int gz = z - 1 + hz, gy = hy - 1, gx = hx - 1;
-                xs[hz][hy][hx] =
-                    (gz >= 0 && gz < kV && gy >= 0 && gy < kV && gx >= 0 && gx < kV) ? xc[(gz * kV + gy) * kV + gx] : 0.f;
+        for (int tap = 0; tap < kTaps; tap++) acc[c][tap] = 0.f;
+    const int u0 = (int)((int64_t)8 * n_cells * blockIdx.x / gridDim.x);
+    const int u1 = (int)((int64_t)8 * n_cells * (blockIdx.x + 1) / gridDim.x);
+    float* out = part + (size_t)blockIdx.x * kParams;
+    for (int u = u0; u < u1; u++) {
+        const int z0 = 2 * (u & 7), z = z0 + zl;
+        const float* xc = x + (size_t)(u >> 3) * kVox;
+        __syncthreads();
+        for (int q = tid; q < 4 * 18 * 20; q += blockDim.x) {
+            const int hz = q / 360, hy = (q / 20) % 18, hx = q % 20;
+            const int gz = z0 - 1 + hz, gy = hy - 1, gx = hx - 1;
+            xs[hz][hy][hx] = (gz >= 0 && gz < kV && gy >= 0 && gy < kV && gx >= 0 && gx < kV) ? xc[(gz * kV + gy) * kV + gx] : 0.f;
+        }
+        const __nv_bfloat16* dp = dz + ((size_t)(u >> 3) * kVox + z * 256 + y0 * kV) * kCh + co;
+        __nv_bfloat16 next[kV];
+#pragma unroll
+        for (int v = 0; v < kV; v++) next[v] = dp[v * kCh];
+        __syncthreads();
+        float sx[9], sp[9], sy[9];  // per (dy, dx): sums of d x-coordinate, d, d y-coordinate over the rows
+#pragma unroll
+        for (int k = 0; k < 9; k++) sx[k] = sp[k] = sy[k] = 0.f;
+#pragma unroll 1
+        for (int r = 0; r < 4; r++) {
+            const int y = y0 + r;
+            float d[kV];
+#pragma unroll
+            for (int v = 0; v < kV; v++) d[v] = __bfloat162float(next[v]);
+            if (r < 3) {
+                dp += kV * kCh;
+#pragma unroll
+                for (int v = 0; v < kV; v++) next[v] = dp[v * kCh];
             }
-            const __nv_bfloat16* dzp = dz + ((size_t)cell * kVox + z * 256) * kCh;
-            for (int q = tid; q < 256 * kCh; q += blockDim.x) ds[q >> 5][q & 31] = __bfloat162float(dzp[q]);
-            __syncthreads();
-            for (int v = 0; v < 256; v++) {
-                const float d = ds[v][co];
-                const int vx = v & 15, vy = v >> 4;
-                accb += d;
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int tap = tg + 8 * i;
-                    if (tap >= kTaps) break;
-                    const int dzt = tap / 9, dyt = (tap / 3) % 3, dxt = tap % 3;
-                    const int gz = z + dzt - 1, gy = vy + dyt - 1, gx = vx + dxt - 1;
-                    if (gz < 0 || gz >= kV || gy < 0 || gy >= kV || gx < 0 || gx >= kV) continue;
-                    acc[i][0] += d * xs[dzt][vy + dyt][vx + dxt];
-                    acc[i][1] += d * coord_of(gx);
-                    acc[i][2] += d * coord_of(gy);
-                    acc[i][3] += d * coord_of(gz);
+            for (int q = 0; q < 9; q++) {
+                const float4* row = reinterpret_cast<const float4*>(xs[zl + q / 3][y + q % 3]);
+                float in[20];
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    const float4 f = row[k];
+                    in[4 * k] = f.x;
+                    in[4 * k + 1] = f.y;
+                    in[4 * k + 2] = f.z;
+                    in[4 * k + 3] = f.w;
+                }
+#pragma unroll
+                for (int v = 0; v < kV; v++)
+#pragma unroll
+                    for (int dx = 0; dx < 3; dx++) acc[0][3 * q + dx] += d[v] * in[v + dx];
+            }
+            float mid = 0.f, xm = 0.f, xz = 0.f, xp = 0.f;
+#pragma unroll
+            for (int v = 0; v < kV; v++) {
+                if (v > 0 && v < kV - 1) mid += d[v];
+                if (v > 0) xm += d[v] * coord_of(v - 1);
+                xz += d[v] * coord_of(v);
+                if (v < kV - 1) xp += d[v] * coord_of(v + 1);
+            }
+            const float sums[3] = {mid + d[kV - 1], mid + d[0] + d[kV - 1], mid + d[0]}, xsum[3] = {xm, xz, xp};
+            accb += sums[1];
+#pragma unroll
+            for (int dy = 0; dy < 3; dy++) {
+                const int gy = y + dy - 1;
+                if (gy < 0 || gy >= kV) continue;
+                const float cy = coord_of(gy);
+#pragma unroll
+                for (int dx = 0; dx < 3; dx++) {
+                    sx[3 * dy + dx] += xsum[dx];
+                    sp[3 * dy + dx] += sums[dx];
+                    sy[3 * dy + dx] += sums[dx] * cy;
                 }
             }
         }
-    }
-    float* out = part + (size_t)blockIdx.x * kPart0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int tap = tg + 8 * i;
-        if (tap >= kTaps) break;
+        for (int d = 0; d < 3; d++) {
+            const int gz = z + d - 1;
+            if (gz < 0 || gz >= kV) continue;
+            const float cz = coord_of(gz);
 #pragma unroll
-        for (int c = 0; c < kCin0; c++) out[(tap * kCh + co) * kCin0 + c] = acc[i][c];
+            for (int k = 0; k < 9; k++) {
+                acc[1][9 * d + k] += sx[k];
+                acc[2][9 * d + k] += sy[k];
+                acc[3][9 * d + k] += sp[k] * cz;
+            }
+        }
+        const int done = u + 1 - u0;
+        if (done % kFirstFlush && u + 1 < u1) continue;
+        // the eight warps' sums in warp order, added to the CTA's partial
+#pragma unroll
+        for (int c = 0; c < kCin0 + 1; c++) {
+            __syncthreads();
+            if (c < kCin0) {
+#pragma unroll
+                for (int tap = 0; tap < kTaps; tap++) {
+                    red[warp][tap][co] = acc[c < kCin0 ? c : 0][tap];
+                    acc[c < kCin0 ? c : 0][tap] = 0.f;
+                }
+            } else {
+                red[warp][0][co] = accb;
+                accb = 0.f;
+            }
+            __syncthreads();
+            for (int q = tid; q < (c < kCin0 ? kTaps * kCh : kCh); q += blockDim.x) {
+                float s = 0.f;
+                for (int k = 0; k < 8; k++) s += (&red[k][0][0])[q];
+                float& o = out[c < kCin0 ? kW0 + q * kCin0 + c : kB0 + q];
+                o = done <= kFirstFlush ? s : o + s;
+            }
+        }
     }
-    if (tg == 0) out[kB0 + co] = accb;
 }
 
 // ------------------------------------------------------------------ 32 -> 32 convolutions (tensor cores)
@@ -284,6 +337,16 @@ __device__ __forceinline__ void cv_load_plane(unsigned char* slot, const __nv_bf
     }
 }
 
+// the 68 border records of every chunk of the first `slots` slots
+__device__ __forceinline__ void cv_zero_borders(unsigned char* ring, int slots)
+{
+    for (int q = threadIdx.x; q < slots * 4 * 68; q += blockDim.x) {
+        const int r = q % 68, k = r - 36;
+        const int rec = r < 18 ? r : r < 36 ? 17 * 18 + r - 18 : (1 + (k >> 1)) * 18 + 17 * (k & 1);
+        *reinterpret_cast<uint4*>(ring + (q / 68) * kCvChunk + rec * 16) = make_uint4(0, 0, 0, 0);
+    }
+}
+
 // lane t of a quad holds word t of four groups; afterwards it holds the four words of group t
 __device__ __forceinline__ uint4 quad_transpose(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int t)
 {
@@ -320,12 +383,7 @@ __global__ void __launch_bounds__(256, 1) k_conv32(int n_cells, const __nv_bfloa
         const int row = q >> 2, c = q & 3;
         cp_async16(smem_u32(ws) + c * kCvWChunk + row * 16, w + (size_t)row * kCh + c * 8);
     }
-    // the 68 border records of every slot and chunk that a plane will use
-    for (int q = tid; q < (s1 - s0 > 1 ? kCvSlots : 4) * 4 * 68; q += blockDim.x) {
-        const int r = q % 68, k = r - 36;
-        const int rec = r < 18 ? r : r < 36 ? 17 * 18 + r - 18 : (1 + (k >> 1)) * 18 + 17 * (k & 1);
-        *reinterpret_cast<uint4*>(sm + (q / 68) * kCvChunk + rec * 16) = make_uint4(0, 0, 0, 0);
-    }
+    cv_zero_borders(sm, s1 - s0 > 1 ? kCvSlots : 4);
     for (int k = 0; k < 4; k++) cv_load_plane(slot_of(k), cell_of(s0), 2 * (s0 & 7) - 1 + k);
     const uint32_t bar = smem_u32(sm + kCvBar);
     if (tid == 0) {
@@ -1041,113 +1099,199 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_conv32_ws(int n_cells, const 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(kWsTmemCols));
 }
 
-// dW[tap][co][ci] = sum_v dZ[v][co] A[v + tap][ci] and db[co] = sum_v dZ[v][co] over the cells of
-// this CTA (one fixed-order partial per CTA).  M = co (two m16 tiles, A operand = dZ^T through
-// ldmatrix.trans), N = ci (four n8 tiles, B operand = shifted activations through ldmatrix.trans),
-// K = voxels (16 per step: one x-row).  Warp w owns the taps w, w + 8, w + 16, w + 24 (< 27).
-__global__ void __launch_bounds__(256, 1) k_wgrad32(int n_cells, int cells_per_cta, const __nv_bfloat16* __restrict__ act,
-                                                    const __nv_bfloat16* __restrict__ dz, float* __restrict__ part)
+// dW[tap][co][ci] = sum_v dZ[v][co] A[v + tap][ci] and db[co] = sum_v dZ[v][co] over a contiguous
+// range of units (two z-planes of one cell; one fixed-order partial per CTA).  M = co (two m16 tiles, A
+// operand = dZ^T through ldmatrix.trans), N = ci (four n8 tiles, B operand = shifted activations through
+// ldmatrix.trans), K = voxels (16 per step: one x-row).  Warp w owns the taps w, w + 8, w + 16, w + 24
+// (< 27).  The activations go through k_conv32's ring of planes, dZ through two buffers, so that the next
+// unit lands under this one's products.
+// A CTA's accumulators are added to its partial after every eight units, so that no chain of tensor-core
+// sums is longer than a cell's.
+// A layer of 128 cells: 89 us (the products alone at the mma.sync rate: 53); with a CTA a cell and loads
+// before products, 124, and a batch of 9 cells kept 9 multiprocessors busy.
+constexpr int kWgChunk = 512 * 16 + 32;                    // a channel chunk of dZ; 32 B keep the chunks' banks apart
+constexpr int kWgDz = 4 * kWgChunk;
+constexpr int kWgSmem = kCvSlots * kCvPlane + 2 * kWgDz;   // 231,680 B
+constexpr int kWgFlush = 8;
+
+// the products of one unit for a warp's NT taps; the fragments of the next tap are in flight under this one's
+template <int NT>
+__device__ __forceinline__ void wg_products(float (&acc)[4][2][4][4], const uint32_t (&off)[4], const int (&dzt)[4], int g0,
+                                            uint32_t dbuf)
 {
-    extern __shared__ __align__(128) unsigned char sm[];
-    unsigned char* halo = sm;
-    unsigned char* ds = sm + kHaloRec * 64;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ntap = warp < 3 ? 4 : 3;
-    float acc[4][2][4][4];
+    uint32_t a[2][2][4], b[2][4][2];
+    auto fetch_a = [&](int buf, int row) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+        for (int mt = 0; mt < 2; mt++) ldsm_x4_t(a[buf][mt], dbuf + 2 * mt * kWgChunk + row * kV * 16);
+    };
+    auto fetch_b = [&](int buf, uint32_t base) {
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++)
+        for (int pr = 0; pr < 2; pr++) {
+            uint32_t r[4];
+            ldsm_x4_t(r, base + 2 * pr * kCvChunk);
+            b[buf][2 * pr][0] = r[0];
+            b[buf][2 * pr][1] = r[1];
+            b[buf][2 * pr + 1][0] = r[2];
+            b[buf][2 * pr + 1][1] = r[3];
+        }
+    };
+#pragma unroll 1
+    for (int zl = 0; zl < 2; zl++) {
+        uint32_t bb[NT];
 #pragma unroll
-            for (int nt = 0; nt < 4; nt++)
+        for (int i = 0; i < NT; i++) bb[i] = off[i] + (uint32_t)((g0 + zl + dzt[i]) & (kCvSlots - 1)) * kCvPlane;
+        fetch_a(0, zl * kV);
+        fetch_b(0, bb[0]);
+#pragma unroll 1
+        for (int y2 = 0; y2 < kV; y2 += 2) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) acc[i][mt][nt][q] = 0.f;
-    float accb = 0.f;
-    const uint32_t hb = smem_u32(halo), db = smem_u32(ds);
-    const int lr = lane & 7, lj = lane >> 3;
-    const int c0 = blockIdx.x * cells_per_cta, c1 = min(n_cells, c0 + cells_per_cta);
-    for (int cell = c0; cell < c1; cell++) {
-        for (int slab = 0; slab < 8; slab++) {
-            __syncthreads();
-            load_halo(halo, act + (size_t)cell * kVox * kCh, 2 * slab);
-            const __nv_bfloat16* dzp = dz + ((size_t)cell * kVox + slab * 512) * kCh;
-            for (int q = tid; q < 512 * 4; q += blockDim.x) cp_async16(db + swz(q >> 2, q & 3), dzp + (size_t)q * 8);
-            cp_async_wait_all();
-            __syncthreads();
-            {   // bias: thread (co = lane, voxels warp, warp + 8, ...)
-                for (int v = warp; v < 512; v += 8) {
-                    const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(ds + swz(v, lane >> 3));
-                    accb += __bfloat162float(r[lane & 7]);
-                }
-            }
-            for (int rr = 0; rr < 32; rr++) {
-                const int zl = rr >> 4, y = rr & 15;
-                uint32_t a[2][4];
-#pragma unroll
-                for (int mt = 0; mt < 2; mt++) {
-                    const int xv = lr + 8 * (lj >> 1);
-                    ldsm_x4_t(a[mt], db + swz(rr * 16 + xv, 2 * mt + (lj & 1)));
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (i >= ntap) break;
-                    const int tap = warp + 8 * i;
-                    const int dzt = tap / 9, dyt = (tap / 3) % 3, dxt = tap % 3;
-                    uint32_t b[4][2];
-#pragma unroll
-                    for (int pr = 0; pr < 2; pr++) {
-                        uint32_t r[4];
-                        const int xv = lr + 8 * (lj & 1);
-                        const int rec = ((zl + dzt) * 18 + (y + dyt)) * 18 + (xv + dxt);
-                        ldsm_x4_t(r, hb + swz(rec, 2 * pr + (lj >> 1)));
-                        b[2 * pr][0] = r[0];
-                        b[2 * pr][1] = r[1];
-                        b[2 * pr + 1][0] = r[2];
-                        b[2 * pr + 1][1] = r[3];
+            for (int k = 0; k < 2 * NT; k++) {
+                const int h = k / NT, i = k % NT;
+                if (k == NT - 1) fetch_a(1, zl * kV + y2 + 1);
+                if (k == 2 * NT - 1) {
+                    if (y2 + 2 < kV) {
+                        fetch_a(0, zl * kV + y2 + 2);
+                        fetch_b(0, bb[0] + (y2 + 2) * 18 * 16);
                     }
+                } else
+                    fetch_b((k + 1) & 1, bb[(k + 1) % NT] + (y2 + (k + 1) / NT) * 18 * 16);
 #pragma unroll
-                    for (int mt = 0; mt < 2; mt++)
+                for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-                        for (int nt = 0; nt < 4; nt++) mma16816(acc[i][mt][nt], a[mt], b[nt][0], b[nt][1]);
-                }
+                    for (int nt = 0; nt < 4; nt++) mma16816(acc[i][mt][nt], a[h][mt], b[k & 1][nt][0], b[k & 1][nt][1]);
             }
         }
     }
-    float* out = part + (size_t)blockIdx.x * kLayer;
-    const int g = lane >> 2, t = lane & 3;
+}
+
+__global__ void __launch_bounds__(256, 1) k_wgrad32(int n_cells, const __nv_bfloat16* __restrict__ act,
+                                                    const __nv_bfloat16* __restrict__ dz, float* __restrict__ part)
+{
+    extern __shared__ __align__(128) unsigned char sm[];
+    unsigned char* ds = sm + kCvSlots * kCvPlane;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ntap = warp < 3 ? 4 : 3;
+    float acc[4][2][4][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) acc[i][mt][nt][q] = 0.f;
+    };
+    clear();
+    float2 accb = make_float2(0.f, 0.f);
+    const int u0 = (int)((int64_t)8 * n_cells * blockIdx.x / gridDim.x);
+    const int u1 = (int)((int64_t)8 * n_cells * (blockIdx.x + 1) / gridDim.x);
+    if (u0 >= u1) return;
+    auto slot_of = [&](int g) { return sm + (g & (kCvSlots - 1)) * kCvPlane; };
+    auto load = [&](int u, int g, int first) {  // planes first .. 3 of unit u's four from slot g, and its dZ
+        for (int k = first; k < 4; k++)
+            cv_load_plane(slot_of(g + k - first), act + (size_t)(u >> 3) * kVox * kCh, 2 * (u & 7) - 1 + k);
+        const __nv_bfloat16* dp = dz + ((size_t)(u >> 3) * kVox + (u & 7) * 512) * kCh;
+        unsigned char* buf = ds + ((u - u0) & 1) * kWgDz;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int q = tid + 256 * i;
+            cp_async16(smem_u32(buf) + (q & 3) * kWgChunk + (q >> 2) * 16, dp + (size_t)q * 8);
+        }
+    };
+    cv_zero_borders(sm, u1 - u0 > 1 ? kCvSlots : 4);
+    load(u0, 0, 0);
+    const int lr = lane & 7, lj = lane >> 3;
+    // lane addresses: dZ as [chunk][512 voxels], activations as [chunk][18 y][18 x]
+    const uint32_t da = smem_u32(ds) + (lj & 1) * kWgChunk + (lr + 8 * (lj >> 1)) * 16;
+    uint32_t off[4];
+    int dzt[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        if (i >= ntap) break;
         const int tap = warp + 8 * i;
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-            for (int nt = 0; nt < 4; nt++) {
-                const int ci = 8 * nt + 2 * t;
-                const int co0 = 16 * mt + g, co1 = co0 + 8;
-                *reinterpret_cast<float2*>(out + (tap * kCh + co0) * kCh + ci) = make_float2(acc[i][mt][nt][0], acc[i][mt][nt][1]);
-                *reinterpret_cast<float2*>(out + (tap * kCh + co1) * kCh + ci) = make_float2(acc[i][mt][nt][2], acc[i][mt][nt][3]);
-            }
+        dzt[i] = tap / 9;
+        off[i] = smem_u32(sm) + (lj >> 1) * kCvChunk + (((tap / 3) % 3) * 18 + tap % 3 + lr + 8 * (lj & 1)) * 16;
     }
-    // bias partials: 8 warps x 32 channels, summed in warp order
-    __shared__ float sb[8][32];
-    sb[warp][lane] = accb;
+    float* out = part + (size_t)blockIdx.x * kParams;
+    const int g = lane >> 2, t = lane & 3;
+    int g0 = 0;
+    for (int u = u0; u < u1; u++) {
+        cp_async_wait_all();
+        __syncthreads();
+        const bool turn = (u & 7) == 7;
+        if (u + 1 < u1) load(u + 1, g0 + 4, turn ? 0 : 2);
+        asm volatile("cp.async.commit_group;\n" ::);
+        const unsigned char* buf = ds + ((u - u0) & 1) * kWgDz;
+        // bias: lane = (channel pair, one of two voxels), voxels 2 warp, 2 warp + 16, ...
+        const unsigned char* bp = buf + ((lane & 15) >> 2) * kWgChunk + (lane & 3) * 4 + (2 * warp + (lane >> 4)) * 16;
+#pragma unroll 8
+        for (int v = 0; v < 512; v += 16) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(bp + v * 16));
+            accb.x += f.x;
+            accb.y += f.y;
+        }
+        const uint32_t dbuf = da + ((u - u0) & 1) * kWgDz;
+        if (ntap == 4)
+            wg_products<4>(acc, off, dzt, g0, dbuf);
+        else
+            wg_products<3>(acc, off, dzt, g0, dbuf);
+        g0 += turn ? 4 : 2;
+        const int done = u + 1 - u0;
+        if (done % kWgFlush == 0 || u + 1 == u1) {
+            const bool first = done <= kWgFlush;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                if (i >= ntap) break;
+                const int tap = warp + 8 * i;
+#pragma unroll
+                for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                    for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int ci = 8 * nt + 2 * t, co = 16 * mt + g + 8 * h;
+                            float2* o = reinterpret_cast<float2*>(out + (tap * kCh + co) * kCh + ci);
+                            float2 v = make_float2(acc[i][mt][nt][2 * h], acc[i][mt][nt][2 * h + 1]);
+                            if (!first) {
+                                const float2 old = *o;
+                                v.x += old.x;
+                                v.y += old.y;
+                            }
+                            *o = v;
+                        }
+            }
+            clear();
+        }
+    }
+    // bias partials: 16 sums of 32 channels, in order
+    float* sb = reinterpret_cast<float*>(sm);
+    __syncthreads();
+    reinterpret_cast<float2*>(sb)[(2 * warp + (lane >> 4)) * 16 + (lane & 15)] = accb;
     __syncthreads();
     if (tid < 32) {
         float s = 0.f;
-        for (int k = 0; k < 8; k++) s += sb[k][tid];
+        for (int k = 0; k < 16; k++) s += sb[32 * k + tid];
         out[kLayerW + tid] = s;
     }
 }
 
-// out[i] = sum_p part[p][i] in p order
-__global__ void k_reduce_parts(int n_parts, int len, const float* __restrict__ part, float* __restrict__ out)
+// out[i] = sum_p part[p][i] in p order, sixteen loads in flight; all layers at once.  Bound by L2 latency:
+// 12 us (a launch a layer, one load at a time: 4 x 15)
+__global__ void __launch_bounds__(256) k_reduce_parts(int n_parts, const float* __restrict__ part, float* __restrict__ out)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int p = 0; p < n_parts; p++) s += part[(size_t)p * len + i];
-        out[i] = s;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kParams) return;
+    float s = 0.f;
+    int p = 0;
+    for (; p + 16 <= n_parts; p += 16) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) v[k] = part[(size_t)(p + k) * kParams + i];
+#pragma unroll
+        for (int k = 0; k < 16; k++) s += v[k];
     }
+    for (; p < n_parts; p++) s += part[(size_t)p * kParams + i];
+    out[i] = s;
 }
 
 // ------------------------------------------------------------------ loss, nodes, bases
@@ -1169,20 +1313,52 @@ __device__ __forceinline__ float node_corr(const float* __restrict__ o, int i, i
     return s / (float)(node_count(i) * node_count(j) * node_count(k));
 }
 
-// per cell: sum of (corr - y)^2 into lossp[cell]; gnode = d loss / d corr (times the node mask)
+// Thread (node, four channels) of one cell: the corrections of the node from its up to eight voxels, the
+// sum of (corr - y)^2 (one partial a CTA), and d loss / d L3 output, which is one value per node, written
+// to the same voxels (BF16, channels >= 24 zero): each voxel belongs to one node, so the voxel outputs
+// are read once, the gradient written once, and no node array is kept.  Bound by HBM: 128 cells 24 us; a
+// CTA a cell into a node array and a pass from there, 156 + 36.
+constexpr int kNodeItems = kNodes * 8;
+constexpr int kNodeBlocks = (kNodeItems + 255) / 256;
 __global__ void __launch_bounds__(256) k_loss_nodes(const float* __restrict__ o, const float* __restrict__ y,
-                                                    float inv_norm, float* __restrict__ gnode, float* __restrict__ lossp)
+                                                    float inv_norm, __nv_bfloat16* __restrict__ d0, float* __restrict__ lossp)
 {
-    const int cell = blockIdx.x;
-    const float* oc = o + (size_t)cell * kVox * kCh;
+    const int cell = blockIdx.y, item = blockIdx.x * 256 + threadIdx.x;
+    const float4* oc = reinterpret_cast<const float4*>(o + (size_t)cell * kVox * kCh);
+    uint2* dc = reinterpret_cast<uint2*>(d0 + (size_t)cell * kVox * kCh);
     float s = 0.f;
-    for (int q = threadIdx.x; q < kNodes * kOut; q += blockDim.x) {
-        const int n = q / kOut, ch = q - n * kOut;
+    if (item < kNodeItems) {
+        const int n = item >> 3, q = item & 7;
         const int i = n % kN, j = (n / kN) % kN, k = n / (kN * kN);
-        const float d = node_corr(oc, i, j, k, ch) - y[(size_t)cell * kNodes * kOut + q];
-        s += d * d;
-        gnode[(size_t)cell * kNodes * kOut + q] =
-            is_vertex(i, j, k) ? 0.f : 2.f * d * inv_norm / (float)(node_count(i) * node_count(j) * node_count(k));
+        const bool zero = is_vertex(i, j, k);
+        const int a0 = max(0, 2 * i - 1), a1 = min(kV - 1, 2 * i), b0 = max(0, 2 * j - 1), b1 = min(kV - 1, 2 * j);
+        const int c0 = max(0, 2 * k - 1), c1 = min(kV - 1, 2 * k);
+        __nv_bfloat162 g01 = __floats2bfloat162_rn(0.f, 0.f), g23 = g01;
+        if (q < kOut / 4) {
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!zero)
+                for (int c = c0; c <= c1; c++)
+                    for (int b = b0; b <= b1; b++)
+                        for (int a = a0; a <= a1; a++) {
+                            const float4 v = oc[((c * kV + b) * kV + a) * 8 + q];
+                            f.x += v.x;
+                            f.y += v.y;
+                            f.z += v.z;
+                            f.w += v.w;
+                        }
+            const float cnt = (float)(node_count(i) * node_count(j) * node_count(k));
+            const float4 t = reinterpret_cast<const float4*>(y + (size_t)cell * kNodes * kOut + n * kOut)[q];
+            const float e0 = f.x / cnt - t.x, e1 = f.y / cnt - t.y, e2 = f.z / cnt - t.z, e3 = f.w / cnt - t.w;
+            s = e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
+            if (!zero) {
+                g01 = __floats2bfloat162_rn(2.f * e0 * inv_norm / cnt, 2.f * e1 * inv_norm / cnt);
+                g23 = __floats2bfloat162_rn(2.f * e2 * inv_norm / cnt, 2.f * e3 * inv_norm / cnt);
+            }
+        }
+        const uint2 g = make_uint2(*reinterpret_cast<const uint32_t*>(&g01), *reinterpret_cast<const uint32_t*>(&g23));
+        for (int c = c0; c <= c1; c++)
+            for (int b = b0; b <= b1; b++)
+                for (int a = a0; a <= a1; a++) dc[((c * kV + b) * kV + a) * 8 + q] = g;
     }
     __shared__ float red[256];
     red[threadIdx.x] = s;
@@ -1191,30 +1367,21 @@ __global__ void __launch_bounds__(256) k_loss_nodes(const float* __restrict__ o,
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) lossp[cell] = red[0];
+    if (threadIdx.x == 0) lossp[cell * kNodeBlocks + blockIdx.x] = red[0];
 }
 
-// d loss / d L3 output (BF16, channels >= 24 zero): each voxel belongs to one node
-__global__ void k_dout(int n_cells, const float* __restrict__ gnode, __nv_bfloat16* __restrict__ d)
+__global__ void __launch_bounds__(256) k_loss_sum(int n, const float* __restrict__ lossp, float inv_norm, float* __restrict__ out)
 {
-    const int64_t total = (int64_t)n_cells * kVox * kCh;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(q & 31);
-        const int64_t v = q >> 5;
-        const int cell = (int)(v / kVox), vl = (int)(v % kVox);
-        const int vx = vl & 15, vy = (vl >> 4) & 15, vz = vl >> 8;
-        const int n = ((vx + 1) >> 1) + kN * (((vy + 1) >> 1) + kN * ((vz + 1) >> 1));
-        d[q] = __float2bfloat16_rn(ch < kOut ? gnode[((size_t)cell * kNodes + n) * kOut + ch] : 0.f);
+    __shared__ double red[256];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) s += lossp[i];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
     }
-}
-
-__global__ void k_loss_sum(int n, const float* __restrict__ lossp, float inv_norm, float* __restrict__ out)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < n; i++) s += lossp[i];
-        *out = (float)(s * inv_norm);
-    }
+    if (threadIdx.x == 0) *out = (float)(red[0] * inv_norm);
 }
 
 __device__ __forceinline__ float q1(int v, int i, int j, int k)
@@ -1375,7 +1542,8 @@ int grid_for(int64_t n, int threads = 256) { return (int)std::max<int64_t>(1, st
 
 struct NetHandle {
     int device = 0;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, copy = nullptr;
+    cudaEvent_t copied = nullptr;
     double E_ref = 1.0, in_scale = 1.0;
     DBuf<float> p, g, m, v;
     DBuf<__nv_bfloat16> wf, wb;
@@ -1383,7 +1551,7 @@ struct NetHandle {
     int n_data = 0;
     DBuf<float> data_x, data_y;
     int cap = 0;
-    DBuf<float> x, y, o, gnode, lossp, part, loss_dev;
+    DBuf<float> x, y, o, lossp, part, loss_dev;
     DBuf<__nv_bfloat16> a0, a1, a2, d0, d1;
     DBuf<int32_t> idx;
     DBuf<int> flag;
@@ -1393,11 +1561,16 @@ struct NetHandle {
     int sms = 148;       // multiprocessors of the device (the persistent kernel's grid)
     ~NetHandle()
     {
+        if (copied) cudaEventDestroy(copied);
+        if (copy) cudaStreamDestroy(copy);
         if (stream) cudaStreamDestroy(stream);
     }
 };
 
 namespace {
+
+// CTAs (and partials) of the weight-gradient kernels: one per multiprocessor over the units of n cells
+int grad_parts(const NetHandle& N, int n) { return std::min(8 * n, N.sms); }
 
 int net_reserve(NetHandle& N, int cap)
 {
@@ -1406,14 +1579,13 @@ int net_reserve(NetHandle& N, int cap)
     MSFEM_TRY(N.x.alloc(c * kVox));
     MSFEM_TRY(N.y.alloc(c * kNodes * kOut));
     MSFEM_TRY(N.o.alloc(c * kVox * kCh));
-    MSFEM_TRY(N.gnode.alloc(c * kNodes * kOut));
-    MSFEM_TRY(N.lossp.alloc(c));
+    MSFEM_TRY(N.lossp.alloc(c * kNodeBlocks));
     MSFEM_TRY(N.a0.alloc(c * kVox * kCh));
     MSFEM_TRY(N.a1.alloc(c * kVox * kCh));
     MSFEM_TRY(N.a2.alloc(c * kVox * kCh));
     MSFEM_TRY(N.d0.alloc(c * kVox * kCh));
     MSFEM_TRY(N.d1.alloc(c * kVox * kCh));
-    MSFEM_TRY(N.part.alloc(std::max<size_t>(c, 1) * kLayer));
+    MSFEM_TRY(N.part.alloc((size_t)grad_parts(N, cap) * kParams));
     MSFEM_TRY(N.idx.alloc(c));
     N.cap = cap;
     return 0;
@@ -1426,7 +1598,7 @@ int conv_attrs()
     MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCvSmem));
-    MSFEM_CK(cudaFuncSetAttribute(k_wgrad32, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgradSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_wgrad32, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tc<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tc<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tc<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
@@ -1482,43 +1654,27 @@ int check_err(NetHandle& N)
     return 0;
 }
 
-int wgrad_layer(NetHandle& N, int n, const __nv_bfloat16* act, const __nv_bfloat16* dz, float* grad_out)
+// after net_forward: loss and gradients of n cells (inputs N.x, targets N.y) into N.g; loss into *d_loss (device)
+int net_backward(NetHandle& N, int n, float* d_loss)
 {
     cudaStream_t st = N.stream;
-    const int n_parts = std::min(n, N.cap);
-    const int per = (n + n_parts - 1) / n_parts;
-    const int used = (n + per - 1) / per;
-    k_wgrad32<<<used, 256, kWgradSmem, st>>>(n, per, act, dz, N.part.p);
-    k_reduce_parts<<<grid_for(kLayer), 256, 0, st>>>(used, kLayer, N.part.p, grad_out);
-    MSFEM_CK(cudaGetLastError());
-    return 0;
-}
-
-// loss and gradients of n cells (inputs N.x, targets N.y) into N.g; loss into *d_loss (device)
-int net_loss_backward(NetHandle& N, int n, float* d_loss)
-{
-    cudaStream_t st = N.stream;
-    MSFEM_TRY(net_forward(N, n));
     const float inv_norm = 1.0f / ((float)n * kNodes * kOut);
-    k_loss_nodes<<<n, 256, 0, st>>>(N.o.p, N.y.p, inv_norm, N.gnode.p, N.lossp.p);
-    k_loss_sum<<<1, 32, 0, st>>>(n, N.lossp.p, inv_norm, d_loss);
-    k_dout<<<grid_for((int64_t)n * kVox * kCh), 256, 0, st>>>(n, N.gnode.p, N.d0.p);
+    k_loss_nodes<<<dim3(kNodeBlocks, n), 256, 0, st>>>(N.o.p, N.y.p, inv_norm, N.d0.p, N.lossp.p);
+    k_loss_sum<<<1, 256, 0, st>>>(n * kNodeBlocks, N.lossp.p, inv_norm, d_loss);
     const __nv_bfloat16* wb = N.wb.p;
+    const int parts = grad_parts(N, n);
     // layer 3
-    MSFEM_TRY(wgrad_layer(N, n, N.a2.p, N.d0.p, N.g.p + layer_base(3)));
+    k_wgrad32<<<parts, 256, kWgSmem, st>>>(n, N.a2.p, N.d0.p, N.part.p + layer_base(3));
     conv<kEpiMask>(N, n, N.d0.p, wb + 2 * kLayerW, nullptr, N.a2.p, N.d1.p, nullptr);
     // layer 2
-    MSFEM_TRY(wgrad_layer(N, n, N.a1.p, N.d1.p, N.g.p + layer_base(2)));
+    k_wgrad32<<<parts, 256, kWgSmem, st>>>(n, N.a1.p, N.d1.p, N.part.p + layer_base(2));
     conv<kEpiMask>(N, n, N.d1.p, wb + kLayerW, nullptr, N.a1.p, N.d0.p, nullptr);
     // layer 1
-    MSFEM_TRY(wgrad_layer(N, n, N.a0.p, N.d0.p, N.g.p + layer_base(1)));
+    k_wgrad32<<<parts, 256, kWgSmem, st>>>(n, N.a0.p, N.d0.p, N.part.p + layer_base(1));
     conv<kEpiMask>(N, n, N.d0.p, wb, nullptr, N.a0.p, N.d1.p, nullptr);
-    // layer 0
-    const int n_parts = std::min(n, N.cap);
-    const int per = (n + n_parts - 1) / n_parts;
-    const int used = (n + per - 1) / per;
-    k_first_wgrad<<<used, 256, 0, st>>>(n, per, N.x.p, N.d1.p, N.part.p);
-    k_reduce_parts<<<grid_for(kPart0), 256, 0, st>>>(used, kPart0, N.part.p, N.g.p);
+    // layer 0, and the partials of all layers
+    k_first_wgrad<<<parts, 256, 0, st>>>(n, N.x.p, N.d1.p, N.part.p);
+    k_reduce_parts<<<(kParams + 255) / 256, 256, 0, st>>>(parts, N.part.p, N.g.p);
     MSFEM_CK(cudaGetLastError());
     return 0;
 }
@@ -1607,6 +1763,8 @@ int msfem_net_create(uint64_t seed, double E_ref, double in_scale, msfem_net_t* 
     MSFEM_CK(cudaGetDevice(&h->device));
     MSFEM_CK(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
     MSFEM_CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+    MSFEM_CK(cudaStreamCreateWithFlags(&h->copy, cudaStreamNonBlocking));
+    MSFEM_CK(cudaEventCreateWithFlags(&h->copied, cudaEventDisableTiming));
     h->E_ref = E_ref;
     h->in_scale = in_scale;
     MSFEM_TRY(h->p.alloc(kParams));
@@ -1766,7 +1924,8 @@ int msfem_net_train(msfem_net_t h, int steps, int batch, float lr, uint64_t seed
     for (int k = 0; k < steps; k++) {
         k_gather<<<grid_for((int64_t)batch * (kVox + kNodes * kOut)), 256, 0, st>>>(
             batch, didx.p + (size_t)k * batch, h->data_x.p, h->data_y.p, h->x.p, h->y.p);
-        MSFEM_TRY(net_loss_backward(*h, batch, dloss.p + k));
+        MSFEM_TRY(net_forward(*h, batch));
+        MSFEM_TRY(net_backward(*h, batch, dloss.p + k));
         h->adam_t++;
         const float c1 = (float)(1.0 / (1.0 - std::pow((double)b1, (double)h->adam_t)));
         const float c2 = (float)(1.0 / (1.0 - std::pow((double)b2, (double)h->adam_t)));
@@ -1789,8 +1948,12 @@ int msfem_net_loss_grad(msfem_net_t h, int n, const float* vox, const float* tar
     MSFEM_TRY(net_reserve(*h, n));
     cudaStream_t st = h->stream;
     MSFEM_CK(cudaMemcpyAsync(h->x.p, vox, sizeof(float) * n * kVox, cudaMemcpyHostToDevice, st));
-    MSFEM_CK(cudaMemcpyAsync(h->y.p, target, sizeof(float) * n * kNodes * kOut, cudaMemcpyHostToDevice, st));
-    MSFEM_TRY(net_loss_backward(*h, n, h->loss_dev.p));
+    MSFEM_TRY(net_forward(*h, n));
+    // the targets (four fifths of the bytes) are copied on a stream of their own, under the forward pass
+    MSFEM_CK(cudaMemcpyAsync(h->y.p, target, sizeof(float) * n * kNodes * kOut, cudaMemcpyHostToDevice, h->copy));
+    MSFEM_CK(cudaEventRecord(h->copied, h->copy));
+    MSFEM_CK(cudaStreamWaitEvent(st, h->copied, 0));
+    MSFEM_TRY(net_backward(*h, n, h->loss_dev.p));
     if (loss) MSFEM_CK(cudaMemcpyAsync(loss, h->loss_dev.p, sizeof(float), cudaMemcpyDeviceToHost, st));
     if (grad) MSFEM_CK(cudaMemcpyAsync(grad, h->g.p, sizeof(float) * kParams, cudaMemcpyDeviceToHost, st));
     MSFEM_CK(cudaStreamSynchronize(st));

@@ -34,3 +34,35 @@ def test_conv_ring_gives_the_bits_of_the_cell_kernel(cuda, n):
     loss, g = net.loss_grad(vox, tgt)
     assert loss == l_ref
     np.testing.assert_array_equal(g, g_ref)
+
+
+@pytest.mark.parametrize("n", [1, 3, 19])
+def test_gradient_matches_the_oracle(cuda, n):
+    """Loss and every layer's gradient against the oracle (64 bits, the network's BF16 points) over
+    partials of one unit a block and of one or two; the bars of the two-cell test: BF16 values that fall on the
+    other side of a rounding boundary cost up to 2e-3 of a layer's gradient."""
+    net = _net(3)
+    p = on.init_params(3)
+    vox, tgt = _inputs(n, 40 + n)
+    loss, g = net.loss_grad(vox, tgt)
+    loss_ref, g_ref = on.loss_grad(p, vox, tgt)
+    assert loss == pytest.approx(loss_ref, rel=1e-4)
+    for lo, hi in [(0, on.L1), (on.layer_base(1), on.layer_base(2)), (on.layer_base(2), on.layer_base(3)),
+                   (on.layer_base(3), on.PARAMS)]:
+        assert np.linalg.norm(g[lo:hi] - g_ref[lo:hi]) <= 2e-3 * np.linalg.norm(g_ref[lo:hi])
+
+
+@pytest.mark.parametrize("n", [320, 1280])
+def test_gradient_of_a_batch_is_the_mean_of_its_eighths(cuda, n):
+    """Ranges long enough for partial sums to be put away on the way (8 units of the 32-channel layers, 64 of
+    the first).  A factor of eight in the norm is exact in every rounding, so batch and eighths have the same
+    terms and differ by the FP32 order of their sums: 1e-4, as between two kernels of one pass."""
+    net = _net(5)
+    vox, tgt = _inputs(n, n)
+    loss, g = net.loss_grad(vox, tgt)
+    parts = [net.loss_grad(vox[k::8].copy(), tgt[k::8].copy()) for k in range(8)]
+    assert loss == pytest.approx(np.mean([l for l, _ in parts]), rel=1e-5)
+    ref = np.mean([q for _, q in parts], axis=0, dtype=np.float64)
+    for lo, hi in [(0, on.L1), (on.layer_base(1), on.layer_base(2)), (on.layer_base(2), on.layer_base(3)),
+                   (on.layer_base(3), on.PARAMS)]:
+        assert np.linalg.norm(g[lo:hi] - ref[lo:hi]) <= 1e-4 * np.linalg.norm(ref[lo:hi])
