@@ -126,41 +126,142 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
 
 __device__ __forceinline__ float coord_of(int i) { return (2.0f * i + 1.0f) / kV - 1.0f; }
 
-__global__ void __launch_bounds__(256) k_first_fwd(const float* __restrict__ x, const float* __restrict__ p,
-                                                   __nv_bfloat16* __restrict__ a0)
+// packed pairs of FP32 (one instruction, each half rounded as the scalar operation)
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
 {
-    __shared__ float xs[3][18][18];
-    __shared__ float w[kTaps * kCh * kCin0 + kCh];
-    const int z = blockIdx.x, cell = blockIdx.y, tid = threadIdx.x;
-    const float* xc = x + (size_t)cell * kVox;
-    for (int q = tid; q < 3 * 18 * 18; q += blockDim.x) {
-        const int hz = q / 324, rem = q % 324, hy = rem / 18, hx = rem % 18;
-        const int gz = z - 1 + hz, gy = hy - 1, gx = hx - 1;
-        xs[hz][hy][hx] = (gz >= 0 && gz < kV && gy >= 0 && gy < kV && gx >= 0 && gx < kV) ? xc[(gz * kV + gy) * kV + gx] : 0.f;
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Thread = eight voxels along y and half the channels, as eight packed pairs; a CTA (128 threads, two
+// resident) walks a contiguous range of units of two z-planes.  A tap adds w0 I0 + w1 I1 + w2 I2 + w3 I3
+// (five roundings, in this order) to the sum; outside the cell all four inputs are zero.  The eight voxels
+// share x and with it w1 I1.  Bound by the FP32 pipe; the weights, [tap][input][channel] in shared memory,
+// are read as 16-byte broadcasts, each serving eight voxels (it writes four registers of every lane, as
+// long as four products take).  128 cells: 102 us (156 with a voxel a thread, scalar); of the FP32 rate 0.62.
+constexpr int kFirstThreads = 128;
+__global__ void __launch_bounds__(kFirstThreads, 2) k_first_fwd(int n_cells, const float* __restrict__ x,
+                                                                const float* __restrict__ p, __nv_bfloat16* __restrict__ a0)
+{
+    constexpr int V = 8, H = kCh / 2;
+    __shared__ float xs[4][18][20];
+    __shared__ __align__(16) float w[kTaps][kCin0][kCh];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int q = tid; q < kTaps * kCh; q += kFirstThreads) {
+        const float4 f = reinterpret_cast<const float4*>(p + kW0)[q];
+        float* o = &w[q / kCh][0][q % kCh];
+        o[0] = f.x;
+        o[kCh] = f.y;
+        o[2 * kCh] = f.z;
+        o[3 * kCh] = f.w;
     }
-    for (int q = tid; q < kTaps * kCh * kCin0 + kCh; q += blockDim.x) w[q] = p[kW0 + q];
-    __syncthreads();
-    const int vx = tid & 15, vy = tid >> 4;
-    float acc[kCh];
+    const int vx = lane & 15, vy = V * (lane >> 4), zl = warp >> 1, c0 = H * (warp & 1);
+    uint64_t cy[V + 2];  // y-coordinate of voxels vy - 1 .. vy + V, zero outside
 #pragma unroll
-    for (int co = 0; co < kCh; co++) acc[co] = w[kB0 + co];
-    for (int tap = 0; tap < kTaps; tap++) {
-        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-        const int gz = z + dz - 1, gy = vy + dy - 1, gx = vx + dx - 1;
-        if (gz < 0 || gz >= kV || gy < 0 || gy >= kV || gx < 0 || gx >= kV) continue;
-        const float in0 = xs[dz][vy + dy][vx + dx], in1 = coord_of(gx), in2 = coord_of(gy), in3 = coord_of(gz);
-        const float* wt = w + tap * kCh * kCin0;
-#pragma unroll
-        for (int co = 0; co < kCh; co++)
-            acc[co] += wt[4 * co] * in0 + wt[4 * co + 1] * in1 + wt[4 * co + 2] * in2 + wt[4 * co + 3] * in3;
+    for (int k = 0; k < V + 2; k++) {
+        const int gy = vy + k - 1;
+        const float c = gy >= 0 && gy < kV ? coord_of(gy) : 0.f;
+        cy[k] = pack2(c, c);
     }
-    __nv_bfloat162 o[kCh / 2];
+    const int u0 = (int)((int64_t)8 * n_cells * blockIdx.x / gridDim.x);
+    const int u1 = (int)((int64_t)8 * n_cells * (blockIdx.x + 1) / gridDim.x);
+#pragma unroll 1
+    for (int u = u0; u < u1; u++) {
+        const int z = 2 * (u & 7) + zl;
+        const float* xc = x + (size_t)(u >> 3) * kVox;
+        __syncthreads();
+        for (int q = tid; q < 4 * 18 * 20; q += kFirstThreads) {
+            const int hz = q / 360, hy = (q / 20) % 18, hx = q % 20;
+            const int gz = z - zl - 1 + hz, gy = hy - 1, gx = hx - 1;
+            xs[hz][hy][hx] = (gz >= 0 && gz < kV && gy >= 0 && gy < kV && gx >= 0 && gx < kV) ? xc[(gz * kV + gy) * kV + gx] : 0.f;
+        }
+        uint64_t acc[V][H / 2];
 #pragma unroll
-    for (int k = 0; k < kCh / 2; k++) o[k] = __floats2bfloat162_rn(fmaxf(acc[2 * k], 0.f), fmaxf(acc[2 * k + 1], 0.f));
-    uint4* dst = reinterpret_cast<uint4*>(a0 + ((size_t)cell * kVox + (z * kV + vy) * kV + vx) * kCh);
-    const uint4* src = reinterpret_cast<const uint4*>(o);
+        for (int k = 0; k < H / 2; k++) {
+            const uint64_t b = pack2(p[kB0 + c0 + 2 * k], p[kB0 + c0 + 2 * k + 1]);
 #pragma unroll
-    for (int k = 0; k < 4; k++) dst[k] = src[k];
+            for (int v = 0; v < V; v++) acc[v][k] = b;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int dz = 0; dz < 3; dz++) {
+            const int gz = z + dz - 1;
+            if (gz < 0 || gz >= kV) continue;
+            const uint64_t cz = pack2(coord_of(gz), coord_of(gz));
+            const uint64_t czl = vy ? cz : 0ull, czr = vy ? 0ull : cz;  // of the neighbours above and below the eight
+#pragma unroll
+            for (int dy = 0; dy < 3; dy++)
+#pragma unroll 1
+                for (int dx = 0; dx < 3; dx++) {
+                    const int gx = vx + dx - 1;
+                    if (gx < 0 || gx >= kV) continue;
+                    const uint64_t cx = pack2(coord_of(gx), coord_of(gx));
+                    uint64_t in[V];
+#pragma unroll
+                    for (int v = 0; v < V; v++) {
+                        const float f = xs[zl + dz][vy + v + dy][vx + dx];
+                        in[v] = pack2(f, f);
+                    }
+                    const float* wt = &w[9 * dz + 3 * dy + dx][0][c0];
+#pragma unroll
+                    for (int k = 0; k < H / 4; k++) {
+                        ulonglong2 wk[kCin0];
+#pragma unroll
+                        for (int c = 0; c < kCin0; c++) wk[c] = reinterpret_cast<const ulonglong2*>(wt + c * kCh)[k];
+                        const uint64_t x0 = mul2(wk[1].x, cx), x1 = mul2(wk[1].y, cx);
+#pragma unroll
+                        for (int v = 0; v < V; v++) {
+                            const bool low = v + dy == 0, high = v + dy == V + 1;
+                            const uint64_t iz = low ? czl : high ? czr : cz;
+                            // outside the cell w1 I1 is zero as well
+                            const uint64_t p0 = (low && !vy) || (high && vy) ? 0ull : x0, p1 = (low && !vy) || (high && vy) ? 0ull : x1;
+                            const uint64_t s0 = fma2(wk[2].x, cy[v + dy], fma2(wk[0].x, in[v], p0));
+                            const uint64_t s1 = fma2(wk[2].y, cy[v + dy], fma2(wk[0].y, in[v], p1));
+                            acc[v][2 * k] = add2(acc[v][2 * k], fma2(wk[3].x, iz, s0));
+                            acc[v][2 * k + 1] = add2(acc[v][2 * k + 1], fma2(wk[3].y, iz, s1));
+                        }
+                    }
+                }
+        }
+        uint4* dst = reinterpret_cast<uint4*>(a0 + ((size_t)(u >> 3) * kVox + (z * kV + vy) * kV + vx) * kCh + c0);
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            uint32_t o[H / 2];
+#pragma unroll
+            for (int k = 0; k < H / 2; k++) {
+                const float2 f = unpack2(acc[v][k]);
+                const __nv_bfloat162 r = __floats2bfloat162_rn(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+                o[k] = *reinterpret_cast<const uint32_t*>(&r);
+            }
+            dst[4 * kV * v] = make_uint4(o[0], o[1], o[2], o[3]);
+            dst[4 * kV * v + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+    }
 }
 
 // dW0[tap][co][c] = sum_v dZ0[v][co] I[v + tap][c], db0[co] = sum_v dZ0[v][co]; one partial per CTA
@@ -1302,15 +1403,22 @@ __device__ __forceinline__ bool is_vertex(int i, int j, int k)
     return (i == 0 || i == kN - 1) && (j == 0 || j == kN - 1) && (k == 0 || k == kN - 1);
 }
 
-// corr of node (i, j, k), channel ch, from the voxel outputs of one cell
-__device__ __forceinline__ float node_corr(const float* __restrict__ o, int i, int j, int k, int ch)
+// corr of node (i, j, k), channels 4q .. 4q+3, from the voxel outputs of one cell
+__device__ __forceinline__ float4 node_corr(const float* __restrict__ o, int i, int j, int k, int q)
 {
-    if (is_vertex(i, j, k)) return 0.f;
-    float s = 0.f;
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (is_vertex(i, j, k)) return f;
     for (int c = max(0, 2 * k - 1); c <= min(kV - 1, 2 * k); c++)
         for (int b = max(0, 2 * j - 1); b <= min(kV - 1, 2 * j); b++)
-            for (int a = max(0, 2 * i - 1); a <= min(kV - 1, 2 * i); a++) s += o[((c * kV + b) * kV + a) * kCh + ch];
-    return s / (float)(node_count(i) * node_count(j) * node_count(k));
+            for (int a = max(0, 2 * i - 1); a <= min(kV - 1, 2 * i); a++) {
+                const float4 v = reinterpret_cast<const float4*>(o)[((c * kV + b) * kV + a) * 8 + q];
+                f.x += v.x;
+                f.y += v.y;
+                f.z += v.z;
+                f.w += v.w;
+            }
+    const float cnt = (float)(node_count(i) * node_count(j) * node_count(k));
+    return make_float4(f.x / cnt, f.y / cnt, f.z / cnt, f.w / cnt);
 }
 
 // Thread (node, four channels) of one cell: the corrections of the node from its up to eight voxels, the
@@ -1324,7 +1432,6 @@ __global__ void __launch_bounds__(256) k_loss_nodes(const float* __restrict__ o,
                                                     float inv_norm, __nv_bfloat16* __restrict__ d0, float* __restrict__ lossp)
 {
     const int cell = blockIdx.y, item = blockIdx.x * 256 + threadIdx.x;
-    const float4* oc = reinterpret_cast<const float4*>(o + (size_t)cell * kVox * kCh);
     uint2* dc = reinterpret_cast<uint2*>(d0 + (size_t)cell * kVox * kCh);
     float s = 0.f;
     if (item < kNodeItems) {
@@ -1335,20 +1442,10 @@ __global__ void __launch_bounds__(256) k_loss_nodes(const float* __restrict__ o,
         const int c0 = max(0, 2 * k - 1), c1 = min(kV - 1, 2 * k);
         __nv_bfloat162 g01 = __floats2bfloat162_rn(0.f, 0.f), g23 = g01;
         if (q < kOut / 4) {
-            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!zero)
-                for (int c = c0; c <= c1; c++)
-                    for (int b = b0; b <= b1; b++)
-                        for (int a = a0; a <= a1; a++) {
-                            const float4 v = oc[((c * kV + b) * kV + a) * 8 + q];
-                            f.x += v.x;
-                            f.y += v.y;
-                            f.z += v.z;
-                            f.w += v.w;
-                        }
+            const float4 f = node_corr(o + (size_t)cell * kVox * kCh, i, j, k, q);
             const float cnt = (float)(node_count(i) * node_count(j) * node_count(k));
             const float4 t = reinterpret_cast<const float4*>(y + (size_t)cell * kNodes * kOut + n * kOut)[q];
-            const float e0 = f.x / cnt - t.x, e1 = f.y / cnt - t.y, e2 = f.z / cnt - t.z, e3 = f.w / cnt - t.w;
+            const float e0 = f.x - t.x, e1 = f.y - t.y, e2 = f.z - t.z, e3 = f.w - t.w;
             s = e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
             if (!zero) {
                 g01 = __floats2bfloat162_rn(2.f * e0 * inv_norm / cnt, 2.f * e1 * inv_norm / cnt);
@@ -1418,24 +1515,28 @@ __global__ void k_targets(int n_cells, int c_first, const int64_t* __restrict__ 
     }
 }
 
-// bases of cells c_first .. c_first + n - 1 from the L3 output of this chunk
-__global__ void k_predict(int n_cells, int c_first, const float* __restrict__ o, const int64_t* __restrict__ node_off,
-                          double* __restrict__ bx)
+// bases of cells c_first .. c_first + n - 1 from the L3 output of this chunk: thread = (node, four
+// channels) of one cell, up to eight 16-byte loads.  Bound by HBM: 512 cells 55 us (a channel a thread: 86)
+__global__ void __launch_bounds__(256) k_predict(int c_first, const float* __restrict__ o,
+                                                 const int64_t* __restrict__ node_off, double* __restrict__ bx)
 {
-    const int64_t total = (int64_t)n_cells * kNodes * kOut;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const int cell = (int)(q / (kNodes * kOut)), r = (int)(q % (kNodes * kOut));
-        const int n = r / kOut, ch = r % kOut, v = ch / 3;
-        const int i = n % kN, j = (n / kN) % kN, k = n / (kN * kN);
-        const float corr = node_corr(o + (size_t)cell * kVox * kCh, i, j, k, ch);
-        bx[(node_off[c_first + cell] + n) * 24 + ch] = (double)q1(v, i, j, k) + (double)corr;
-    }
+    const int cell = blockIdx.y, item = blockIdx.x * 256 + threadIdx.x;
+    if (item >= kNodes * (kOut / 4)) return;
+    const int n = item / (kOut / 4), q = item % (kOut / 4);
+    const int i = n % kN, j = (n / kN) % kN, k = n / (kN * kN);
+    const float4 f = node_corr(o + (size_t)cell * kVox * kCh, i, j, k, q);
+    const float c[4] = {f.x, f.y, f.z, f.w};
+    double r[4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) r[m] = (double)q1((4 * q + m) / 3, i, j, k) + (double)c[m];
+    double2* dst = reinterpret_cast<double2*>(bx + (node_off[c_first + cell] + n) * 24 + 4 * q);
+    dst[0] = make_double2(r[0], r[1]);
+    dst[1] = make_double2(r[2], r[3]);
 }
 
 // ------------------------------------------------------------------ voxels and cell checks
 
 __constant__ int c_kuhn_order[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-__constant__ int c_kuhn_corners[6][4] = {{0, 1, 3, 7}, {0, 1, 5, 7}, {0, 2, 3, 7}, {0, 2, 6, 7}, {0, 4, 5, 7}, {0, 4, 6, 7}};
 
 // share of octant oct (bit a: upper half along axis a) of a hexahedron inside Kuhn tetrahedron t
 // (coordinates ordered as c_kuhn_order[t], largest first): zero unless the octant's halves are
@@ -1454,46 +1555,54 @@ __device__ float kuhn_share(int oct, int t)
     return mine ? 1.f / (float)n : 0.f;
 }
 
-__global__ void k_voxelise(int n_cells, const int64_t* __restrict__ tet_off, const int32_t* __restrict__ mat,
-                           const double* __restrict__ logE, int n_mat, float* __restrict__ vox)
+// thread = one hexahedron of a cell (two CTAs a cell): its eight voxels from its six tetrahedra; 512 cells
+// 9 us (the shares worked out voxel by voxel: 86)
+__global__ void __launch_bounds__(256) k_voxelise(const int64_t* __restrict__ tet_off, const int32_t* __restrict__ mat,
+                                                  const double* __restrict__ logE, int n_mat, float* __restrict__ vox)
 {
-    const int64_t total = (int64_t)n_cells * kVox;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const int cell = (int)(q / kVox), v = (int)(q % kVox);
-        const int vx = v & 15, vy = (v >> 4) & 15, vz = v >> 8;
-        const int hex = (vx >> 1) + 8 * ((vy >> 1) + 8 * (vz >> 1));
-        const int oct = (vx & 1) | ((vy & 1) << 1) | ((vz & 1) << 2);
-        double s = 0.0;
-        for (int t = 0; t < 6; t++) {
-            const float f = kuhn_share(oct, t);
-            if (f == 0.f) continue;
-            int m = mat[tet_off[cell] + 6 * hex + t];
-            m = min(max(m, 0), n_mat - 1);  // ids were range-checked when the cells were created
-            s += (double)f * logE[m];
+    __shared__ float share[8][6];
+    if (threadIdx.x < 48) share[threadIdx.x / 6][threadIdx.x % 6] = kuhn_share(threadIdx.x / 6, threadIdx.x % 6);
+    __syncthreads();
+    const int cell = blockIdx.x >> 1, hex = 256 * (blockIdx.x & 1) + threadIdx.x;
+    double e[6];
+#pragma unroll
+    for (int t = 0; t < 6; t++) {
+        const int m = mat[tet_off[cell] + 6 * hex + t];
+        e[t] = logE[min(max(m, 0), n_mat - 1)];  // ids were range-checked when the cells were created
+    }
+    float2* out = reinterpret_cast<float2*>(vox + (size_t)cell * kVox) + (hex & 7) + kV * ((hex >> 3) & 7) + kV * kV * (hex >> 6);
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        float v[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            double s = 0.0;
+            for (int t = 0; t < 6; t++) {
+                const float f = share[2 * p + h][t];
+                if (f != 0.f) s += (double)f * e[t];
+            }
+            v[h] = (float)s;
         }
-        vox[q] = (float)s;
+        out[(p & 1) * (kV / 2) + (p >> 1) * (kV * kV / 2)] = make_float2(v[0], v[1]);
     }
 }
 
-__global__ void k_check_kuhn8(int n_cells, const int64_t* __restrict__ node_off, const int64_t* __restrict__ tet_off,
-                              const int32_t* __restrict__ elems, int* bad)
+// twelve CTAs a cell, a tetrahedron a thread
+__global__ void __launch_bounds__(256) k_check_kuhn8(const int64_t* __restrict__ node_off, const int64_t* __restrict__ tet_off,
+                                                     const int32_t* __restrict__ elems, int* bad)
 {
-    const int64_t total = (int64_t)n_cells * kTets;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const int cell = (int)(q / kTets), e = (int)(q % kTets);
-        if (node_off[cell + 1] - node_off[cell] != kNodes || tet_off[cell + 1] - tet_off[cell] != kTets) {
-            atomicExch(bad, 1);
-            continue;
-        }
-        const int hex = e / 6, t = e % 6;
-        const int hi = hex % 8, hj = (hex / 8) % 8, hk = hex / 64;
-        const int32_t* nd = elems + 4 * (tet_off[cell] + e);
-        for (int c = 0; c < 4; c++) {
-            const int b = c_kuhn_corners[t][c];
-            const int want = (hi + (b & 1)) + kN * ((hj + ((b >> 1) & 1)) + kN * (hk + ((b >> 2) & 1)));
-            if ((int64_t)nd[c] - node_off[cell] != want) atomicExch(bad, 1);
-        }
+    const int cell = blockIdx.x / (kTets / 256), e = 256 * (blockIdx.x % (kTets / 256)) + threadIdx.x;
+    if (node_off[cell + 1] - node_off[cell] != kNodes || tet_off[cell + 1] - tet_off[cell] != kTets) {
+        atomicExch(bad, 1);
+        return;
     }
+    const int hex = e / 6, t = e % 6;
+    const int4 nd = reinterpret_cast<const int4*>(elems)[tet_off[cell] + e];
+    // corners 0, 2^a, 2^a + 2^b, 7 of tetrahedron t (the orders in the header)
+    const int b1 = 1 << (t >> 1), b2 = (0x656353 >> (4 * t)) & 7;
+    const int first = hex % 8 + kN * ((hex / 8) % 8 + kN * (hex / 64));
+    auto node = [&](int b) { return node_off[cell] + first + (b & 1) + kN * (((b >> 1) & 1) + kN * (b >> 2)); };
+    if (nd.x != node(0) || nd.y != node(b1) || nd.z != node(b2) || nd.w != node(7)) atomicExch(bad, 1);
 }
 
 // ------------------------------------------------------------------ optimiser
@@ -1633,7 +1742,7 @@ int net_forward(NetHandle& N, int n)
     cudaStream_t st = N.stream;
     MSFEM_TRY(conv_attrs());
     const __nv_bfloat16* wf = N.wf.p;
-    k_first_fwd<<<dim3(kV, n), 256, 0, st>>>(N.x.p, N.p.p, N.a0.p);
+    k_first_fwd<<<std::min(8 * n, 2 * N.sms), kFirstThreads, 0, st>>>(n, N.x.p, N.p.p, N.a0.p);
     conv<kEpiRelu>(N, n, N.a0.p, wf, N.p.p + layer_base(1) + kLayerW, nullptr, N.a1.p, nullptr);
     conv<kEpiRelu>(N, n, N.a1.p, wf + kLayerW, N.p.p + layer_base(2) + kLayerW, nullptr, N.a2.p, nullptr);
     conv<kEpiF32>(N, n, N.a2.p, wf + 2 * kLayerW, N.p.p + layer_base(3) + kLayerW, nullptr, nullptr, N.o.p);
@@ -1705,8 +1814,7 @@ int check_cells(NetHandle& N, CellsHandle& C)
     MSFEM_TRY(N.flag.alloc(1));
     MSFEM_CK(cudaMemsetAsync(N.flag.p, 0, sizeof(int), N.stream));
     MSFEM_CK(cudaStreamSynchronize(C.stream));
-    k_check_kuhn8<<<grid_for((int64_t)C.n_cells * kTets), 256, 0, N.stream>>>(C.n_cells, C.node_off.p, C.tet_off.p,
-                                                                              C.vols.elems.p, N.flag.p);
+    k_check_kuhn8<<<C.n_cells * (kTets / 256), 256, 0, N.stream>>>(C.node_off.p, C.tet_off.p, C.vols.elems.p, N.flag.p);
     MSFEM_CK(cudaGetLastError());
     int bad = 0;
     MSFEM_CK(cudaMemcpyAsync(&bad, N.flag.p, sizeof(int), cudaMemcpyDeviceToHost, N.stream));
@@ -1848,7 +1956,7 @@ int msfem_net_voxelise(msfem_net_t h, msfem_cells_t cells, float* vox)
     DBuf<float> dv;
     MSFEM_TRY(log_moduli(*h, C, le));
     MSFEM_TRY(dv.alloc((size_t)C.n_cells * kVox));
-    k_voxelise<<<grid_for((int64_t)C.n_cells * kVox), 256, 0, h->stream>>>(C.n_cells, C.tet_off.p, C.mat.p, le.p, C.n_mat, dv.p);
+    k_voxelise<<<2 * C.n_cells, 256, 0, h->stream>>>(C.tet_off.p, C.mat.p, le.p, C.n_mat, dv.p);
     MSFEM_CK(cudaGetLastError());
     MSFEM_CK(cudaMemcpyAsync(vox, dv.p, sizeof(float) * C.n_cells * kVox, cudaMemcpyDeviceToHost, h->stream));
     MSFEM_CK(cudaStreamSynchronize(h->stream));
@@ -1875,8 +1983,7 @@ int msfem_net_add_cells(msfem_net_t h, msfem_cells_t cells, int* n_total)
     }
     DBuf<double> le;
     MSFEM_TRY(log_moduli(*h, C, le));
-    k_voxelise<<<grid_for((int64_t)C.n_cells * kVox), 256, 0, st>>>(C.n_cells, C.tet_off.p, C.mat.p, le.p, C.n_mat,
-                                                                    nx.p + n_old * kVox);
+    k_voxelise<<<2 * C.n_cells, 256, 0, st>>>(C.tet_off.p, C.mat.p, le.p, C.n_mat, nx.p + n_old * kVox);
     DBuf<uint8_t> wild;
     MSFEM_TRY(wild.alloc(C.n_cells));
     k_wild_targets<<<C.n_cells, 256, 0, st>>>(0, C.node_off.p, C.bx.p, wild.p);
@@ -1997,10 +2104,10 @@ int msfem_net_predict(msfem_net_t h, msfem_cells_t cells, float* ms)
     int rc = 0;
     for (int c0 = 0; c0 < C.n_cells && rc == 0; c0 += chunk) {
         const int n = std::min(chunk, C.n_cells - c0);
-        k_voxelise<<<grid_for((int64_t)n * kVox), 256, 0, st>>>(n, C.tet_off.p + c0, C.mat.p, le.p, C.n_mat, h->x.p);
+        k_voxelise<<<2 * n, 256, 0, st>>>(C.tet_off.p + c0, C.mat.p, le.p, C.n_mat, h->x.p);
         rc = net_forward(*h, n);
         if (rc == 0)
-            k_predict<<<grid_for((int64_t)n * kNodes * kOut), 256, 0, st>>>(n, c0, h->o.p, C.node_off.p, C.bx.p);
+            k_predict<<<dim3((kNodes * (kOut / 4) + 255) / 256, n), 256, 0, st>>>(c0, h->o.p, C.node_off.p, C.bx.p);
     }
     MSFEM_CK(cudaEventRecord(e1, st));
     MSFEM_CK(cudaEventSynchronize(e1));

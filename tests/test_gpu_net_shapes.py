@@ -66,3 +66,16 @@ def test_gradient_of_a_batch_is_the_mean_of_its_eighths(cuda, n):
     for lo, hi in [(0, on.L1), (on.layer_base(1), on.layer_base(2)), (on.layer_base(2), on.layer_base(3)),
                    (on.layer_base(3), on.PARAMS)]:
         assert np.linalg.norm(g[lo:hi] - ref[lo:hi]) <= 1e-4 * np.linalg.norm(ref[lo:hi])
+
+
+@pytest.mark.parametrize("n", [1, 2, 38])
+def test_forward_matches_the_oracle(cuda, n):
+    """The first layer's ranges of plane pairs (fewer than two a multiprocessor, and more) through to the
+    output, cell by cell at the bar of the few-cell test (BF16 rounding boundaries)."""
+    net = _net(9)
+    vox, _ = _inputs(n, 70 + n)
+    vox *= np.linspace(0.2, 3.0, 16, dtype=np.float32).repeat(256)  # no two planes alike
+    out = net.forward(vox)
+    for k in sorted({0, n // 2, n - 1}):
+        ref = on.forward(on.init_params(9), vox[k:k + 1])[0][1]
+        assert np.linalg.norm(out[k] - ref) <= 5e-3 * np.linalg.norm(ref), k
