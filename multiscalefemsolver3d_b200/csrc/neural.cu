@@ -17,7 +17,7 @@
 //          average of s ln(E / E_ref) (exact Kuhn-tetrahedron volume fractions per voxel),
 //          c = 1..3: the voxel centre in [-1, 1]^3; zero outside the cell (zero padding)
 //   L0     3x3x3 conv 4 -> 32, bias, ReLU           FP32 CUDA cores, output BF16
-//   L1, L2 3x3x3 conv 32 -> 32, bias, ReLU          BF16 tensor cores (mma m16n8k16), FP32 accumulate
+//   L1, L2 3x3x3 conv 32 -> 32, bias, ReLU          BF16 tensor cores, FP32 accumulate
 //   L3     3x3x3 conv 32 -> 24 (padded to 32), bias  same kernel, FP32 output
 //   node   corr[n][3 v + a] = mean of L3 over the voxels touching node n (a partition: voxel x
 //          belongs to node (x + 1) / 2 along each axis), zero at the 8 cell vertices
@@ -1200,6 +1200,300 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_conv32_ws(int n_cells, const 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(kWsTmemCols));
 }
 
+// ---- pieces of k_conv32_st
+__device__ __forceinline__ constexpr uint32_t st_idesc(int n)  // BF16 x BF16 -> FP32, M = 128, N = n
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.b32 %0, 1, 0, P;\n\t}\n" : "=r"(p));
+    return p;
+}
+
+__device__ __forceinline__ void st_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc));
+}
+
+__device__ __forceinline__ void tc_load32(uint32_t (&v)[32], uint32_t taddr)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+        "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+__device__ __forceinline__ void tc_zero32(uint32_t taddr)
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};\n" ::"r"(taddr),
+        "r"(0)
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+}
+
+// one voxel's 32 sums through the epilogue; the lanes of a quad hold neighbouring voxels and exchange 16-byte
+// pieces, so that a store covers whole voxels
+template <int EPI>
+__device__ __forceinline__ void tc_store_voxel(const uint32_t (&v)[32], size_t vox, const float* __restrict__ bias,
+                                               const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* __restrict__ out,
+                                               float* __restrict__ outf)
+{
+    const int t = threadIdx.x & 3;
+    const size_t vox0 = vox - t;
+    if (EPI == kEpiF32) {
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            uint4 r[4];  // component c of the four pieces -> the four components ...
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                float f[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int ch = 16 * half + 4 * k + c;
+                    f[k] = __uint_as_float(v[ch]) + bias[ch];
+                }
+                r[c] = quad_transpose(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]), t);
+            }
+            // ... of piece t of the four voxels
+            uint4* o = reinterpret_cast<uint4*>(outf + vox0 * kCh) + 4 * half + t;
+            o[0] = make_uint4(r[0].x, r[1].x, r[2].x, r[3].x);
+            o[8] = make_uint4(r[0].y, r[1].y, r[2].y, r[3].y);
+            o[16] = make_uint4(r[0].z, r[1].z, r[2].z, r[3].z);
+            o[24] = make_uint4(r[0].w, r[1].w, r[2].w, r[3].w);
+        }
+    } else {
+        uint32_t wd[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            float f0 = __uint_as_float(v[2 * k]), f1 = __uint_as_float(v[2 * k + 1]);
+            if (EPI == kEpiRelu) {
+                f0 = fmaxf(f0 + bias[2 * k], 0.f);
+                f1 = fmaxf(f1 + bias[2 * k + 1], 0.f);
+            }
+            const __nv_bfloat162 r = __floats2bfloat162_rn(f0, f1);
+            wd[k] = *reinterpret_cast<const uint32_t*>(&r);
+        }
+        uint4 r[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) r[c] = quad_transpose(wd[c], wd[4 + c], wd[8 + c], wd[12 + c], t);
+        uint4 o[4] = {make_uint4(r[0].x, r[1].x, r[2].x, r[3].x), make_uint4(r[0].y, r[1].y, r[2].y, r[3].y),
+                      make_uint4(r[0].z, r[1].z, r[2].z, r[3].z), make_uint4(r[0].w, r[1].w, r[2].w, r[3].w)};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (EPI == kEpiMask) {
+                const uint4 m = reinterpret_cast<const uint4*>(mask + (vox0 + j) * kCh)[t];
+                o[j].x = positive_only(o[j].x, m.x);
+                o[j].y = positive_only(o[j].y, m.y);
+                o[j].z = positive_only(o[j].z, m.z);
+                o[j].w = positive_only(o[j].w, m.w);
+            }
+            reinterpret_cast<uint4*>(out + (vox0 + j) * kCh)[t] = o[j];
+        }
+    }
+}
+
+// ---- the convolution on tcgen05 with the three z-taps stacked (the default).
+// An input plane p meets, for each of the nine (dy, dx) and two k16 halves, the weights of all three dz at
+// once: M = 128 voxels (16 y rows x 8 x of one x-half), N = 96 = 32 channels of the output planes p - 1
+// (dz = 2), p (dz = 1), p + 1 (dz = 0).  So a plane costs 36 instructions, each of which reads its 4 KB of
+// voxels once for three output planes (k_conv32_ws: 216 of M = 64, N = 32).  An output plane still sums
+// dz, dy, dx, k half in this order: the bits of the other paths.
+// Operands are K-major, no-swizzle, as in k_conv32_tc; the weights are [chunk][dy dx][2 - dz][co] x 16 B, so
+// the rows of any run of output planes are contiguous.  The accumulators of an x-half are a ring of eight
+// 32-column slots in TMEM (both halves: all 512 columns); a run of output planes that wraps around the ring
+// is two instructions.  Every instruction accumulates: the epilogue writes zeros to a slot that it has read.
+// Instructions of one plane on one half have one shape and accumulator and run in order; those of the next
+// plane overlap them in part, which the hardware does not order, so a plane is issued when the last one has
+// completed.  The two halves alternate, so that consecutive instructions are independent.
+// A plane has one completion barrier: it frees the ring slot, lets the next plane go and tells the epilogue
+// of the output that it completes.  (No waiter can miss a phase: plane g + 8 begins an output that needs the
+// slot of one drained after the output that plane g completes.)
+//   warps 0-7   epilogue, x-half = warp / 4, TMEM lanes 32 (warp % 4) ..
+//   warp 8      producer: planes into a ring of eight slots (cp.async), three in flight
+//   warp 9      one thread issues
+// A CTA walks a contiguous range of output planes, cell by cell; at a cut inside a cell it reads one more
+// plane on either side and multiplies it for the planes it owns.  The planes outside the cell are zero and
+// left out.  Waits are bounded as in k_conv32_ws.
+// Bound by the issue and the operand reads of the instructions (a plane: 2.1 us, 1.4 of them; one of M = 128,
+// K = 16 takes 60 clocks up to N = 96) and the wait between planes.  A layer of 518 cells: 117 us; k_conv32 276
+// (mma.sync alone 212 at its rate).  Both halves of a plane back to back instead of alternating: 167; issued
+// behind `lane == 0`: 212.
+constexpr int kStSlots = 8;
+constexpr int kStW = kStSlots * kTcSlot;                    // weights after the ring
+constexpr int kStWChunk = 9 * 96 * 16;                      // 13,824 B
+constexpr int kStBar = kStW + 4 * kStWChunk;
+constexpr int kStNBar = 3 * kStSlots;                       // full, done, drained
+constexpr int kStSmem = kStBar + 8 * kStNBar + 16;
+constexpr int kStThreads = 320;
+
+template <int EPI>
+__global__ void __launch_bounds__(kStThreads, 1) k_conv32_st(int n_cells, const __nv_bfloat16* __restrict__ in,
+                                                             const __nv_bfloat16* __restrict__ w,
+                                                             const float* __restrict__ bias,
+                                                             const __nv_bfloat16* __restrict__ mask,
+                                                             __nv_bfloat16* __restrict__ out, float* __restrict__ outf,
+                                                             int* err)
+{
+    extern __shared__ __align__(128) unsigned char sm[];
+    const uint32_t bar0 = smem_u32(sm + kStBar);
+    auto full = [&](int s) { return bar0 + 8u * s; };
+    auto done = [&](int s) { return bar0 + 8u * (kStSlots + s); };
+    auto drained = [&](int s) { return bar0 + 8u * (2 * kStSlots + s); };
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kStBar + 8 * kStNBar);
+    volatile int* abort = reinterpret_cast<volatile int*>(sm + kStBar + 8 * kStNBar + 4);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < kStSlots; s++) {
+            mb_init(full(s), 32);
+            mb_init(done(s), 1);
+            mb_init(drained(s), 8);
+        }
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(tslot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    for (int q = tid; q < kTaps * kCh * 4; q += kStThreads) {
+        const int row = q >> 2, c = q & 3, tap = row / kCh, co = row % kCh;
+        cp_async16(smem_u32(sm) + kStW + c * kStWChunk + ((tap % 9) * 96 + (2 - tap / 9) * kCh + co) * 16,
+                   w + (size_t)row * kCh + c * 8);
+    }
+    const int t0 = (int)((int64_t)kV * n_cells * blockIdx.x / gridDim.x);
+    const int t1 = (int)((int64_t)kV * n_cells * (blockIdx.x + 1) / gridDim.x);
+    const int lead = (t0 & 15) ? 1 : 0;  // plane q of output t is plane number t - t0 + lead of this CTA
+    cv_zero_borders(sm, min(kStSlots, t1 - t0 + 2));
+    cp_async_wait_all();
+    asm volatile("fence.proxy.async.shared::cta;\n" ::);
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+    const uint32_t tbase = *tslot;
+    const uint32_t tmine = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + 256u * ((warp >> 2) & 1);
+    if (warp < 8)
+        for (int s = 0; s < min(kStSlots, t1 - t0); s++) tc_zero32(tmine + 32 * s);
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+
+    if (warp == 8) {
+        int g = 0;  // planes so far; plane g in slot g % kStSlots
+        const uint32_t dst0 = smem_u32(sm) + (lane & 3) * kTcChunk + kTcRow + 16 + (lane >> 2) * 16;
+        bool ok = true;
+        for (int t = t0; t < t1 && ok;) {
+            const int qa = t & 15, qb = min(kV, qa + t1 - t);
+            const __nv_bfloat16* src = in + (size_t)(t >> 4) * kVox * kCh + lane * 8;
+            for (int p = max(qa - 1, 0); p <= min(qb, kV - 1); p++, g++) {
+                const int s = g & (kStSlots - 1);
+                if (g >= kStSlots && !__all_sync(0xffffffffu, ws_wait(done(s), (g / kStSlots - 1) & 1, abort))) {
+                    ok = false;
+                    break;
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i++)
+                    cp_async16(dst0 + s * kTcSlot + (i >> 1) * kTcRow + (i & 1) * 128, src + (size_t)p * 256 * kCh + i * 256);
+                asm volatile("cp.async.commit_group;\n" ::);
+                if (g >= 2) {
+                    asm volatile("cp.async.wait_group 2;\n" ::);
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::);
+                    mb_arrive(full((g - 2) & (kStSlots - 1)));
+                }
+            }
+            t += qb - qa;
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::);
+        if (ok)
+            for (int k = max(g - 2, 0); k < g; k++) mb_arrive(full(k & (kStSlots - 1)));
+    } else if (warp == 9) {
+        // one thread, chosen by elect.sync: the compiler then knows that it is one and issues an instruction in
+        // 60 clocks; behind `lane == 0` it loops over the active lanes to make the operands uniform (150)
+        if (elect_one()) {
+            const uint32_t a0 = smem_u32(sm), b0 = smem_u32(sm) + kStW;
+            int g = 0, o0 = 0;  // planes so far; outputs before this segment: output q is number o0 + q - qa
+            bool ok = true;
+            for (int t = t0; t < t1 && ok;) {
+                const int qa = t & 15, qb = min(kV, qa + t1 - t);
+                int fresh = qa;  // the next output not yet begun
+                for (int p = max(qa - 1, 0); p <= min(qb, kV - 1); p++, g++) {
+                    const int s = g & (kStSlots - 1), lo = max(p - 1, qa), hi = min(p + 1, qb - 1);
+                    ok = ws_wait(full(s), (g / kStSlots) & 1, abort);
+                    for (; fresh <= hi && ok; fresh++) {
+                        const int o = o0 + fresh - qa;
+                        if (o >= kStSlots) ok = ws_wait(drained(o & (kStSlots - 1)), (o / kStSlots - 1) & 1, abort);
+                    }
+                    if (ok && g > 0) ok = ws_wait(done((g - 1) & (kStSlots - 1)), ((g - 1) / kStSlots) & 1, abort);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+                    // one run of columns, or two where it wraps
+                    const int c0 = (o0 + lo - qa) & (kStSlots - 1), n0 = min(hi - lo + 1, kStSlots - c0), n1 = hi - lo + 1 - n0;
+                    const uint32_t d0 = tbase + 32u * c0, d1 = tbase;
+                    const uint32_t i0 = st_idesc(32 * n0), i1 = st_idesc(32 * n1);
+                    const uint64_t ad = tc_desc(a0 + s * kTcSlot, kTcChunk, kTcRow);
+                    const uint64_t bd = tc_desc(b0 + 32 * (lo - p + 1) * 16, kStWChunk, 128);
+#pragma unroll
+                    for (int k = 0; k < 18; k++) {
+                        const int dy = k / 6, dx = (k / 2) % 3, kc = k & 1;
+                        const uint64_t a = ad + ((2 * kc * kTcChunk + (dy * 18 + dx) * 16) >> 4);
+                        const uint64_t b = bd + ((2 * kc * kStWChunk + (3 * dy + dx) * 96 * 16) >> 4);
+                        st_mma(d0, a, b, i0);
+                        st_mma(d0 + 256, a + 8, b, i0);
+                        if (n1 > 0) {
+                            st_mma(d1, a, b + 32 * n0, i1);
+                            st_mma(d1 + 256, a + 8, b + 32 * n0, i1);
+                        }
+                    }
+                    // the plane's slot is free, and its last output complete
+                    tc_commit(done(s));
+                }
+                o0 += qb - qa;
+                t += qb - qa;
+            }
+            // every issued MMA has completed before the CTA frees TMEM
+            if (g > 0 && !tc_wait(done((g - 1) & (kStSlots - 1)), ((g - 1) / kStSlots) & 1)) *abort = 1;
+        }
+        __syncwarp();
+    } else {
+        const int h = warp >> 2;
+        int o = 0;
+        for (int t = t0; t < t1; t++, o++) {
+            // complete with plane q + 1, the cell's last with its own
+            const int s = o & (kStSlots - 1), g = o + lead + ((t & 15) == kV - 1 ? 0 : 1);
+            if (!__all_sync(0xffffffffu, ws_wait(done(g & (kStSlots - 1)), (g / kStSlots) & 1, abort))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+            uint32_t v[32];
+            tc_load32(v, tmine + 32 * s);
+            tc_zero32(tmine + 32 * s);
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+            __syncwarp();
+            if (lane == 0) mb_arrive(drained(s));
+            const int y = 4 * (warp & 3) + (lane >> 3), xv = 8 * h + (lane & 7);
+            tc_store_voxel<EPI>(v, ((size_t)(t >> 4) * kV + (t & 15)) * 256 + y * kV + xv, bias, mask, out, outf);
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+    if (*abort && tid == 0) atomicExch(err, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tbase));
+}
+
 // dW[tap][co][ci] = sum_v dZ[v][co] A[v + tap][ci] and db[co] = sum_v dZ[v][co] over a contiguous
 // range of units (two z-planes of one cell; one fixed-order partial per CTA).  M = co (two m16 tiles, A
 // operand = dZ^T through ldmatrix.trans), N = ci (four n8 tiles, B operand = shifted activations through
@@ -1649,6 +1943,9 @@ int grid_for(int64_t n, int threads = 256) { return (int)std::max<int64_t>(1, st
 
 }  // namespace
 
+// layers 1-3 unless the caller selects a path: tcgen05, z-taps stacked (k_conv32_st)
+constexpr int kStacked = 4;
+
 struct NetHandle {
     int device = 0;
     cudaStream_t stream = nullptr, copy = nullptr;
@@ -1665,8 +1962,8 @@ struct NetHandle {
     DBuf<int32_t> idx;
     DBuf<int> flag;
     DBuf<int> err;       // set by a tcgen05 kernel whose completion wait timed out
-    int tcgen05 = 0;     // layers 1-3: 0 mma.sync (k_conv32), 1 tcgen05 M=64 tiles (k_conv32_tc), 2 tcgen05 transposed
-                         // (k_conv32_tt), 3 tcgen05 M=64 tiles warp-specialised and persistent (k_conv32_ws)
+    int tcgen05 = kStacked;  // or, selected by the caller: 0 mma.sync (k_conv32), 1 tcgen05 M=64 tiles (k_conv32_tc), 2
+                             // tcgen05 transposed (k_conv32_tt), 3 M=64 tiles warp-specialised (k_conv32_ws)
     int sms = 148;       // multiprocessors of the device (the persistent kernel's grid)
     ~NetHandle()
     {
@@ -1714,19 +2011,26 @@ int conv_attrs()
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tt<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTtSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tt<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTtSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_tt<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTtSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_conv32_st<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_ws<kEpiRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWsSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_conv32_st<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_ws<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWsSmem));
+    MSFEM_CK(cudaFuncSetAttribute(k_conv32_st<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem));
     MSFEM_CK(cudaFuncSetAttribute(k_conv32_ws<kEpiMask>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWsSmem));
     done = true;
     return 0;
 }
 
-// one 32 -> 32 convolution of n cells on the selected tensor-core path
+// one 32 -> 32 convolution of n cells on the selected tensor-core path.  k_conv32_st is the default at every
+// size: a prediction of 9, 37, 128 and 512 cells takes 167, 195, 336 and 871 us with it, 176, 225, 458 and 1359
+// with k_conv32, and the bits are the same; the others run where the caller asks for them.
 template <int EPI>
 void conv(NetHandle& N, int n, const __nv_bfloat16* in, const __nv_bfloat16* w, const float* bias, const __nv_bfloat16* mask,
           __nv_bfloat16* out, float* outf)
 {
-    if (N.tcgen05 == 3)
+    if (N.tcgen05 == kStacked)
+        k_conv32_st<EPI><<<std::min(kV * n, N.sms), kStThreads, kStSmem, N.stream>>>(n, in, w, bias, mask, out, outf, N.err.p);
+    else if (N.tcgen05 == 3)
         k_conv32_ws<EPI><<<std::min(n, N.sms), kWsThreads, kWsSmem, N.stream>>>(n, in, w, bias, mask, out, outf, N.err.p);
     else if (N.tcgen05 == 2)
         k_conv32_tt<EPI><<<n, 128, kTtSmem, N.stream>>>(in, w, bias, mask, out, outf, N.err.p);

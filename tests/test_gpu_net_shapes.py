@@ -79,3 +79,40 @@ def test_forward_matches_the_oracle(cuda, n):
     for k in sorted({0, n // 2, n - 1}):
         ref = on.forward(on.init_params(9), vox[k:k + 1])[0][1]
         assert np.linalg.norm(out[k] - ref) <= 5e-3 * np.linalg.norm(ref), k
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 10, 19, 37, 38, 301])
+def test_stacked_taps_give_the_bits_of_the_cell_kernel(cuda, n):
+    """The default path (k_conv32_st: three z-taps an instruction, rings of planes and of accumulators,
+    ranges of output planes cut anywhere in a cell) against the tcgen05 kernel that takes a cell a block.
+    The products of each sum are added in one order, so all bits agree: ranges of one plane (n <= 9), of one
+    or two, ranges that end on every plane of a cell (19, 37, 38), and long ones that go round both rings."""
+    net, ref = _net(13), _net(13)
+    ref.set_tensor_path(1)
+    vox, tgt = _inputs(n, 100 + n)
+    np.testing.assert_array_equal(net.forward(vox), ref.forward(vox))
+    (loss, g), (l_ref, g_ref) = net.loss_grad(vox, tgt), ref.loss_grad(vox, tgt)
+    assert loss == l_ref
+    np.testing.assert_array_equal(g, g_ref)
+
+
+def test_default_path_is_repeatable_from_two_threads(cuda):
+    """Two networks on two threads: their kernels take whole multiprocessors (all of the tensor memory) in
+    turn."""
+    import threading
+    vox, _ = _inputs(200, 1)
+    nets = [_net(1), _net(2)]
+    ref = [net.forward(vox) for net in nets]
+    got = [None, None]
+
+    def work(k):
+        for _ in range(4):
+            got[k] = nets[k].forward(vox)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=60)
+    for k in range(2):
+        np.testing.assert_array_equal(got[k], ref[k])
