@@ -126,49 +126,19 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
 
 __device__ __forceinline__ float coord_of(int i) { return (2.0f * i + 1.0f) / kV - 1.0f; }
 
-// packed pairs of FP32 (one instruction, each half rounded as the scalar operation)
-__device__ __forceinline__ uint64_t pack2(float lo, float hi)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// Thread = eight voxels along y and half the channels, as eight packed pairs; a CTA (128 threads, two
-// resident) walks a contiguous range of units of two z-planes.  A tap adds w0 I0 + w1 I1 + w2 I2 + w3 I3
-// (five roundings, in this order) to the sum; outside the cell all four inputs are zero.  The eight voxels
-// share x and with it w1 I1.  Bound by the FP32 pipe; the weights, [tap][input][channel] in shared memory,
-// are read as 16-byte broadcasts, each serving eight voxels (it writes four registers of every lane, as
-// long as four products take).  128 cells: 102 us (156 with a voxel a thread, scalar); of the FP32 rate 0.62.
+// Thread = the sixteen voxels of a y column and a quarter of the channels; a CTA (128 threads, two resident)
+// walks a contiguous range of units of two z-planes.  A tap adds w0 I0 + w1 I1 + w2 I2 + w3 I3 (five
+// roundings, in this order) to the sum; outside the cell nothing.  The column shares x and with it w1 I1, and
+// its y-coordinates are constants.  Bound by the FP32 pipe and by the weights' way from shared memory ([tap]
+// [input][channel]; a 16-byte broadcast writes four registers of every lane, as long as four products take),
+// each of which serves sixteen voxels.  128 cells: 91 us; eight voxels and half the channels 98, the same in
+// packed pairs 102 (a loop of fma.rn.f32x2 on distinct registers runs at 0.61 of the FP32 rate, of scalar ones
+// at 0.81), a voxel a thread 156.
 constexpr int kFirstThreads = 128;
 __global__ void __launch_bounds__(kFirstThreads, 2) k_first_fwd(int n_cells, const float* __restrict__ x,
                                                                 const float* __restrict__ p, __nv_bfloat16* __restrict__ a0)
 {
-    constexpr int V = 8, H = kCh / 2;
+    constexpr int V = kV, H = kCh / 4;
     __shared__ float xs[4][18][20];
     __shared__ __align__(16) float w[kTaps][kCin0][kCh];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -180,14 +150,7 @@ __global__ void __launch_bounds__(kFirstThreads, 2) k_first_fwd(int n_cells, con
         o[2 * kCh] = f.z;
         o[3 * kCh] = f.w;
     }
-    const int vx = lane & 15, vy = V * (lane >> 4), zl = warp >> 1, c0 = H * (warp & 1);
-    uint64_t cy[V + 2];  // y-coordinate of voxels vy - 1 .. vy + V, zero outside
-#pragma unroll
-    for (int k = 0; k < V + 2; k++) {
-        const int gy = vy + k - 1;
-        const float c = gy >= 0 && gy < kV ? coord_of(gy) : 0.f;
-        cy[k] = pack2(c, c);
-    }
+    const int vx = lane & 15, zl = warp >> 1, c0 = H * (2 * (warp & 1) + (lane >> 4));
     const int u0 = (int)((int64_t)8 * n_cells * blockIdx.x / gridDim.x);
     const int u1 = (int)((int64_t)8 * n_cells * (blockIdx.x + 1) / gridDim.x);
 #pragma unroll 1
@@ -200,10 +163,10 @@ __global__ void __launch_bounds__(kFirstThreads, 2) k_first_fwd(int n_cells, con
             const int gz = z - zl - 1 + hz, gy = hy - 1, gx = hx - 1;
             xs[hz][hy][hx] = (gz >= 0 && gz < kV && gy >= 0 && gy < kV && gx >= 0 && gx < kV) ? xc[(gz * kV + gy) * kV + gx] : 0.f;
         }
-        uint64_t acc[V][H / 2];
+        float acc[V][H];
 #pragma unroll
-        for (int k = 0; k < H / 2; k++) {
-            const uint64_t b = pack2(p[kB0 + c0 + 2 * k], p[kB0 + c0 + 2 * k + 1]);
+        for (int k = 0; k < H; k++) {
+            const float b = p[kB0 + c0 + k];
 #pragma unroll
             for (int v = 0; v < V; v++) acc[v][k] = b;
         }
@@ -212,54 +175,52 @@ __global__ void __launch_bounds__(kFirstThreads, 2) k_first_fwd(int n_cells, con
         for (int dz = 0; dz < 3; dz++) {
             const int gz = z + dz - 1;
             if (gz < 0 || gz >= kV) continue;
-            const uint64_t cz = pack2(coord_of(gz), coord_of(gz));
-            const uint64_t czl = vy ? cz : 0ull, czr = vy ? 0ull : cz;  // of the neighbours above and below the eight
+            const float cz = coord_of(gz);
 #pragma unroll
             for (int dy = 0; dy < 3; dy++)
 #pragma unroll 1
                 for (int dx = 0; dx < 3; dx++) {
                     const int gx = vx + dx - 1;
                     if (gx < 0 || gx >= kV) continue;
-                    const uint64_t cx = pack2(coord_of(gx), coord_of(gx));
-                    uint64_t in[V];
+                    const float cx = coord_of(gx);
+                    float in[V];
 #pragma unroll
-                    for (int v = 0; v < V; v++) {
-                        const float f = xs[zl + dz][vy + v + dy][vx + dx];
-                        in[v] = pack2(f, f);
-                    }
+                    for (int v = 0; v < V; v++) in[v] = xs[zl + dz][v + dy][vx + dx];
                     const float* wt = &w[9 * dz + 3 * dy + dx][0][c0];
 #pragma unroll
                     for (int k = 0; k < H / 4; k++) {
-                        ulonglong2 wk[kCin0];
+                        float wk[kCin0][4];
 #pragma unroll
-                        for (int c = 0; c < kCin0; c++) wk[c] = reinterpret_cast<const ulonglong2*>(wt + c * kCh)[k];
-                        const uint64_t x0 = mul2(wk[1].x, cx), x1 = mul2(wk[1].y, cx);
+                        for (int c = 0; c < kCin0; c++) {
+                            const float4 f = reinterpret_cast<const float4*>(wt + c * kCh)[k];
+                            wk[c][0] = f.x;
+                            wk[c][1] = f.y;
+                            wk[c][2] = f.z;
+                            wk[c][3] = f.w;
+                        }
 #pragma unroll
-                        for (int v = 0; v < V; v++) {
-                            const bool low = v + dy == 0, high = v + dy == V + 1;
-                            const uint64_t iz = low ? czl : high ? czr : cz;
-                            // outside the cell w1 I1 is zero as well
-                            const uint64_t p0 = (low && !vy) || (high && vy) ? 0ull : x0, p1 = (low && !vy) || (high && vy) ? 0ull : x1;
-                            const uint64_t s0 = fma2(wk[2].x, cy[v + dy], fma2(wk[0].x, in[v], p0));
-                            const uint64_t s1 = fma2(wk[2].y, cy[v + dy], fma2(wk[0].y, in[v], p1));
-                            acc[v][2 * k] = add2(acc[v][2 * k], fma2(wk[3].x, iz, s0));
-                            acc[v][2 * k + 1] = add2(acc[v][2 * k + 1], fma2(wk[3].y, iz, s1));
+                        for (int q = 0; q < 4; q++) {
+                            const float wx = __fmul_rn(wk[1][q], cx);
+#pragma unroll
+                            for (int v = 0; v < V; v++) {
+                                if (v + dy == 0 || v + dy == V + 1) continue;  // outside the cell
+                                const float t = __fmaf_rn(wk[2][q], coord_of(v + dy - 1), __fmaf_rn(wk[0][q], in[v], wx));
+                                acc[v][4 * k + q] = __fadd_rn(acc[v][4 * k + q], __fmaf_rn(wk[3][q], cz, t));
+                            }
                         }
                     }
                 }
         }
-        uint4* dst = reinterpret_cast<uint4*>(a0 + ((size_t)(u >> 3) * kVox + (z * kV + vy) * kV + vx) * kCh + c0);
+        uint4* dst = reinterpret_cast<uint4*>(a0 + ((size_t)(u >> 3) * kVox + z * 256 + vx) * kCh + c0);
 #pragma unroll
         for (int v = 0; v < V; v++) {
             uint32_t o[H / 2];
 #pragma unroll
             for (int k = 0; k < H / 2; k++) {
-                const float2 f = unpack2(acc[v][k]);
-                const __nv_bfloat162 r = __floats2bfloat162_rn(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+                const __nv_bfloat162 r = __floats2bfloat162_rn(fmaxf(acc[v][2 * k], 0.f), fmaxf(acc[v][2 * k + 1], 0.f));
                 o[k] = *reinterpret_cast<const uint32_t*>(&r);
             }
             dst[4 * kV * v] = make_uint4(o[0], o[1], o[2], o[3]);
-            dst[4 * kV * v + 1] = make_uint4(o[4], o[5], o[6], o[7]);
         }
     }
 }
