@@ -182,8 +182,13 @@ struct EpiStoreZ {
     }
     __device__ __forceinline__ void finish() {}
 };
-// the z-marching configurations: 16 x 16 hexahedron columns (15 x 15 owned nodes); FP32 two CTAs
-// per SM, FP64 one
-constexpr int kKzTX = 16, kKzTY = 16, kKzMinB = 2, kKzMinB64 = 1;
+// The z-marching configurations: 16 x 8 hexahedron columns (15 x 7 owned nodes); FP32 four CTAs per SM,
+// FP64 two.  A step is a long chain (six tetrahedra a thread, one barrier), so a grid that does not fill the
+// SMs evenly waits for the fullest one; CTAs of four warps divide it finer than those of eight, and on large
+// grids four independent CTAs hide each other's barriers better than two, which outweighs the wider overlap of
+// the smaller tile.  A smoother step at 24^3, 32^3, 40^3, 64^3, 128^3, us: 16 x 8: 4.7, 5.9, 7.7, 17.5, 93;
+// 16 x 16: 5.4, 8.5, 9.3, 19.3, 95; 8 x 8: 5.3, 6.5, 8.4, 20.4, 120; 16 x 6: 4.7, 5.8, 7.7, 17.0, 98; 32 x 8: 4.7, 8.0,
+// 8.2, 21.0, 93; 24 x 8: 5.6, 6.5, 8.5, 18.0, 97.
+constexpr int kKzTX = 16, kKzTY = 8, kKzMinB = 4, kKzMinB64 = 2;
 
 }  // namespace msfem

@@ -1666,7 +1666,7 @@ void mg_cycle(CoarseHandle& C, const double* z, const double* r2, double* r_out,
     };
     // The cycle is a chain of kernels of 4 to 13 us at 40^3, so it is launched as one (launch_chained): the
     // next kernel's launch and its set-up overlap the end of the last.  A MINRES iteration at 24^3, 40^3,
-    // 64^3 and 128^3 took 98, 152, 314 and 1551 us with plain launches and takes 80, 135, 298 and 1535.
+    // 64^3 and 128^3 took 98, 152, 314 and 1551 us with plain launches and 80, 135, 298 and 1535 chained.
     // Only the kernels of a few blocks and the z-marches at their last step call chain_next: with it at the
     // head of the long vector kernels as well, the waiting blocks crowd the SMs (98, 147, 333 and 1752 us).
     launch_chained(k_mg_in, gvec, kVecThreads, 0, st, n, z, r2, r_out, s_t, rhat, res, dA, x, C.cc, S, lanczos,
