@@ -12,7 +12,9 @@ namespace msfem {
 // as every block of this kernel is resident; chain_wait holds until the predecessor has completed and
 // its writes are visible, and comes before the first access to anything an earlier kernel of the
 // chain reads or writes; what was complete before the chain began may be read ahead of it.  Every block
-// waits (or has nothing to do), so that a kernel's completion implies that of all before it.  In a
+// waits (or has nothing to do), so that a kernel's completion implies that of all before it.  What an
+// earlier kernel of the chain writes is read by ordinary loads, not as constant data (no __ldg, no const
+// __restrict__): it changes while the reader is already resident.  In a
 // kernel launched the plain way both do nothing.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_z(KzArgs<T> A, Epi epi)
 #pragma unroll
             for (int q = 0; q < Epi::NE; q++)
 #pragma unroll
-                for (int a = 0; a < 3; a++) e[q][a] = __ldg(ev[q] + 3 * gk + a);
+                for (int a = 0; a < 3; a++) e[q][a] = ev[q][3 * gk + a];
         }
         // slab kz: this thread's hexahedron
         {
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_kuhn_zp(KzArgs<T> A, Epi epi)
 #pragma unroll
             for (int q = 0; q < Epi::NE; q++)
 #pragma unroll
-                for (int a = 0; a < 3; a++) e[q][a] = __ldg(ev[q] + 3 * gk + a);
+                for (int a = 0; a < 3; a++) e[q][a] = ev[q][3 * gk + a];
         }
         // slab kz: this thread's hexahedron
         {

@@ -412,7 +412,7 @@ __global__ void k_pack_sym(const double* __restrict__ A, int64_t ld, int n, cons
 // lanes of a row, column sums over the lane pair (l, l+16) and then the 8 warps in shared memory,
 // in fixed orders.  Persistent: CTA c takes blocks c, c + grid, ...
 __global__ void __launch_bounds__(256) k_tl_symv(int nb, int n_blocks, const int2* __restrict__ blocks,
-                                                 const float* __restrict__ P, const float* __restrict__ x,
+                                                 const float* __restrict__ P, const float* x,
                                                  float* __restrict__ part, const TlState* S)
 {
     __shared__ float colp[8][kSymB];
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(256) k_tl_symv(int nb, int n_blocks, const int
 #pragma unroll
             for (int k = 0; k < 4; k++) an[k] = __ldcs(nxt + t + 256 * k);
         }
-        const float4 xq = __ldg(reinterpret_cast<const float4*>(x + J * kSymB) + cq);
+        const float4 xq = reinterpret_cast<const float4*>(x + J * kSymB)[cq];
         float xi[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) xi[k] = x[I * kSymB + r0 + 16 * k];
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(256) k_tl_symv(int nb, int n_blocks, const int
 }
 
 // y[i] = sum over block columns K of part[i / 64][K][i % 64], K ascending
-__global__ void k_tl_symv_sum(int n_pad, int nb, const float* __restrict__ part, float* __restrict__ y,
+__global__ void k_tl_symv_sum(int n_pad, int nb, const float* part, float* __restrict__ y,
                               const TlState* S)
 {
     chain_next();
@@ -503,7 +503,7 @@ constexpr int kRestrictThreads = 256;
 template <class VT>
 __global__ void __launch_bounds__(kRestrictThreads)
     k_tl_restrict(const int32_t* __restrict__ own_ptr, const int32_t* __restrict__ own,
-                  const float* __restrict__ psi_hat, const VT* __restrict__ z, const VT* __restrict__ r2,
+                  const float* __restrict__ psi_hat, const VT* z, const VT* r2,
                   VT* __restrict__ out, float* __restrict__ cpart, const double* __restrict__ s, const TlState* S,
                   int lanczos)
 {
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(kRestrictThreads)
 
 // coarse residual: rc[d] = sum of the cell partials of coarse DOF d (fixed order)
 __global__ void k_tl_gather(int n_cf, const int32_t* __restrict__ dptr, const int32_t* __restrict__ dent,
-                            const float* __restrict__ cpart, float* __restrict__ rc, const TlState* S)
+                            const float* cpart, float* __restrict__ rc, const TlState* S)
 {
     chain_next();
     chain_wait();
@@ -704,8 +704,8 @@ __global__ void __launch_bounds__(256) k_tl_spmv(SellView<VT> A, const VT* __res
 // w_new = (v - oldeps w1 - delta w2) / gamma (over w1); x += phi w_new.  Runs on the step that
 // set the stopping flag (its update), not after.
 template <class VT>
-__global__ void __launch_bounds__(kVecThreads) k_tl_update(int n, const VT* __restrict__ v, VT* __restrict__ w1,
-                                                          const VT* __restrict__ w2, VT* __restrict__ x,
+__global__ void __launch_bounds__(kVecThreads) k_tl_update(int n, const VT* v, VT* __restrict__ w1,
+                                                          const VT* w2, VT* __restrict__ x,
                                                           TlState* S)
 {
     chain_wait();
@@ -884,7 +884,7 @@ struct ChebCoef {
 // rhat = S_t r_new; res = rhat; d = rhat / theta; x = d; and, for the matrix-free smoother (dh
 // non-null), dh = s d with the eliminated columns zero (s32: the operator's FP32 Jacobi scale,
 // fixw: its Dirichlet words, bit 3 + c of node i / 3 for component c)
-__global__ void __launch_bounds__(kVecThreads) k_mg_in(int n, const double* __restrict__ z, const double* __restrict__ r2,
+__global__ void __launch_bounds__(kVecThreads) k_mg_in(int n, const double* z, const double* r2,
                                                       double* __restrict__ out, const double* __restrict__ st,
                                                       float* __restrict__ rhat, float* __restrict__ res,
                                                       float* __restrict__ d, float* __restrict__ x, ChebCoef cc,
@@ -970,7 +970,7 @@ struct EpiMinresZ {
     static constexpr int NE = 1;  // r1
     double* __restrict__ v;
     double* __restrict__ z;
-    const double* __restrict__ r1;
+    const double* r1;
     TlState* S;
     double* __restrict__ partial;
     double acc;
@@ -1018,7 +1018,7 @@ struct EpiChebP {
     float* __restrict__ dh;
     float* __restrict__ res;
     float* __restrict__ x;
-    const float* __restrict__ dprev;
+    const float* dprev;
     const float* __restrict__ scale;
     float a, b;
     const TlState* S;
@@ -1057,12 +1057,12 @@ struct EpiChebP {
 // d = res / theta, dh = s d (masked, the next step's input) and x2 = x + d
 struct EpiResidP {
     static constexpr int NE = 3;  // rhat, x, the Jacobi scale
-    const float* __restrict__ rhat;
+    const float* rhat;
     float* __restrict__ res;
     float* __restrict__ d;
     float* __restrict__ dh;
     float* __restrict__ x2;
-    const float* __restrict__ x;
+    const float* x;
     const float* __restrict__ scale;
     float inv_theta;
     const TlState* S;
@@ -1101,7 +1101,7 @@ using KMinres = KzKernel<1, false, double, kKzTX, kKzTY, kKzMinB64, EpiMinresZ>;
 // input: s32 the operator's FP32 Jacobi scale, fixw its Dirichlet words)
 __global__ void __launch_bounds__(kVecThreads) k_mg_prolong(int n_fine, const int32_t* __restrict__ owner,
                                                            const int32_t* __restrict__ cdof,
-                                                           const float* __restrict__ psi, const float* __restrict__ ec,
+                                                           const float* __restrict__ psi, const float* ec,
                                                            float* __restrict__ x, const TlState* S,
                                                            const float* __restrict__ s32,
                                                            const uint32_t* __restrict__ fixw, float* __restrict__ xh)
@@ -1134,8 +1134,8 @@ __global__ void __launch_bounds__(kVecThreads) k_mg_prolong(int n_fine, const in
 }
 
 // exit of the cycle: y = S_t x (FP64), bb = (r, y) and the Givens step
-__global__ void __launch_bounds__(kVecThreads) k_mg_out(int n, const float* __restrict__ x, const double* __restrict__ st,
-                                                       const double* __restrict__ r, double* __restrict__ y, TlState* S,
+__global__ void __launch_bounds__(kVecThreads) k_mg_out(int n, const float* x, const double* __restrict__ st,
+                                                       const double* r, double* __restrict__ y, TlState* S,
                                                        double* __restrict__ partial, int init)
 {
     chain_wait();
