@@ -159,8 +159,8 @@ struct MrRhs {
 // numbers in the same order).
 template <int R>
 struct CtaShared {
-    double red[2][16 * R];             // partials per warp
-    double slot[2][kMaxCluster * R];   // partials per CTA, written by every CTA of the cluster
+    double red[4][16 * R];             // partials per warp
+    double slot[4][kMaxCluster * R];   // partials per CTA, written by every CTA of the cluster
     double s1[R], s2[R];
     MrRhs mr[R];
     double rr_prev[R];
@@ -180,6 +180,10 @@ struct Place {
 // sums a[] over the cluster for every right-hand side, in a fixed order: warp shuffles, the warps of
 // a CTA, then the CTAs by rank.  One CTA barrier and one cluster barrier, which also makes the
 // vectors written before it visible to the whole cluster.
+//
+// The slots are read after that barrier, so a buffer may be written again only when another cluster
+// barrier has passed: two sums in a row never share one.  The residual takes buffers 2 and 3, the
+// Krylov sums 0 and 1 in turn.
 template <int R, int N>
 __device__ __forceinline__ void cluster_sum(CtaShared<R>& sh, const Place<R>& P, const int (&buf)[N],
                                             double (&a)[N][Lanes<R>::NR])
@@ -264,7 +268,7 @@ __device__ void residual_pass(const BatchArgs& A, const Place<R>& P, VT* V, CtaS
             o.store(V + ((int64_t)row * 3 + c) * R + P.j * L::NR);
         }
     }
-    const int buf[2] = {0, 1};
+    const int buf[2] = {2, 3};  // the first Krylov sum follows with no cluster barrier between
     cluster_sum<R, 2>(sh, P, buf, acc);
     if (threadIdx.x < L::LPR)
 #pragma unroll
