@@ -7,6 +7,7 @@
 #include "internal.cuh"
 #include "kuhn.cuh"
 #include "kuhn25.cuh"
+#include "zmarch_grid.h"
 
 namespace msfem {
 
@@ -38,6 +39,11 @@ struct KzKernel {
         prepared |= bit;
         return cudaSuccess;
     }
+    // the CTAs of a launch; prepare() first
+    static ZmarchGrid grid(const KuhnView<T>& K, int sms)
+    {
+        return zmarch_grid(K.nx, K.ny, K.nz, L::OX, L::OY, (int64_t)blocks_per_sm * sms);
+    }
     // The bulk copies need 16-byte-aligned sources (and read up to 12 bytes past a vector's last
     // element, so every staged vector carries 16 bytes of slack): refused here, never launched.
     static bool aligned(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -54,24 +60,12 @@ struct KzKernel {
         A.K = K;
         A.x = x;
         A.err = err;
-        A.tiles_x = (K.nx + 1 + L::OX - 1) / L::OX;
-        A.tiles_y = (K.ny + 1 + L::OY - 1) / L::OY;
-        const int nnz = K.nz + 1, tiles = A.tiles_x * A.tiles_y;
-        // z segments: the count that minimises waves x steps per CTA (a segment of s layers takes
-        // s + 1 steps; the CTAs run in ceil(tiles * segments / resident CTAs) waves)
-        const int64_t slots = (int64_t)blocks_per_sm * sms;
-        int64_t best = -1;
-        for (int n_seg = 1; n_seg <= nnz; n_seg++) {
-            const int len = (nnz + n_seg - 1) / n_seg;
-            const int segs = (nnz + len - 1) / len;
-            const int64_t cost = ((int64_t)tiles * segs + slots - 1) / slots * (len + 1);
-            if (best < 0 || cost < best) {
-                best = cost;
-                A.seg_len = len;
-                A.n_seg = segs;
-            }
-        }
-        return launch_chained(K.iso ? kernel_iso : kernel_aniso, tiles * A.n_seg, L::THREADS, L::smem, st, A, epi);
+        const ZmarchGrid g = grid(K, sms);
+        A.tiles_x = g.tiles_x;
+        A.tiles_y = g.tiles_y;
+        A.seg_len = g.seg_len;
+        A.n_seg = g.n_seg;
+        return launch_chained(K.iso ? kernel_iso : kernel_aniso, (unsigned)g.ctas(), L::THREADS, L::smem, st, A, epi);
     }
 };
 
@@ -104,6 +98,11 @@ struct KzpKernel {
         prepared |= bit;
         return cudaSuccess;
     }
+    // the CTAs of a launch; prepare() first
+    static ZmarchGrid grid(const KuhnView<T>& K, int sms)
+    {
+        return zmarch_grid(K.nx, K.ny, K.nz, L::OX, L::OY, (int64_t)blocks_per_sm * sms);
+    }
     // 16-byte-aligned sources with 16 bytes of slack, as KzKernel
     static bool aligned(const void* p) { return ((uintptr_t)p & 15) == 0; }
     static cudaError_t launch(const KuhnView<T>& K, const T* x, const Epi& epi, int sms, int* err, cudaStream_t st)
@@ -119,22 +118,12 @@ struct KzpKernel {
         A.K = K;
         A.x = x;
         A.err = err;
-        A.tiles_x = (K.nx + 1 + L::OX - 1) / L::OX;
-        A.tiles_y = (K.ny + 1 + L::OY - 1) / L::OY;
-        const int nnz = K.nz + 1, tiles = A.tiles_x * A.tiles_y;
-        const int64_t slots = (int64_t)blocks_per_sm * sms;
-        int64_t best = -1;
-        for (int n_seg = 1; n_seg <= nnz; n_seg++) {
-            const int len = (nnz + n_seg - 1) / n_seg;
-            const int segs = (nnz + len - 1) / len;
-            const int64_t cost = ((int64_t)tiles * segs + slots - 1) / slots * (len + 1);
-            if (best < 0 || cost < best) {
-                best = cost;
-                A.seg_len = len;
-                A.n_seg = segs;
-            }
-        }
-        return launch_chained(K.iso ? kernel_iso : kernel_aniso, tiles * A.n_seg, L::THREADS, L::smem, st, A, epi);
+        const ZmarchGrid g = grid(K, sms);
+        A.tiles_x = g.tiles_x;
+        A.tiles_y = g.tiles_y;
+        A.seg_len = g.seg_len;
+        A.n_seg = g.n_seg;
+        return launch_chained(K.iso ? kernel_iso : kernel_aniso, (unsigned)g.ctas(), L::THREADS, L::smem, st, A, epi);
     }
 };
 

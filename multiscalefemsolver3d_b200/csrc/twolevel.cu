@@ -1243,6 +1243,7 @@ struct CoarseHandle {
     int storage = 0;
     KuhnOperator kt;      // matrix-free textbook operator (storage 2)
     KuhnOperator ka;      // matrix-free reference operator for MINRES's products (msfem_coarse_set_matrix_free)
+    DBuf<double> zpart;   // its inner product's partial sums, one per CTA: the grid follows from the box and has no bound
     bool mf_fine = false;
     ~CoarseHandle()
     {
@@ -1717,6 +1718,10 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
     mg_cycle(C, R[1], nullptr, nullptr, Y, 0, 1, st);
     const SellView<double> A = sell_view<double>(F);
     const unsigned gsp = spmv_grid_of((const void*)k_tl_spmv<double>, F);
+    if (C.mf_fine && KMinres::grid(C.ka.v64, C.ka.sms).ctas() > (int64_t)C.zpart.n) {
+        set_error("two-level MINRES: the matrix-free product's partial sums do not fit their buffer");
+        return MSFEM_ERR_ARGUMENT;
+    }
     auto two = [&]() {
         for (int p = 0; p < 2; p++) {
             double* r1 = R[p];
@@ -1724,8 +1729,7 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
             double* w1 = Wb[p];
             double* w2 = Wb[1 - p];
             if (C.mf_fine)
-                KMinres::launch(C.ka.v64, Y, EpiMinresZ{V, Z, r1, S, C.partial.p + 2048, 0.0}, C.ka.sms, C.ka.err.p,
-                                st);
+                KMinres::launch(C.ka.v64, Y, EpiMinresZ{V, Z, r1, S, C.zpart.p, 0.0}, C.ka.sms, C.ka.err.p, st);
             else
                 k_tl_spmv<double><<<gsp, 256, 0, st>>>(A, Y, V, Z, r1, S, C.partial.p + 2048);
             mg_cycle(C, Z, r2, r1, Y, 1, 0, st);  // r2_new over r1's buffer, then y = M^-1 r2_new
@@ -2159,6 +2163,7 @@ int msfem_coarse_set_matrix_free(msfem_coarse_t c, int on)
     if (!on) return MSFEM_OK;
     MSFEM_TRY(kuhn_operator_build(*C.fine, 1, true, false, C.ka));
     MSFEM_CK(KMinres::prepare());
+    MSFEM_TRY(C.zpart.alloc((size_t)KMinres::grid(C.ka.v64, C.ka.sms).ctas()));
     C.mf_fine = true;
     return MSFEM_OK;
 }
