@@ -321,9 +321,13 @@ struct GmShape {
         out->rows = (A.n_slices + out->G - 1) / out->G * kSlice * A.bs;
         const size_t small = sizeof(double) * (4 * (size_t)(m + 1) + 3 * (size_t)m) + 1024;
         const size_t w = sizeof(double) * out->rows, v = sizeof(VT) * (size_t)(m + 1) * out->rows;
-        const bool vs = small + w + v <= (size_t)most;
+        // beside the kernels' own (static) arrays, which count against the same limit
+        cudaFuncAttributes fs{}, fg{};
+        MSFEM_CK(cudaFuncGetAttributes(&fs, (const void*)k_gm_coop<VT, true>));
+        MSFEM_CK(cudaFuncGetAttributes(&fg, (const void*)k_gm_coop<VT, false>));
+        const bool vs = small + w + v + fs.sharedSizeBytes <= (size_t)most;
         out->basis_shared = vs;
-        out->w_shared = small + w <= (size_t)most;
+        out->w_shared = vs || small + w + fg.sharedSizeBytes <= (size_t)most;
         out->threads = vs ? 512 : 1024;
         out->smem = small + (out->w_shared ? w : 0) + (vs ? v : 0);
         out->kernel = vs ? (const void*)k_gm_coop<VT, true> : (const void*)k_gm_coop<VT, false>;
