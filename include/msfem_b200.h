@@ -24,7 +24,8 @@
  *    (Library/CSSD_Matrix.h:11-15).  Structural zeros are kept.
  *  - One handle = one system on one device with its own CUDA stream.  Calls on
  *    different handles may run concurrently from different host threads; calls
- *    on the same handle must not.
+ *    on the same handle must not.  A CG or GMRES solve is one kernel on every
+ *    multiprocessor: what other handles launch meanwhile may wait for its end.
  */
 #ifndef MSFEM_B200_H
 #define MSFEM_B200_H

@@ -313,25 +313,23 @@ struct GmShape {
     bool w_shared, basis_shared;
     static int make(const SellView<VT>& A, int m, GmShape* out)
     {
-        int dev = 0, sms = 0, most = 0;
+        int dev = 0, sms = 0;
         MSFEM_CK(cudaGetDevice(&dev));
         MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        MSFEM_CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        const void *in_shared = (const void*)k_gm_coop<VT, true>, *in_global = (const void*)k_gm_coop<VT, false>;
+        size_t room_s = 0, room_g = 0;
+        MSFEM_TRY(open_shared_memory(in_shared, &room_s));
+        MSFEM_TRY(open_shared_memory(in_global, &room_g));
         out->G = std::max(1, std::min(sms, A.n_slices));
         out->rows = (A.n_slices + out->G - 1) / out->G * kSlice * A.bs;
         const size_t small = sizeof(double) * (4 * (size_t)(m + 1) + 3 * (size_t)m) + 1024;
         const size_t w = sizeof(double) * out->rows, v = sizeof(VT) * (size_t)(m + 1) * out->rows;
-        // beside the kernels' own (static) arrays, which count against the same limit
-        cudaFuncAttributes fs{}, fg{};
-        MSFEM_CK(cudaFuncGetAttributes(&fs, (const void*)k_gm_coop<VT, true>));
-        MSFEM_CK(cudaFuncGetAttributes(&fg, (const void*)k_gm_coop<VT, false>));
-        const bool vs = small + w + v + fs.sharedSizeBytes <= (size_t)most;
+        const bool vs = small + w + v <= room_s;
         out->basis_shared = vs;
-        out->w_shared = vs || small + w + fg.sharedSizeBytes <= (size_t)most;
+        out->w_shared = vs || small + w <= room_g;
         out->threads = vs ? 512 : 1024;
         out->smem = small + (out->w_shared ? w : 0) + (vs ? v : 0);
-        out->kernel = vs ? (const void*)k_gm_coop<VT, true> : (const void*)k_gm_coop<VT, false>;
-        MSFEM_CK(cudaFuncSetAttribute(out->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out->smem));
+        out->kernel = vs ? in_shared : in_global;
         return MSFEM_OK;
     }
 };

@@ -227,6 +227,10 @@ int ensure_kstate(System& s);
 int solve(System& s, int method, int precision, int restart_m, int maxiter, double tol, double* relres, int* iters);
 int ensure_state(System& s);
 int read_state(System& s);
+// Lets `kernel` be launched with all the shared memory that a block of it can have on the current device; room: the
+// dynamic part, what its own arrays leave.  The limit belongs to the kernel and not to a handle, so it is always
+// set to this one value: another thread's solve of another size finds it the same.
+int open_shared_memory(const void* kernel, size_t* room);
 // ---- CG in one cooperative launch (krylov_coop.cu): S->tol2 set; iter, rr, done, breakdown left in
 // the host's KState mirror.  FP64 from the residual r; FP32 from x = 0 with right-hand side r, to tol
 // times its norm, or until (r, r) has not set a 2 % low for stall_limit iterations

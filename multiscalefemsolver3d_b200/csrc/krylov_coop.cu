@@ -565,7 +565,8 @@ int coop_shape(System& s, int vectors, size_t width, bool col16, CoopArgs& P, Co
 
 int coop_launch(System& s, const void* kernel, const CoopShape& c, CoopArgs& P, void** args)
 {
-    MSFEM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
+    size_t room = 0;
+    MSFEM_TRY(open_shared_memory(kernel, &room));
     const size_t bytes = 16 + sizeof(double) * 4 * (size_t)c.G;
     MSFEM_TRY(s.coop.alloc(bytes));
     MSFEM_CK(cudaMemsetAsync(s.coop.p, 0, 16, s.stream));
@@ -599,6 +600,18 @@ const void* cg2_kernel(int mode, int bs)
 }
 
 }  // namespace
+
+int open_shared_memory(const void* kernel, size_t* room)
+{
+    int dev = 0, most = 0;
+    cudaFuncAttributes a{};
+    MSFEM_CK(cudaGetDevice(&dev));
+    MSFEM_CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    MSFEM_CK(cudaFuncGetAttributes(&a, kernel));
+    *room = (size_t)most - a.sharedSizeBytes;
+    MSFEM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*room));
+    return MSFEM_OK;
+}
 
 int pcg64_coop(System& s, bool jacobi, double* x, double* r, double* p, double* q, double* z, int maxiter)
 {
