@@ -231,6 +231,9 @@ int read_state(System& s);
 // dynamic part, what its own arrays leave.  The limit belongs to the kernel and not to a handle, so it is always
 // set to this one value: another thread's solve of another size finds it the same.
 int open_shared_memory(const void* kernel, size_t* room);
+// the columns of an SM's share of the rows reach over more than half of the system (nodes in no spatial order): the
+// gathered vector has no window, and its loads need the L1
+bool scattered_columns(const System& s);
 // ---- CG in one cooperative launch (krylov_coop.cu): S->tol2 set; iter, rr, done, breakdown left in
 // the host's KState mirror.  FP64 from the residual r; FP32 from x = 0 with right-hand side r, to tol
 // times its norm, or until (r, r) has not set a 2 % low for stall_limit iterations

@@ -6,11 +6,12 @@
 // written to global memory by its owners; a CTA then copies the range that its columns span (its
 // window) into shared memory once per iteration and gathers there.
 //
-// Two forms, by what fits the shared memory beside the window:
+// Three forms, by what fits the shared memory beside the window:
 //  - kResident: the CTA's share of the matrix too, copied once; several warps share a slice, each with
 //    every W-th column chunk of its rows.  FP64 PCG forms p = z + beta p while it copies the window,
 //    which saves one of its three grid-wide waits;
-//  - kPlain: matrix and gathers from global memory, one warp per slice.
+//  - kPlain: matrix and gathers from global memory, one warp per slice;
+//  - kTurns: as kPlain, but the grid takes the rows in turn (large scalar systems, see coop_shape).
 // The other vectors are in shared memory as far as they fit, the rest in their global arrays.
 //
 // What bounds it: small systems the grid-wide waits (about 2 microseconds each), large ones the matrix
@@ -29,7 +30,7 @@
 namespace msfem {
 namespace {
 
-enum CoopMode { kResident = 0, kPlain = 1 };
+enum CoopMode { kResident = 0, kPlain = 1, kTurns = 2 };
 
 constexpr int kResidentThreads = 512;
 constexpr int kPlainThreads = 1024;
@@ -66,16 +67,21 @@ template <int MODE, int BS, class VT>
 __device__ __forceinline__ Share<VT> share_of(const SellView<VT>& A, const CoopArgs& P, unsigned char* sm, int* s_span)
 {
     Share<VT> R;
+    R.warp = threadIdx.x >> 5;
+    R.lane = threadIdx.x & 31;
+    R.nw = blockDim.x >> 5;
+    R.rest = sm;
+    if constexpr (MODE == kTurns) {
+        R.row0 = 0;
+        R.nr = P.n;
+        return R;
+    }
     R.s0 = (int)((int64_t)A.n_slices * blockIdx.x / gridDim.x);
     R.s1 = (int)((int64_t)A.n_slices * (blockIdx.x + 1) / gridDim.x);
     R.row0 = R.s0 * kSlice * BS;
     R.nr = min((R.s1 - R.s0) * kSlice * BS, max(0, P.n - R.row0));
-    R.warp = threadIdx.x >> 5;
-    R.lane = threadIdx.x & 31;
-    R.nw = blockDim.x >> 5;
     R.base = A.sp[R.s0];
-    R.rest = sm;
-    if constexpr (MODE == kPlain) return R;
+    if constexpr (MODE != kResident) return R;
     if (threadIdx.x < 2) s_span[threadIdx.x] = threadIdx.x == 0 ? 0x7fffffff : -1;
     __syncthreads();
     for (int k = R.s0 + threadIdx.x; k < R.s1; k += blockDim.x) {
@@ -160,18 +166,44 @@ __device__ __forceinline__ void fill_window(const Share<VT>& R, const VT* a, con
     }
 }
 
+// a thread's first row, and the step to its next: within the CTA's range, kTurns over the grid
+template <int MODE>
+__device__ __forceinline__ int first_row()
+{
+    return MODE == kTurns ? blockIdx.x * blockDim.x + threadIdx.x : threadIdx.x;
+}
+template <int MODE>
+__device__ __forceinline__ int row_step()
+{
+    return MODE == kTurns ? gridDim.x * blockDim.x : blockDim.x;
+}
+
+// f(row) for every row of the thread.  The product of 3x3 blocks uses all 64 registers that 1024 threads leave, so
+// its kernels read the step anew (kept in a register through the product it costs the overlap of the matrix loads:
+// 128^3, us an iteration, CG 543 against 495, FP32 319 against 277); scalar ones keep it (PCG 140^3: 105 against 114).
+template <int MODE, int BS, class F>
+__device__ __forceinline__ void each_row(int nr, int step, F&& f)
+{
+    if constexpr (BS == 3) {
+        for (int i = threadIdx.x; i < nr; i += blockDim.x) f(i);
+    } else {
+        for (int i = first_row<MODE>(); i < nr; i += step) f(i);
+    }
+}
+
 // f(row, u) in batches of U rows per thread: `load` reads the vectors of row i into slot u, `use` forms
 // and stores the new ones -- the loads of a batch are in flight together whatever the arrays alias
-template <int U, class L, class F>
+template <int MODE, int U, class L, class F>
 __device__ __forceinline__ void for_rows(int nr, L&& load, F&& use)
 {
-    for (int i0 = threadIdx.x; i0 < nr; i0 += U * blockDim.x) {
+    const int step = row_step<MODE>();
+    for (int i0 = first_row<MODE>(); i0 < nr; i0 += U * step) {
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u * (int)blockDim.x < nr) load(i0 + u * blockDim.x, u);
+            if (i0 + u * step < nr) load(i0 + u * step, u);
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u * (int)blockDim.x < nr) use(i0 + u * blockDim.x, u);
+            if (i0 + u * step < nr) use(i0 + u * step, u);
     }
 }
 
@@ -256,10 +288,18 @@ __device__ __forceinline__ void resident_product(const SellView<VT>& A, const Sh
     }
 }
 
-// kPlain: f(local row, value) for every row of A v that the CTA owns
-template <int BS, class VT, class F>
+// f(row, value) for every row of A v that the CTA owns: kPlain local rows, kTurns (scalar) the system's
+template <int MODE, int BS, class VT, class F>
 __device__ __forceinline__ void plain_product(const SellView<VT>& A, const Share<VT>& R, int keep, const VT* v, F&& f)
 {
+    if constexpr (MODE == kTurns) {
+        static_assert(BS == 1, "rows in turn: scalar systems");
+        for (int sl = blockIdx.x * R.nw + R.warp; sl < A.n_slices; sl += gridDim.x * R.nw) {
+            const VT t = sell_row_kept<VT>(A, sl, R.lane, v, false);
+            if (const int row = sl * kSlice + R.lane; row < R.nr) f(row, t);
+        }
+        return;
+    }
     const int kept = R.s0 + ((R.s1 - R.s0) * keep + 512) / 1024;
     for (int sl = R.s0 + R.warp; sl < R.s1; sl += R.nw) {
         const int lr = (sl - R.s0) * kSlice * BS + R.lane * BS;
@@ -291,7 +331,7 @@ __device__ __forceinline__ VT row_value(const VT* q, int W, int i)
     }
 }
 
-constexpr int coop_threads(int mode) { return mode == kPlain ? kPlainThreads : kResidentThreads; }
+constexpr int coop_threads(int mode) { return mode == kResident ? kResidentThreads : kPlainThreads; }
 
 // FP64 (Jacobi-)PCG as in CSSD_Matrix::MSG_PreconditioningSSOR (CSSD_Matrix.h:1336-1362), with
 // M = diag(A) or M = I: q = A p, alpha = rz / (p, q); x += alpha p, r -= alpha q; beta from (r, z) with
@@ -306,21 +346,22 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
     __shared__ int s_ok, s_span[2];
     constexpr bool RES = MODE == kResident;
     const Share<double> R = share_of<MODE, BS>(A, P, sm, s_span);
-    const int T = blockDim.x, tid = threadIdx.x;
+    const int T = row_step<MODE>(), tid = threadIdx.x;
     double* r = place(R, P, 0, gr);
     double* p = place(R, P, 1, gp);
     double* x = place(R, P, 2, gx);
     double* d = place(R, P, 3, const_cast<double*>(dinv));
-    double* q = MODE == kPlain ? place(R, P, 4, gq) : R.q;
+    double* q = MODE != kResident ? place(R, P, 4, gq) : R.q;
     auto scaled = [&](int i, double v) { return JAC ? v * d[i] : v; };
+    auto each = [&](auto&& f) { each_row<MODE, BS>(R.nr, T, f); };
     GridSync gs(P.bar, &s_ok);
     GridSum<2> sums(P.parts, gs, sh);
     const double tol2 = P.S->tol2;
     double* pp[2] = {gp, gq};
     double v[2] = {0.0, 0.0};
     if (JAC && P.in_shared > 3)
-        for (int i = tid; i < R.nr; i += T) d[i] = dinv[R.row0 + i];
-    for (int i = tid; i < R.nr; i += T) {
+        each([&](int i) { d[i] = dinv[R.row0 + i]; });
+    each([&](int i) {
         const double rv = gr[R.row0 + i], zv = scaled(i, rv);
         r[i] = rv;
         x[i] = gx[R.row0 + i];
@@ -329,7 +370,7 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
         if (RES) gz[R.row0 + i] = zv;
         v[0] += rv * zv;
         v[1] += rv * rv;
-    }
+    });
     bool live = sums.sum(v, R.nr);
     double rz = v[0], rr = v[1], beta = 0.0;
     int iter = 0, done = rr <= tol2 ? 1 : 0, breakdown = 0;
@@ -340,15 +381,15 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
             const double *z = gz, *po = pp[iter & 1];
             double* pn = pp[(iter + 1) & 1];
             fill_window<true>(R, z, po, beta);
-            for (int i = tid; i < R.nr; i += T) {
+            each([&](int i) {
                 const double pv = fma(beta, p[i], scaled(i, r[i]));
                 p[i] = pv;
                 pn[R.row0 + i] = pv;
-            }
+            });
             __syncthreads();
             resident_product<BS>(A, R, P);
             __syncthreads();
-            for (int i = tid; i < R.nr; i += T) pq[0] += p[i] * row_value<MODE, BS>(q, P.W, i);
+            each([&](int i) { pq[0] += p[i] * row_value<MODE, BS>(q, P.W, i); });
         } else {
             if (!(live = gs.sync())) break;  // the gathered p
             busy = T;
@@ -356,7 +397,7 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
                 q[i] = t;
                 pq[0] += p[i] * t;
             };
-            plain_product<BS>(A, R, P.keep, (const double*)gp, take);
+            plain_product<MODE, BS>(A, R, P.keep, (const double*)gp, take);
         }
         if (!(live = sums.sum(pq, busy))) break;
         if (pq[0] == 0.0 || pq[0] != pq[0]) {
@@ -366,7 +407,7 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
         }
         const double alpha = rz / pq[0];
         v[0] = v[1] = 0.0;
-        for (int i = tid; i < R.nr; i += T) {
+        each([&](int i) {
             x[i] += alpha * p[i];
             const double rv = r[i] - alpha * row_value<MODE, BS>(q, P.W, i);
             r[i] = rv;
@@ -374,7 +415,7 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
             if (RES) gz[R.row0 + i] = zv;
             v[0] += rv * zv;
             v[1] += rv * rv;
-        }
+        });
         if (!(live = sums.sum(v, R.nr))) break;
         beta = v[0] / rz;
         rz = v[0];
@@ -387,14 +428,14 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_pcg_coop(SellView<dou
             done = 3;
         }
         if (!RES && !done)
-            for (int i = tid; i < R.nr; i += T) {
+            each([&](int i) {
                 const double pv = fma(beta, p[i], scaled(i, r[i]));
-                p[i] = pv;
+                if (MODE != kTurns) p[i] = pv;
                 gp[R.row0 + i] = pv;
-            }
+            });
     }
     if (P.in_shared > 2)
-        for (int i = tid; i < R.nr; i += T) gx[R.row0 + i] = x[i];
+        each([&](int i) { gx[R.row0 + i] = x[i]; });
     if (live && blockIdx.x == 0 && tid == 0) {
         P.S->rz = rz;
         P.S->rr = rr;
@@ -418,20 +459,21 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_cg2_coop(SellView<flo
     __shared__ double sh[2 * 33];
     __shared__ int s_ok, s_span[2];
     const Share<float> R = share_of<MODE, BS>(A, P, sm, s_span);
-    const int T = blockDim.x, tid = threadIdx.x;
+    const int T = row_step<MODE>(), tid = threadIdx.x;
     float* r = place(R, P, 0, gr);
     float* s = place(R, P, 1, gsv);
     float* p = place(R, P, 2, gp);
     float* x = place(R, P, 3, gx);
-    float* w = MODE == kPlain ? place(R, P, 4, gw) : R.q;
+    float* w = MODE != kResident ? place(R, P, 4, gw) : R.q;
+    auto each = [&](auto&& f) { each_row<MODE, BS>(R.nr, T, f); };
     GridSync gs(P.bar, &s_ok);
     GridSum<2> sums(P.parts, gs, sh);
-    for (int i = tid; i < R.nr; i += T) {
+    each([&](int i) {
         r[i] = gr[R.row0 + i];
         x[i] = 0.0f;
         p[i] = 0.0f;
         s[i] = 0.0f;
-    }
+    });
     __syncthreads();
     double gamma = 0.0, alpha_old = 1.0, gamma_old = 0.0, rr_min = 0.0, tol2 = 0.0;
     int iter = 0, stall = 0, done = 0;
@@ -452,14 +494,14 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_cg2_coop(SellView<flo
         if constexpr (MODE == kResident) {
             resident_product<BS>(A, R, P);
             __syncthreads();
-            for (int i = tid; i < R.nr; i += T) {
+            each([&](int i) {
                 const double rv = (double)r[i];
                 v[0] += rv * rv;
                 v[1] += (double)row_value<MODE, BS>(w, P.W, i) * rv;
-            }
+            });
         } else {
             busy = T;
-            plain_product<BS>(A, R, P.keep, (const float*)gr, take);
+            plain_product<MODE, BS>(A, R, P.keep, (const float*)gr, take);
         }
         if (!(live = sums.sum(v, busy))) break;
         gamma = v[0];
@@ -486,7 +528,7 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_cg2_coop(SellView<flo
         const float al = (float)alpha, be = (float)beta;
         {
             float rs[4], ps[4], ws[4], ss[4], xs[4];
-            for_rows<MODE == kResident || BS == 3 ? 1 : 4>(
+            for_rows<MODE, MODE == kResident || BS == 3 ? 1 : 4>(
                 R.nr,
                 [&](int i, int u) {
                     rs[u] = r[i];
@@ -502,14 +544,14 @@ __global__ void __launch_bounds__(coop_threads(MODE), 1) k_cg2_coop(SellView<flo
                     s[i] = si;
                     x[i] = xs[u] + al * pi;
                     const float rv = rs[u] - al * si;
-                    r[i] = rv;
+                    if (MODE != kTurns) r[i] = rv;
                     gr[R.row0 + i] = rv;
                 });
         }
         if (!(live = gs.sync())) break;  // the gathered r
     }
     if (P.in_shared > 3)
-        for (int i = tid; i < R.nr; i += T) gx[R.row0 + i] = x[i];
+        each([&](int i) { gx[R.row0 + i] = x[i]; });
     if (live && blockIdx.x == 0 && tid == 0) {
         P.S->rr = gamma;
         P.S->iter = iter;
@@ -552,13 +594,30 @@ int coop_shape(System& s, int vectors, size_t width, bool col16, CoopArgs& P, Co
         c->smem = need + one * P.in_shared;
         return MSFEM_OK;
     }
-    c->mode = kPlain;
+    int l2 = 0;
+    MSFEM_CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    const bool scattered = scattered_columns(s);
     P.W = 1;
+    // The CTAs sweep their ranges at the same time, each behind its own window of the gathered vector.  Where the
+    // windows together exceed the L2, the grid takes the rows in turn, so that one window serves all.  Scalar FP64, us
+    // an iteration, ranges / turns: CG 160^3 175 / 176, 200^3 387 / 375, 240^3 683 / 635; 3x3 blocks, whose matrix is
+    // nine times the window's traffic, are faster by ranges (CG 128^3 495 / 515), and so are scattered columns, whose
+    // windows are the whole vector either way (CG 200^3 660 / 695).
+    if (bs == 1 && !scattered && (double)c->G * s.sell.max_span * width > l2) {
+        c->mode = kTurns;
+        c->threads = kPlainThreads;
+        P.in_shared = 0;
+        c->smem = 0;
+        return MSFEM_OK;
+    }
+    c->mode = kPlain;
     P.keep = keep_share(s, width);
     c->threads = std::min(kPlainThreads, std::max(per * 32, 256));
     // shared memory beyond this leaves the gathers too little L1 (FP64 at 100^3: 45 us an iteration with
-    // four vectors, 223 KB, in shared memory, 38 with three; FP32 at 140^3: 69 with three, 63 with two)
-    P.in_shared = (int)std::min<size_t>(vectors, std::min<size_t>(room, 176 << 10) / one);
+    // four vectors, 223 KB, in shared memory, 38 with three; FP32 at 140^3: 69 with three, 63 with two), and
+    // scattered columns need more of it (elasticity 64^3 in random order, CG: four 92 us, three 77, two and one 67; 80^3:
+    // two 171, one 130, none 125; FP32 128^3: one 415, none 345)
+    P.in_shared = (int)std::min<size_t>(vectors, std::min<size_t>(room, (scattered ? 64 : 176) << 10) / one);
     c->smem = one * P.in_shared;
     return MSFEM_OK;
 }
@@ -589,17 +648,25 @@ int coop_launch(System& s, const void* kernel, const CoopShape& c, CoopArgs& P, 
 template <bool JAC>
 const void* pcg_kernel(int mode, int bs)
 {
-    if (mode == kResident) return bs == 1 ? (const void*)k_pcg_coop<kResident, 1, JAC> : (const void*)k_pcg_coop<kResident, 3, JAC>;
+    if (mode == kTurns) return (const void*)k_pcg_coop<kTurns, 1, JAC>;
+    if (mode == kResident && bs == 1) return (const void*)k_pcg_coop<kResident, 1, JAC>;
+    if (mode == kResident) return (const void*)k_pcg_coop<kResident, 3, JAC>;
     return bs == 1 ? (const void*)k_pcg_coop<kPlain, 1, JAC> : (const void*)k_pcg_coop<kPlain, 3, JAC>;
 }
 
 const void* cg2_kernel(int mode, int bs)
 {
+    if (mode == kTurns) return (const void*)k_cg2_coop<kTurns, 1>;
     if (mode == kResident) return bs == 1 ? (const void*)k_cg2_coop<kResident, 1> : (const void*)k_cg2_coop<kResident, 3>;
     return bs == 1 ? (const void*)k_cg2_coop<kPlain, 1> : (const void*)k_cg2_coop<kPlain, 3>;
 }
 
 }  // namespace
+
+bool scattered_columns(const System& s)
+{
+    return 2 * (int64_t)s.sell.max_span > (int64_t)s.sell.n_slices * kSlice;
+}
 
 int open_shared_memory(const void* kernel, size_t* room)
 {
