@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "devutil.cuh"
 #include "internal.cuh"
@@ -45,20 +46,25 @@ struct GmCoop {
     void* gather[2];          // [n] each, VT
     double* partial;          // [2 m + 4][gridDim.x]
     void* V;                  // [m + 1][n] basis, VT, when the CTAs' shares do not fit shared memory
-    double* w;                // [n] work vector, when it does not fit either
+    void* w;                  // [n] work vector, VT, when it does not fit either
     double* H;                // [m (m + 1) / 2] packed upper triangle, column j at j (j + 1) / 2
     double* y;                // [m]
     double* out;              // [0] iterations, [1] cycles, [2] |g|^2 at the end, [3] done, [4] ||b||^2
     GridBar* bar;
 };
 
-// sums of `count` values over the grid: the CTA's value q (written by the caller into vals[q],
-// shared) -> sums[q] (shared), the CTAs added in index order by lanes and a butterfly
-__device__ __forceinline__ bool grid_sums(GridSync& gs, double* partial, const double* vals, double* sums, int count)
+// sums of `count` values over the grid: the CTA's value q (written by the caller into vals[q parts ..], shared,
+// as `parts` numbers) -> sums[q] (shared), the CTAs added in index order by lanes and a butterfly
+__device__ __forceinline__ bool grid_sums(GridSync& gs, double* partial, const double* vals, double* sums, int count,
+                                          int parts = 1)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, G = gridDim.x;
     __syncthreads();
-    for (int q = threadIdx.x; q < count; q += blockDim.x) partial[(size_t)q * G + blockIdx.x] = vals[q];
+    for (int q = threadIdx.x; q < count; q += blockDim.x) {
+        double t = vals[q * parts];
+        for (int p = 1; p < parts; p++) t += vals[q * parts + p];
+        partial[(size_t)q * G + blockIdx.x] = t;
+    }
     if (!gs.sync()) return false;
     for (int q = warp; q < count; q += nw) {
         const double* p = partial + (size_t)q * G;
@@ -76,24 +82,36 @@ __device__ __forceinline__ bool grid_sums(GridSync& gs, double* partial, const d
     return true;
 }
 
-// VS: the basis rows are in shared memory
-template <class VT, bool VS>
-__global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, GmCoop P)
+// where a CTA's rows of the basis and of the work vector are: both in shared memory, the work vector there, neither
+enum GmForm { kBasisShared, kWorkShared, kAllGlobal };
+
+// Restarts of up to kFew vectors with the basis in global memory have passes of their own (FEW): with a vector to a
+// warp most warps idle, and with a row to a thread too little is in flight.  us a step at restart 5, 10, 16, without /
+// with them (the launch-per-kernel cycle): elasticity 128^3 FP64 966, 980, 986 / 686, 710, 780 (797, 895, 1063), FP32 706,
+// 724, 728 / 422, 468, 546 (486, 594, 752); scalar 140^3 FP64 260, 283, 295 / 159, 181, 217 (230, 292, 377).  More vectors
+// fill the warps by themselves (restart 20 at 128^3 FP64: 1031, launch per kernel 1166).
+constexpr int kFew = 16;
+
+template <class VT, int FORM, bool FEW>
+__global__ void __launch_bounds__(FORM == kBasisShared ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, GmCoop P)
 {
+    constexpr bool VS = FORM == kBasisShared;
+    // the work vector holds values rounded to VT: as FP64, which spares the conversions, except where its traffic counts
+    using WT = std::conditional_t<FORM == kAllGlobal && FEW, VT, double>;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ int s_ok;
     __shared__ double s_warp[32], s_one[1], s_norm[1];
     __shared__ double s_state[4];  // [0] |g_{j+1}|, [1] stop code
     const int m = P.m, tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
     // shared memory: FP64 small arrays, then the basis rows and the work rows
-    double* h1 = reinterpret_cast<double*>(sm);  // own partial dots
-    double* h2 = h1 + m + 1;                     // summed: first projection
+    double* h1 = reinterpret_cast<double*>(sm);  // own partial dots, those of a vector in up to a part per warp
+    double* h2 = h1 + m + 1 + 32;                // summed: first projection
     double* h3 = h2 + m + 1;                     // summed: second projection
     double* cs = h3 + m + 1;
     double* sn = cs + m;
     double* g = sn + m;
     double* y = g + m + 1;
-    double* w = P.w;                             // the work vector, holding values rounded to VT
+    WT* w;
     VT* V = (VT*)P.V;
     int64_t ldv = P.n;
     GridSync gs(P.bar, &s_ok);
@@ -107,7 +125,7 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
     } else {
         V += row0;
     }
-    if (w) w += row0;
+    if constexpr (FORM == kAllGlobal) w = (WT*)P.w + row0;
     else w = y + m;
     VT* x = reinterpret_cast<VT*>(P.x);
     const VT* b = reinterpret_cast<const VT*>(P.b);
@@ -118,12 +136,12 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
             const int lr = (sl - s0) * kSlice * A.bs + lane * A.bs;
             if (A.bs == 1) {
                 const VT t = sell_row_kept<VT>(A, sl, lane, v, sl < kept);
-                if (lr < nr) w[lr] = (double)(VT)(t * (VT)scale);
+                if (lr < nr) w[lr] = (WT)(VT)(t * (VT)scale);
             } else {
                 VT t[3];
                 sell_block_kept<VT>(A, sl, lane, v, t, sl < kept);
                 if (lr < nr)
-                    for (int c = 0; c < 3; c++) w[lr + c] = (double)(VT)(t[c] * (VT)scale);
+                    for (int c = 0; c < 3; c++) w[lr + c] = (WT)(VT)(t[c] * (VT)scale);
             }
         }
         __syncthreads();
@@ -131,7 +149,7 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
     // (w, w) over the grid into s_norm[0]
     auto norm2 = [&](double* part) -> bool {
         double t = 0.0;
-        for (int r = tid; r < nr; r += T) t += w[r] * w[r];
+        for (int r = tid; r < nr; r += T) t += (double)w[r] * (double)w[r];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (lane == 0) s_warp[warp] = t;
@@ -146,7 +164,7 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
     // the vector the next product gathers: w, through the right preconditioner
     auto publish = [&](VT* to) {
         for (int r = tid; r < nr; r += T)
-            to[row0 + r] = (VT)(P.dinv ? w[r] * P.dinv[row0 + r] : w[r]);
+            to[row0 + r] = (VT)(P.dinv ? (double)w[r] * P.dinv[row0 + r] : (double)w[r]);
     };
     // h1[i] (+)= (V_i, w) on the CTA's rows [r0, r1), one vector per warp at a time
     auto dots = [&](int j, int r0, int r1, bool add) {
@@ -156,7 +174,7 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
             for (int r = r0 + lane; r < r1; r += 128)
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    if (r + 32 * u < r1) t[u] += (double)v[r + 32 * u] * w[r + 32 * u];
+                    if (r + 32 * u < r1) t[u] += (double)v[r + 32 * u] * (double)w[r + 32 * u];
             double q = (t[0] + t[1]) + (t[2] + t[3]);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
@@ -169,13 +187,13 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
         for (int r0 = 0; r0 < nr; r0 += T) {
             const int r = r0 + tid;
             if (r < nr) {
-                double t[4] = {w[r], 0.0, 0.0, 0.0};
+                double t[4] = {(double)w[r], 0.0, 0.0, 0.0};
                 int i = 0;
                 for (; i + 3 <= j; i += 4)
 #pragma unroll
                     for (int u = 0; u < 4; u++) t[u] -= h[i + u] * (double)V[(i + u) * ldv + r];
                 for (; i <= j; i++) t[0] -= h[i] * (double)V[i * ldv + r];
-                w[r] = (double)(VT)((t[0] + t[1]) + (t[2] + t[3]));
+                w[r] = (WT)(VT)((t[0] + t[1]) + (t[2] + t[3]));
             }
             if (again) {
                 __syncthreads();
@@ -184,6 +202,46 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
         }
         if (again && nr == 0)
             for (int i = tid; i <= j; i += T) h1[i] = 0.0;
+        __syncthreads();
+    };
+
+    // FEW: nw / nv warps share the rows of each of the nv vectors, a thread keeps four rows in flight, and a vector's
+    // sums stay in registers over the tiles; h1[i parts + p] = part p of vector i
+    auto few_dots = [&](int nv, int parts, int r0, int r1, double (&t)[4]) {
+        const int i = warp / parts, p = warp - i * parts;
+        if (i >= nv) return;
+        const VT* v = V + i * ldv;
+        for (int r = r0 + 128 * p + lane; r < r1; r += 128 * parts)
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (r + 32 * u < r1) t[u] += (double)v[r + 32 * u] * (double)w[r + 32 * u];
+    };
+    auto few_dots_end = [&](double (&t)[4]) {
+        double q = (t[0] + t[1]) + (t[2] + t[3]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        if (lane == 0) h1[warp] = q;
+    };
+    auto few_remove = [&](const double* h, int nv, int parts, bool again) {
+        constexpr int U = 4;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int r0 = 0; r0 < nr; r0 += U * T) {
+            double t[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) t[u] = r0 + u * T + tid < nr ? (double)w[r0 + u * T + tid] : 0.0;
+            for (int i = 0; i < nv; i++)
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (r0 + u * T + tid < nr) t[u] -= h[i] * (double)V[i * ldv + r0 + u * T + tid];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (r0 + u * T + tid < nr) w[r0 + u * T + tid] = (WT)(VT)t[u];
+            if (again) {
+                __syncthreads();
+                few_dots(nv, parts, r0, min(r0 + U * T, nr), s);
+            }
+        }
+        if (again) few_dots_end(s);
         __syncthreads();
     };
 
@@ -203,7 +261,7 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
         __syncthreads();
         if (!zero) {  // else w holds b
             product(x, 1.0);
-            for (int r = tid; r < nr; r += T) w[r] = (double)(VT)((double)b[row0 + r] - w[r]);
+            for (int r = tid; r < nr; r += T) w[r] = (WT)(VT)((double)b[row0 + r] - (double)w[r]);
         }
         zero = false;
         __syncthreads();
@@ -218,14 +276,25 @@ __global__ void __launch_bounds__(VS ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, 
         int k = 0;
         for (int j = 0; j < m; j++) {
             const double inv = norm > 0.0 ? 1.0 / norm : 0.0;
-            for (int r = tid; r < nr; r += T) V[j * ldv + r] = (VT)(w[r] * inv);
+            for (int r = tid; r < nr; r += T) V[j * ldv + r] = (VT)((double)w[r] * inv);
             __syncthreads();
             product((const VT*)P.gather[j & 1], inv);
-            dots(j, 0, nr, false);
-            if (!grid_sums(gs, part1, h1, h2, j + 1)) return;
-            remove(h2, j, true);
-            if (!grid_sums(gs, part2, h1, h3, j + 1)) return;
-            remove(h3, j, false);
+            if constexpr (FEW) {
+                const int nv = j + 1, parts = nw / nv;
+                double t[4] = {0.0, 0.0, 0.0, 0.0};
+                few_dots(nv, parts, 0, nr, t);
+                few_dots_end(t);
+                if (!grid_sums(gs, part1, h1, h2, nv, parts)) return;
+                few_remove(h2, nv, parts, true);
+                if (!grid_sums(gs, part2, h1, h3, nv, parts)) return;
+                few_remove(h3, nv, parts, false);
+            } else {
+                dots(j, 0, nr, false);
+                if (!grid_sums(gs, part1, h1, h2, j + 1)) return;
+                remove(h2, j, true);
+                if (!grid_sums(gs, part2, h1, h3, j + 1)) return;
+                remove(h3, j, false);
+            }
             publish((VT*)P.gather[(j + 1) & 1]);
             if (!norm2(part3)) return;
             norm = sqrt(s_norm[0]);
@@ -311,25 +380,33 @@ struct GmShape {
     int G, rows, threads;
     size_t smem;
     bool w_shared, basis_shared;
-    static int make(const SellView<VT>& A, int m, GmShape* out)
+    static int make(const SellView<VT>& A, int m, bool scattered, GmShape* out)
     {
         int dev = 0, sms = 0;
         MSFEM_CK(cudaGetDevice(&dev));
         MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const void *in_shared = (const void*)k_gm_coop<VT, true>, *in_global = (const void*)k_gm_coop<VT, false>;
-        size_t room_s = 0, room_g = 0;
-        MSFEM_TRY(open_shared_memory(in_shared, &room_s));
-        MSFEM_TRY(open_shared_memory(in_global, &room_g));
+        const void* kernels[3] = {(const void*)k_gm_coop<VT, kBasisShared, false>,
+                                  (const void*)k_gm_coop<VT, kWorkShared, false>,
+                                  (const void*)k_gm_coop<VT, kAllGlobal, false>};
+        if (m <= kFew) {
+            kernels[kWorkShared] = (const void*)k_gm_coop<VT, kWorkShared, true>;
+            kernels[kAllGlobal] = (const void*)k_gm_coop<VT, kAllGlobal, true>;
+        }
+        size_t room[3];
+        for (int f = 0; f < 3; f++) MSFEM_TRY(open_shared_memory(kernels[f], &room[f]));
         out->G = std::max(1, std::min(sms, A.n_slices));
         out->rows = (A.n_slices + out->G - 1) / out->G * kSlice * A.bs;
         const size_t small = sizeof(double) * (4 * (size_t)(m + 1) + 3 * (size_t)m) + 1024;
         const size_t w = sizeof(double) * out->rows, v = sizeof(VT) * (size_t)(m + 1) * out->rows;
-        const bool vs = small + w + v <= room_s;
-        out->basis_shared = vs;
-        out->w_shared = vs || small + w <= room_g;
-        out->threads = vs ? 512 : 1024;
-        out->smem = small + (out->w_shared ? w : 0) + (vs ? v : 0);
-        out->kernel = vs ? in_shared : in_global;
+        // gathers in no spatial order need some L1 (us a step, basis in shared / global memory: scalar 80^3 in random
+        // order, FP64 with restart 5, 202 KB, 110 / 59; 100^3 FP32, 223 KB, 188 / 91; 60^3 FP64 restart 10, 147 KB, 29 / 33)
+        const size_t basis_room = std::min<size_t>(room[kBasisShared], scattered ? 164 << 10 : room[kBasisShared]);
+        const GmForm form = small + w + v <= basis_room ? kBasisShared : small + w <= room[kWorkShared] ? kWorkShared : kAllGlobal;
+        out->basis_shared = form == kBasisShared;
+        out->w_shared = form != kAllGlobal;
+        out->threads = form == kBasisShared ? 512 : 1024;
+        out->smem = small + (out->w_shared ? w : 0) + (out->basis_shared ? v : 0);
+        out->kernel = kernels[form];
         return MSFEM_OK;
     }
 };
@@ -341,7 +418,7 @@ int gm_coop_run(System& s, GmCoop P, VT* V, VT* g0, VT* g1, double* out5)
 {
     SellView<VT> A = sell_view<VT>(s);
     GmShape<VT> shape;
-    MSFEM_TRY(GmShape<VT>::make(A, P.m, &shape));
+    MSFEM_TRY(GmShape<VT>::make(A, P.m, scattered_columns(s), &shape));
     const size_t np = (size_t)(2 * P.m + 4) * shape.G, nh = (size_t)P.m * (P.m + 1) / 2;
     MSFEM_TRY(s.gm.alloc(8 + np + nh + P.m + (shape.w_shared ? 0 : (size_t)P.n)));
     MSFEM_CK(cudaMemsetAsync(s.gm.p, 0, sizeof(double) * 8, s.stream));
