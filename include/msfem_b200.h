@@ -651,14 +651,14 @@ int msfem_net_loss_grad(msfem_net_t n, int cells, const float* vox, const float*
 int msfem_net_forward(msfem_net_t n, int cells, const float* vox, float* out);
 /* Predicts the bases of every cell of c into c (as msfem_cells_set_bases would); ms: device time. */
 int msfem_net_predict(msfem_net_t n, msfem_cells_t c, float* ms);
-/* Selects another tensor-core path for layers 1-3 (forward and data gradient) than the default, a
- * persistent tcgen05 kernel that multiplies each plane with the weights of all three z-taps (M = 128
- * voxels, N = 96): 0 = warp-level mma.sync, 1 =
- * tcgen05 with TMEM accumulators and M = 64 voxel tiles (N = 32 channels), 2 = tcgen05 on the
- * transposed product (M = 64 channel rows, N = 256 voxels of a plane), 3 = the M = 64 tcgen05
- * tiles in a persistent warp-specialised kernel (a producer warp fills a ring of plane slots, one
- * thread issues the MMAs into two TMEM accumulators, four epilogue warps drain them).  All compute
- * the same function (FP32 accumulation order may differ). */
+/* Tensor-core path of layers 1-3 (forward and data gradient) of this network: 4 (the default, and the
+ * fastest at every size) = a persistent tcgen05 kernel that multiplies each plane with the weights of
+ * all three z-taps (M = 128 voxels, N = 96), 0 = warp-level mma.sync, 1 = tcgen05 with TMEM
+ * accumulators and M = 64 voxel tiles (N = 32 channels), 2 = tcgen05 on the transposed product (M = 64
+ * channel rows, N = 256 voxels of a plane), 3 = the M = 64 tcgen05 tiles in a persistent
+ * warp-specialised kernel (a producer warp fills a ring of plane slots, one thread issues the MMAs into
+ * two TMEM accumulators, four epilogue warps drain them).  All compute the same function (FP32
+ * accumulation order may differ). */
 int msfem_net_set_tensor_path(msfem_net_t n, int tcgen05);
 int msfem_net_destroy(msfem_net_t n);
 

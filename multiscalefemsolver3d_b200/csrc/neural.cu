@@ -1923,7 +1923,7 @@ struct NetHandle {
     DBuf<int32_t> idx;
     DBuf<int> flag;
     DBuf<int> err;       // set by a tcgen05 kernel whose completion wait timed out
-    int tcgen05 = kStacked;  // or, selected by the caller: 0 mma.sync (k_conv32), 1 tcgen05 M=64 tiles (k_conv32_tc), 2
+    int tcgen05 = kStacked;  // or another that the caller selects: 0 mma.sync (k_conv32), 1 tcgen05 M=64 tiles (k_conv32_tc), 2
                              // tcgen05 transposed (k_conv32_tt), 3 M=64 tiles warp-specialised (k_conv32_ws)
     int sms = 148;       // multiprocessors of the device (the persistent kernel's grid)
     ~NetHandle()
@@ -2389,7 +2389,7 @@ int msfem_net_predict(msfem_net_t h, msfem_cells_t cells, float* ms)
 int msfem_net_set_tensor_path(msfem_net_t h, int tcgen05)
 {
     using namespace msfem;
-    if (!h || tcgen05 < 0 || tcgen05 > 3) {
+    if (!h || tcgen05 < 0 || tcgen05 > kStacked) {
         set_error("msfem_net_set_tensor_path: bad arguments");
         return MSFEM_ERR_ARGUMENT;
     }

@@ -51,10 +51,10 @@ class CoarseNet:
         self.n_train = 0
 
     def set_tensor_path(self, path: int):
-        """Another path for layers 1-3 than the default (tcgen05 with the z-taps stacked, the
-        fastest): 0 = warp-level mma.sync, 1 = tcgen05 with M = 64 voxel tiles, 2 = tcgen05
-        transposed product (N = 256 voxels per instruction), 3 = tcgen05 with M = 64 voxel tiles,
-        warp-specialised (load / MMA / epilogue warps) and persistent over cells."""
+        """Layers 1-3: 4 = tcgen05 with the z-taps stacked (the default, and the fastest), 0 = warp-level
+        mma.sync, 1 = tcgen05 with M = 64 voxel tiles, 2 = tcgen05 transposed product (N = 256 voxels per
+        instruction), 3 = tcgen05 with M = 64 voxel tiles, warp-specialised (load / MMA / epilogue warps) and
+        persistent over cells."""
         check(load().msfem_net_set_tensor_path(self.h, int(path)), "net_set_tensor_path")
 
     def params(self) -> np.ndarray:
