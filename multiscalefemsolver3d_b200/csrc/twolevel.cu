@@ -1222,6 +1222,7 @@ struct CoarseHandle {
     DBuf<TlState> st;
     TlState* h_st = nullptr;
     cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};  // FP32, FP64, multiplicative iteration graphs
+    size_t graph_launches[3] = {0, 0, 0};                    // kernels of a replay
     float ms_setup = 0.f;
     // multiplicative cycle (msfem_coarse_set_smoother): the textbook-orientation system, the
     // Chebyshev degree and coefficients, the prolongation in its scaling, cycle vectors
@@ -1589,6 +1590,7 @@ int inner_solve(CoarseHandle& C, int maxiter, double tau, int* iters)
         }
     };
     cudaGraphExec_t& graph = C.graph[f32 ? 0 : 1];
+    size_t& launches = C.graph_launches[f32 ? 0 : 1];
     if (!graph) {
         cudaGraph_t gr;
         MSFEM_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1598,6 +1600,7 @@ int inner_solve(CoarseHandle& C, int maxiter, double tau, int* iters)
             set_error("two-level MINRES graph capture failed: %s", cudaGetErrorString(e));
             return MSFEM_ERR_CUDA;
         }
+        MSFEM_CK(cudaGraphGetNodes(gr, nullptr, &launches));
         e = cudaGraphInstantiate(&graph, gr, 0);
         cudaGraphDestroy(gr);
         if (e != cudaSuccess) {
@@ -1612,7 +1615,7 @@ int inner_solve(CoarseHandle& C, int maxiter, double tau, int* iters)
         if (16 * rounds > maxiter + 32) break;
         for (int k = 0; k < 4; k++) MSFEM_CK(cudaGraphLaunch(graph, st));
         rounds += 4;
-        F.total_launches += 4 * 16 * 6;
+        F.total_launches += 4 * (int64_t)launches;
     }
     *iters = C.h_st->iter;
     return C.h_st->done == 3 ? MSFEM_ERR_NUMERIC : MSFEM_OK;
@@ -1737,6 +1740,7 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
         }
     };
     cudaGraphExec_t& graph = C.graph[2];
+    size_t& launches = C.graph_launches[2];
     if (!graph) {
         cudaGraph_t gr;
         MSFEM_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1746,6 +1750,7 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
             set_error("two-level MINRES graph capture failed: %s", cudaGetErrorString(e));
             return MSFEM_ERR_CUDA;
         }
+        MSFEM_CK(cudaGraphGetNodes(gr, nullptr, &launches));
         e = cudaGraphInstantiate(&graph, gr, 0);
         cudaGraphDestroy(gr);
         if (e != cudaSuccess) {
@@ -1786,7 +1791,7 @@ int inner_solve_mg(CoarseHandle& C, int maxiter, double tau, double stop2, int* 
         }
         for (int k = 0; k < 4; k++) MSFEM_CK(cudaGraphLaunch(graph, st));
         rounds += 4;
-        F.total_launches += 4 * 16 * (10 + 2 * (C.cheb_deg - 1));
+        F.total_launches += 4 * (int64_t)launches;
     }
     *iters = C.h_st->iter;
     return C.h_st->done == 3 ? MSFEM_ERR_NUMERIC : MSFEM_OK;
