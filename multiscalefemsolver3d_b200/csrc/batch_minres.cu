@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "batch.cuh"
 #include "devutil.cuh"
@@ -25,6 +26,12 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxCluster = 16;
+
+// A cluster of several CTAs a system; one CTA, whose barriers and sums are those of a block; one CTA whose system, of
+// up to 8 slices and 128 rows (some 100 KB of FP64), stays in the L1.  Face problems, ms, with cluster barriers / of a
+// block / and L1: 6 sheets of 8 squares per edge, FP32 to 1e-8, 0.39 / 0.33 / 0.27 (a CTA a system with a CSR product:
+// 0.37), 3000 of them 5.5 / 2.5 / 2.0 (4.4); 12,000 of 5, FP64 to 1e-12, 8.0 / 3.1 / 2.4 (5.6).
+enum Form { kCluster, kSolo, kTiny };
 
 template <int R>
 struct Lanes {
@@ -75,8 +82,13 @@ __device__ __forceinline__ unsigned cluster_size()
 }
 
 // all threads of the cluster; global and shared writes before it are visible after it
+template <int FORM>
 __device__ __forceinline__ void cluster_sync()
 {
+    if constexpr (FORM != kCluster) {
+        __syncthreads();
+        return;
+    }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
@@ -98,24 +110,25 @@ __device__ __forceinline__ void remote_store(int* p, unsigned rank, int v)
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(remote_addr(p, rank)), "r"(v) : "memory");
 }
 
-// matrix entries: read once per product, so they leave the L1 to the gathered vector
-__device__ __forceinline__ double load_stream(const double* p)
+// matrix entries: read once per product, so they leave the L1 to the gathered vector; TINY systems fit it whole
+template <bool TINY, class T>
+__device__ __forceinline__ T load_entry(const T* p)
 {
-    double v;
-    asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float load_stream(const float* p)
-{
-    float v;
-    asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ int load_stream(const int32_t* p)
-{
-    int v;
-    asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
+    if constexpr (TINY) {
+        return __ldg(p);
+    } else if constexpr (sizeof(T) == 8) {
+        double v;
+        asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+        return v;
+    } else if constexpr (std::is_same_v<T, float>) {
+        float v;
+        asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+        return v;
+    } else {
+        int v;
+        asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+        return v;
+    }
 }
 
 // NR neighbouring right-hand sides of one component
@@ -168,8 +181,8 @@ struct CtaShared {
     int q, conv, bad;
 };
 
-// One CTA's place in the cluster's system.
-template <int R>
+// One CTA's place in the cluster's system
+template <int R, int FORM>
 struct Place {
     int64_t slice0;        // first slice of the system
     int sl_lo, sl_hi;      // this CTA's slices within the system
@@ -184,8 +197,8 @@ struct Place {
 // The slots are read after that barrier, so a buffer may be written again only when another cluster
 // barrier has passed: two sums in a row never share one.  The residual takes buffers 2 and 3, the
 // Krylov sums 0 and 1 in turn.
-template <int R, int N>
-__device__ __forceinline__ void cluster_sum(CtaShared<R>& sh, const Place<R>& P, const int (&buf)[N],
+template <int R, int FORM, int N>
+__device__ __forceinline__ void cluster_sum(CtaShared<R>& sh, const Place<R, FORM>& P, const int (&buf)[N],
                                             double (&a)[N][Lanes<R>::NR])
 {
     using L = Lanes<R>;
@@ -201,6 +214,17 @@ __device__ __forceinline__ void cluster_sum(CtaShared<R>& sh, const Place<R>& P,
 #pragma unroll
             for (int u = 0; u < L::NR; u++) sh.red[buf[q]][P.warp * R + P.lane * L::NR + u] = a[q][u];
     __syncthreads();
+    if constexpr (FORM != kCluster) {  // the CTA's own sums, and no second barrier
+#pragma unroll
+        for (int q = 0; q < N; q++)
+#pragma unroll
+            for (int u = 0; u < L::NR; u++) {
+                double s = 0.0;
+                for (int w = 0; w < P.nw; w++) s += sh.red[buf[q]][w * R + P.j * L::NR + u];
+                a[q][u] = s;
+            }
+        return;
+    }
     for (int t = threadIdx.x; t < R * (int)P.size; t += blockDim.x) {
         const int r = t % R, dst = t / R;
 #pragma unroll
@@ -210,7 +234,7 @@ __device__ __forceinline__ void cluster_sum(CtaShared<R>& sh, const Place<R>& P,
             remote_store(&sh.slot[buf[q]][P.rank * R + r], dst, s);
         }
     }
-    cluster_sync();
+    cluster_sync<FORM>();
 #pragma unroll
     for (int q = 0; q < N; q++)
 #pragma unroll
@@ -223,8 +247,8 @@ __device__ __forceinline__ void cluster_sum(CtaShared<R>& sh, const Place<R>& P,
 
 // FP64 residual r = b - A x on the free rows (x holds the Dirichlet values), written scaled (S r)
 // into V; ||r||^2 -> sh.s1, ||S r||^2 -> sh.s2 per right-hand side.
-template <int R, class VT>
-__device__ void residual_pass(const BatchArgs& A, const Place<R>& P, VT* V, CtaShared<R>& sh)
+template <int R, class VT, int FORM>
+__device__ void residual_pass(const BatchArgs& A, const Place<R, FORM>& P, VT* V, CtaShared<R>& sh)
 {
     using L = Lanes<R>;
     double acc[2][L::NR] = {};
@@ -269,7 +293,7 @@ __device__ void residual_pass(const BatchArgs& A, const Place<R>& P, VT* V, CtaS
         }
     }
     const int buf[2] = {2, 3};  // the first Krylov sum follows with no cluster barrier between
-    cluster_sum<R, 2>(sh, P, buf, acc);
+    cluster_sum(sh, P, buf, acc);
     if (threadIdx.x < L::LPR)
 #pragma unroll
         for (int u = 0; u < L::NR; u++) {
@@ -280,8 +304,8 @@ __device__ void residual_pass(const BatchArgs& A, const Place<R>& P, VT* V, CtaS
 }
 
 // x += sign * S y on this CTA's free rows, for the right-hand sides with want[r] set (null: all)
-template <int R, class VT>
-__device__ void apply_correction(const BatchArgs& A, const Place<R>& P, const VT* Y, double sign, const int* want)
+template <int R, class VT, int FORM>
+__device__ void apply_correction(const BatchArgs& A, const Place<R, FORM>& P, const VT* Y, double sign, const int* want)
 {
     using L = Lanes<R>;
     for (int sl = P.sl_lo + P.warp; sl < P.sl_hi; sl += P.nw) {
@@ -308,8 +332,9 @@ __device__ void apply_correction(const BatchArgs& A, const Place<R>& P, const VT
 // u_{k+1} = q - alpha v_k - beta_k v_{k-1} with its norm.  The search direction and the solution of
 // step k are updated during step k + 1, next to the pass that reads v_k anyway; the scalars of
 // step k are formed by R threads while the others start the next product.
-template <int R, class VT>
-__device__ int inner_minres(const BatchArgs& A, const Place<R>& P, const VT* __restrict__ mat, VT* base, CtaShared<R>& sh)
+template <int R, class VT, int FORM>
+__device__ int inner_minres(const BatchArgs& A, const Place<R, FORM>& P, const VT* __restrict__ mat, VT* base,
+                            CtaShared<R>& sh)
 {
     using L = Lanes<R>;
     using Pk = Pack<VT, L::NR>;
@@ -371,10 +396,10 @@ __device__ int inner_minres(const BatchArgs& A, const Place<R>& P, const VT* __r
             VT acc[3][L::NR] = {};
 #pragma unroll 3
             for (int e = 0; e < width; e++) {
-                const int c = load_stream(cp + e * L::G);
+                const int c = load_entry<FORM == kTiny>(cp + e * L::G);
                 VT m[9];
 #pragma unroll
-                for (int t = 0; t < 9; t++) m[t] = load_stream(mp + (e * 9 + t) * L::G);
+                for (int t = 0; t < 9; t++) m[t] = load_entry<FORM == kTiny>(mp + (e * 9 + t) * L::G);
                 const VT* xv = u_cur + (int64_t)c * 3 * R + jr;
                 Pk x0, x1, x2;
                 x0.load(xv);
@@ -400,7 +425,7 @@ __device__ int inner_minres(const BatchArgs& A, const Place<R>& P, const VT* __r
             }
         }
         const int bufA[1] = {0};
-        cluster_sum<R, 1>(sh, P, bufA, a1);
+        cluster_sum(sh, P, bufA, a1);
         // the scalars of step k - 1 are in place since the CTA barrier of the sum above
         if (k > 0) {
             int na = 0;
@@ -445,37 +470,37 @@ __device__ int inner_minres(const BatchArgs& A, const Place<R>& P, const VT* __r
                 if (any) direction(o, vold, upd, ep, de, ig, ta);
             }
         const int bufB[1] = {1};
-        cluster_sum<R, 1>(sh, P, bufB, a2);
+        cluster_sum(sh, P, bufB, a2);
         double bn[L::NR];
 #pragma unroll
         for (int u = 0; u < L::NR; u++) bn[u] = sqrt(a2[0][u]);
-        if (threadIdx.x < L::LPR)  // j = threadIdx.x here: this lane's sums belong to rhs jr, jr + 1
-#pragma unroll
-            for (int u = 0; u < L::NR; u++) {
-                MrRhs& m = sh.mr[jr + u];
-                m.upd = m.active;
-                if (m.active) {
-                    const double alpha = a1[0][u];
-                    const double eps = m.s0 * beta[u];
-                    const double d1 = m.c0 * beta[u];
-                    const double delta = m.c1 * d1 + m.s1 * alpha;
-                    const double g1 = -m.s1 * d1 + m.c1 * alpha;
-                    const double gamma = sqrt(g1 * g1 + bn[u] * bn[u]);
-                    const double inv = gamma > 0.0 ? 1.0 / gamma : 0.0;
-                    const double cs = gamma > 0.0 ? g1 / gamma : 1.0, sn = gamma > 0.0 ? bn[u] / gamma : 0.0;
-                    m.eps = eps;
-                    m.delta = delta;
-                    m.ig = inv;
-                    m.tau = gamma > 0.0 ? cs * m.eta : 0.0;
-                    m.eta = -sn * m.eta;
-                    m.c0 = m.c1;
-                    m.s0 = m.s1;
-                    m.c1 = cs;
-                    m.s1 = sn;
-                    if (!(gamma > 0.0) || !(bn[u] > 0.0) || fabs(m.eta) <= m.target * m.b1) m.active = 0;
-                    if (!(gamma > 0.0)) m.upd = 0;
-                }
+        if (threadIdx.x < R) {  // a right-hand side each: u of the NR whose sums this lane holds
+            const bool second = L::NR == 2 && threadIdx.x >= L::LPR;
+            const double al1 = second ? a1[0][L::NR - 1] : a1[0][0], b0 = second ? beta[L::NR - 1] : beta[0];
+            const double b2 = second ? bn[L::NR - 1] : bn[0];
+            MrRhs& m = sh.mr[jr + (second ? 1 : 0)];
+            m.upd = m.active;
+            if (m.active) {
+                const double eps = m.s0 * b0;
+                const double d1 = m.c0 * b0;
+                const double delta = m.c1 * d1 + m.s1 * al1;
+                const double g1 = -m.s1 * d1 + m.c1 * al1;
+                const double gamma = sqrt(g1 * g1 + b2 * b2);
+                const double inv = gamma > 0.0 ? 1.0 / gamma : 0.0;
+                const double cs = gamma > 0.0 ? g1 / gamma : 1.0, sn = gamma > 0.0 ? b2 / gamma : 0.0;
+                m.eps = eps;
+                m.delta = delta;
+                m.ig = inv;
+                m.tau = gamma > 0.0 ? cs * m.eta : 0.0;
+                m.eta = -sn * m.eta;
+                m.c0 = m.c1;
+                m.s0 = m.s1;
+                m.c1 = cs;
+                m.s1 = sn;
+                if (!(gamma > 0.0) || !(b2 > 0.0) || fabs(m.eta) <= m.target * m.b1) m.active = 0;
+                if (!(gamma > 0.0)) m.upd = 0;
             }
+        }
 #pragma unroll
         for (int u = 0; u < L::NR; u++) {
             beta[u] = bn[u];
@@ -525,13 +550,13 @@ __device__ int inner_minres(const BatchArgs& A, const Place<R>& P, const VT* __r
 // residual has that step undone and continues with FP64 inner solves (ill-conditioned cells: FP32
 // Lanczos vectors lose orthogonality).  Every CTA of the cluster takes the same decisions from the
 // same numbers, so all reach the same barriers.
-template <int R>
+template <int R, int FORM>
 __global__ void __launch_bounds__(512) k_batch_minres(BatchArgs A, int start64)
 {
     using L = Lanes<R>;
     __shared__ CtaShared<R> sh;
     const int tid = threadIdx.x;
-    Place<R> P;
+    Place<R, FORM> P;
     P.rank = cluster_rank();
     P.size = cluster_size();
     P.warp = tid >> 5;
@@ -542,7 +567,7 @@ __global__ void __launch_bounds__(512) k_batch_minres(BatchArgs A, int start64)
     char* base = reinterpret_cast<char*>(A.work) + (int64_t)(blockIdx.x / P.size) * 6 * A.work_stride * sizeof(double);
     float* base32 = reinterpret_cast<float*>(base);
     double* base64 = reinterpret_cast<double*>(base);
-    cluster_sync();  // every CTA runs before the first remote store
+    cluster_sync<FORM>();  // every CTA runs before the first remote store
 
     for (;;) {
         if (P.rank == 0 && tid < (int)P.size) {
@@ -551,7 +576,7 @@ __global__ void __launch_bounds__(512) k_batch_minres(BatchArgs A, int start64)
             q = __shfl_sync((1u << P.size) - 1u, q, 0);
             remote_store(&sh.q, tid, q);
         }
-        cluster_sync();
+        cluster_sync<FORM>();
         const int q = sh.q;
         if (q >= A.n_sys) break;
         const int sys = A.order[q];
@@ -584,7 +609,7 @@ __global__ void __launch_bounds__(512) k_batch_minres(BatchArgs A, int start64)
             if (sh.bad) {
                 // undo those steps (their corrections are still in Y) and recompute in FP64
                 apply_correction<R, float>(A, P, base32 + 5 * A.work_stride, -1.0, sh.s_bad);
-                cluster_sync();
+                cluster_sync<FORM>();
                 use64 = 1;
                 last64 = 1;
                 if (tid < R) sh.s_bad[tid] = 0;
@@ -625,14 +650,14 @@ __global__ void __launch_bounds__(512) k_batch_minres(BatchArgs A, int start64)
                 apply_correction<R, float>(A, P, base32 + 5 * A.work_stride, 1.0, nullptr);
             }
             last64 = use64;
-            cluster_sync();
+            cluster_sync<FORM>();
         }
         if (P.rank == 0 && tid == 0) {
             A.iters[sys] = inner_total;
             A.outers[sys] = outer;
             A.rel[sys] = relmax;
         }
-        cluster_sync();  // sh.q and the scalars are free again
+        cluster_sync<FORM>();  // sh.q and the scalars are free again
     }
 }
 
@@ -744,23 +769,29 @@ int fill_values(BatchSys& b, DBuf<T>& out, bool& ok)
     return 0;
 }
 
-// The launch shape: CTAs per system (the cluster) and threads per CTA.  A product offers one slice
-// per warp, so a cluster never has more warps than the largest system has slices, rounded up.  Below
-// that the cluster doubles while all systems together ask for at most 4 CTAs per SM: few systems
-// are bound by the latency of one SM's share, many by what streams from L2 and HBM, where wider
-// clusters only add barriers.  Measured (volume problems, FP64 to 1e-12, 512 threads, ms for
-// clusters of 1 / 2 / 4 / 8 / 16): 8 cells of 8..20 hexahedra per edge 124 / 63 / 34 / 18 / 11;
-// 64 cells of 8..17: 125 / 65 / 36 / 27 / 34; 512 cells of 8..20: 309 / 302 / 338 / 380 / 428.  The
-// one-CTA kernel with a CSR product that this replaced took 660 / 590 ms on the first two, and
-// 12.6 ms against 0.9 on one cell of 8.  256 threads instead of 512 cost 1.2 to 1.7 times as much
-// on the first and last of these, and are as fast where a system has fewer than 64 slices.
+// The launch shape: CTAs per system (the cluster) and threads per CTA.  A product offers one slice per warp, so a
+// cluster never has more warps than the largest system has slices, rounded up, and a system of a few slices no more
+// than four.  Below that the cluster doubles while all systems together ask for at most 4 CTAs per SM (asked, not
+// resident: 512 threads of 128 registers fill an SM alone): few systems are bound by the latency of one SM's share,
+// many by what streams from L2 and HBM, where wider clusters only add barriers.  Measured (volume problems, 512
+// threads, ms for clusters of 1 / 2 / 4 / 8 / 16), FP64 to 1e-12: 8 cells of 8..20 hexahedra per edge 157 / 81 / 45 /
+// 23 / 14; 64 cells of 8..17: 106 / 56 / 31 / 26 / 33; 74 of 16: 97 / 57 / 61 / 57 / 65; 220 of 16: 184 / 157 / 161 /
+// 165 / 191; 512 of 8..20: 322 / 303 / 339 / 380 / 427; FP32 refinement to 1e-8: 103 / 52 / 29 / 15 / 9; 75 / 38 / 20 /
+// 14 / 19; 70 / 37 / 30 / 32 / 36; 115 / 90 / 81 / 94 / 108; 260 / 179 / 170 / 189 / 242.  So the rule is within a few
+// percent of the best but for more than 130 cells of unequal sizes, which would gain from wider clusters (150 of 8..20:
+// 147 with its 2, 118 with 4; 300: 292 with its 1, 199 with 2).  Face problems, six a cell, are fastest with its 1 or
+// 2.  The one-CTA kernel with a CSR product that this replaced took 660 / 590 ms on the first two, and 12.6 ms against
+// 0.9 on one cell of 8.  256 threads instead of 512 cost 1.2 to 1.7 times as much on many large systems, and are as
+// fast where a system has fewer than 64 slices; warps without a slice cost their barriers (12,000 sheets of 16 free
+// rows, FP64: 32 threads 2.4 ms, 128 5.3).
 struct Shape {
     int threads, cluster;
 };
 
 Shape launch_shape(const BatchSys& b, int threads, int sms)
 {
-    if (threads <= 0) threads = b.max_slices <= 8 ? 128 : (b.max_slices < 64 ? 256 : 512);
+    if (threads <= 0)
+        threads = b.max_slices <= 8 ? 32 * std::min(std::max(b.max_slices, 1), 4) : (b.max_slices < 64 ? 256 : 512);
     Shape s{threads, 1};
     while (s.cluster < kMaxCluster && s.cluster * (threads / 32) < b.max_slices &&
            (int64_t)b.n_sys * 2 * s.cluster <= 4 * (int64_t)sms)
@@ -771,7 +802,10 @@ Shape launch_shape(const BatchSys& b, int threads, int sms)
 template <int R>
 int launch_minres(BatchSys& b, double* d_x, int start64, double tol, int maxiter, const Shape& shape)
 {
-    auto kern = k_batch_minres<R>;
+    const bool tiny = b.max_slices <= 8 && b.max_slices * Lanes<R>::G <= 128;
+    auto kern = shape.cluster > 1 ? k_batch_minres<R, kCluster>
+                : tiny            ? k_batch_minres<R, kTiny>
+                                  : k_batch_minres<R, kSolo>;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
