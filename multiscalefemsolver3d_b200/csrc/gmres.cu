@@ -418,7 +418,7 @@ int gm_coop_run(System& s, GmCoop P, VT* V, VT* g0, VT* g1, double* out5)
 {
     SellView<VT> A = sell_view<VT>(s);
     GmShape<VT> shape;
-    MSFEM_TRY(GmShape<VT>::make(A, P.m, scattered_columns(s), &shape));
+    MSFEM_TRY(GmShape<VT>::make(A, P.m, s.sell.scattered, &shape));
     const size_t np = (size_t)(2 * P.m + 4) * shape.G, nh = (size_t)P.m * (P.m + 1) / 2;
     MSFEM_TRY(s.gm.alloc(8 + np + nh + P.m + (shape.w_shared ? 0 : (size_t)P.n)));
     MSFEM_CK(cudaMemsetAsync(s.gm.p, 0, sizeof(double) * 8, s.stream));

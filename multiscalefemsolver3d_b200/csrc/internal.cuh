@@ -82,6 +82,8 @@ struct Sell {
     int max_width = 0;   // widest slice, in entries (blocks) per row
     DBuf<int2> span;     // lowest and highest column (node) of each slice
     int max_span = 0;    // widest column range of an SM's share of the slices
+    bool scattered = false;    // most slices span more than half of the system: nodes in no spatial order
+    double slice_span = 0.0;   // mean column range of the slices that do not
     DBuf<int64_t> slice_ptr;
     DBuf<int32_t> col;    // absolute column (3x3 blocks, or scalar when deltas do not fit 16 bits)
     DBuf<int16_t> col16;  // scalar: column - min(row, n-1), when every delta fits in 16 bits
@@ -231,9 +233,6 @@ int read_state(System& s);
 // dynamic part, what its own arrays leave.  The limit belongs to the kernel and not to a handle, so it is always
 // set to this one value: another thread's solve of another size finds it the same.
 int open_shared_memory(const void* kernel, size_t* room);
-// the columns of an SM's share of the rows reach over more than half of the system (nodes in no spatial order): the
-// gathered vector has no window, and its loads need the L1
-bool scattered_columns(const System& s);
 // ---- CG in one cooperative launch (krylov_coop.cu): S->tol2 set; iter, rr, done, breakdown left in
 // the host's KState mirror.  FP64 from the residual r; FP32 from x = 0 with right-hand side r, to tol
 // times its norm, or until (r, r) has not set a 2 % low for stall_limit iterations

@@ -596,14 +596,16 @@ int coop_shape(System& s, int vectors, size_t width, bool col16, CoopArgs& P, Co
     }
     int l2 = 0;
     MSFEM_CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
-    const bool scattered = scattered_columns(s);
+    // the window of a CTA's range, of which a few columns may lie far away; without a spatial order there is none
+    const double window_of_range = s.sell.slice_span + (double)per * kSlice;
+    const bool scattered = s.sell.scattered;
     P.W = 1;
     // The CTAs sweep their ranges at the same time, each behind its own window of the gathered vector.  Where the
     // windows together exceed the L2, the grid takes the rows in turn, so that one window serves all.  Scalar FP64, us
     // an iteration, ranges / turns: CG 160^3 175 / 176, 200^3 387 / 375, 240^3 683 / 635; 3x3 blocks, whose matrix is
     // nine times the window's traffic, are faster by ranges (CG 128^3 495 / 515), and so are scattered columns, whose
     // windows are the whole vector either way (CG 200^3 660 / 695).
-    if (bs == 1 && !scattered && (double)c->G * s.sell.max_span * width > l2) {
+    if (bs == 1 && !scattered && c->G * window_of_range * width > l2) {
         c->mode = kTurns;
         c->threads = kPlainThreads;
         P.in_shared = 0;
@@ -662,11 +664,6 @@ const void* cg2_kernel(int mode, int bs)
 }
 
 }  // namespace
-
-bool scattered_columns(const System& s)
-{
-    return 2 * (int64_t)s.sell.max_span > (int64_t)s.sell.n_slices * kSlice;
-}
 
 int open_shared_memory(const void* kernel, size_t* room)
 {

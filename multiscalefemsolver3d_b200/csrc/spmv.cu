@@ -44,9 +44,10 @@ __global__ void k_slice_width(int n_rows, int n_slices, const int32_t* __restric
     }
 }
 
-// lowest and highest column (node) of each slice
+// lowest and highest column (node) of each slice; reach[0]: slices that span more than half of the system, reach[1]:
+// the others' columns
 __global__ void k_slice_span(int n_rows, int n_slices, const int32_t* __restrict__ rp, const int32_t* __restrict__ ncol,
-                             int2* __restrict__ span)
+                             int2* __restrict__ span, unsigned long long* __restrict__ reach)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n_slices) return;
@@ -62,7 +63,12 @@ __global__ void k_slice_span(int n_rows, int n_slices, const int32_t* __restrict
         lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
-    if (lane == 0) span[warp] = make_int2(lo, hi);
+    if (lane == 0) {
+        span[warp] = make_int2(lo, hi);
+        const int columns = hi - lo + 1;
+        if (columns > n_rows / 2) atomicAdd(&reach[0], 1ull);
+        else atomicAdd(&reach[1], (unsigned long long)columns);
+    }
 }
 
 // the widest span of G equal shares of the slices
@@ -310,7 +316,11 @@ int prepare_sell(System& s)
         int sms = 0;
         MSFEM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
         MSFEM_TRY(S.span.alloc((size_t)S.n_slices));
-        k_slice_span<<<grid_for((int64_t)S.n_slices * 32, 256), 256, 0, st>>>(nbr, S.n_slices, s.nrp.p, s.ncol.p, S.span.p);
+        DBuf<unsigned long long> reach;
+        MSFEM_TRY(reach.alloc(2));
+        MSFEM_CK(cudaMemsetAsync(reach.p, 0, 2 * sizeof(unsigned long long), st));
+        k_slice_span<<<grid_for((int64_t)S.n_slices * 32, 256), 256, 0, st>>>(nbr, S.n_slices, s.nrp.p, s.ncol.p, S.span.p,
+                                                                              reach.p);
         k_share_span<<<1, 256, 0, st>>>(S.n_slices, std::min(sms, S.n_slices), S.span.p, widest.p + 1);
         k_slice_width<<<grid_for((int64_t)S.n_slices * 32, 256), 256, 0, st>>>(nbr, S.n_slices, s.nrp.p,
                                                                                s.bs == 1 ? kChunk : 1, w.p, widest.p);
@@ -323,10 +333,14 @@ int prepare_sell(System& s)
         int64_t stored = 0;
         MSFEM_CK(cudaMemcpyAsync(&stored, S.slice_ptr.p + S.n_slices, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         int wide[2] = {0, 0};
+        unsigned long long far[2] = {0, 0};
         MSFEM_CK(cudaMemcpyAsync(wide, widest.p, sizeof(wide), cudaMemcpyDeviceToHost, st));
+        MSFEM_CK(cudaMemcpyAsync(far, reach.p, sizeof(far), cudaMemcpyDeviceToHost, st));
         MSFEM_CK(cudaStreamSynchronize(st));
         S.max_width = wide[0];
         S.max_span = wide[1];
+        S.scattered = 2 * far[0] > (unsigned long long)S.n_slices;
+        S.slice_span = (double)far[1] / std::max<double>(1.0, (double)S.n_slices - (double)far[0]);
         S.stored = stored;
         MSFEM_TRY(S.col.alloc((size_t)stored));
         const size_t nv = (size_t)stored * (s.bs == 1 ? 1 : 9);
