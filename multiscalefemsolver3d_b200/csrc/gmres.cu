@@ -86,17 +86,18 @@ __device__ __forceinline__ bool grid_sums(GridSync& gs, double* partial, const d
 enum GmForm { kBasisShared, kWorkShared, kAllGlobal };
 
 // Restarts of up to kFew vectors with the basis in global memory have passes of their own (FEW): with a vector to a
-// warp most warps idle, and with a row to a thread too little is in flight.  us a step at restart 5, 10, 16, without /
-// with them (the launch-per-kernel cycle): elasticity 128^3 FP64 966, 980, 986 / 686, 710, 780 (797, 895, 1063), FP32 706,
-// 724, 728 / 422, 468, 546 (486, 594, 752); scalar 140^3 FP64 260, 283, 295 / 159, 181, 217 (230, 292, 377).  More vectors
-// fill the warps by themselves (restart 20 at 128^3 FP64: 1031, launch per kernel 1166).
+// warp most warps idle, and with a row to a thread too little is in flight.  us a step at restart 5, 10, 16, without
+// / with them (the launch-per-kernel cycle): elasticity 128^3 FP64 966, 980, 986 / 686, 710, 780 (797, 895, 1063),
+// FP32 706, 724, 728 / 422, 468, 546 (486, 594, 752); scalar 140^3 FP64 260, 283, 295 / 159, 181, 217 (230, 292,
+// 377).  More vectors fill the warps by themselves (restart 20 at 128^3 FP64: 1031, launch per kernel 1166).
 constexpr int kFew = 16;
 
 template <class VT, int FORM, bool FEW>
 __global__ void __launch_bounds__(FORM == kBasisShared ? 512 : 1024, 1) k_gm_coop(SellView<VT> A, GmCoop P)
 {
     constexpr bool VS = FORM == kBasisShared;
-    // the work vector holds values rounded to VT: as FP64, which spares the conversions, except where its traffic counts
+    // the work vector holds values rounded to VT: as FP64, which spares the conversions, except where its traffic
+    // counts
     using WT = std::conditional_t<FORM == kAllGlobal && FEW, VT, double>;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ int s_ok;
@@ -396,12 +397,16 @@ struct GmShape {
         for (int f = 0; f < 3; f++) MSFEM_TRY(open_shared_memory(kernels[f], &room[f]));
         out->G = std::max(1, std::min(sms, A.n_slices));
         out->rows = (A.n_slices + out->G - 1) / out->G * kSlice * A.bs;
+        // the small arrays; the 1 KB holds the parts of h1 too
         const size_t small = sizeof(double) * (4 * (size_t)(m + 1) + 3 * (size_t)m) + 1024;
         const size_t w = sizeof(double) * out->rows, v = sizeof(VT) * (size_t)(m + 1) * out->rows;
         // gathers in no spatial order need some L1 (us a step, basis in shared / global memory: scalar 80^3 in random
-        // order, FP64 with restart 5, 202 KB, 110 / 59; 100^3 FP32, 223 KB, 188 / 91; 60^3 FP64 restart 10, 147 KB, 29 / 33)
+        // order, FP64 with restart 5, 202 KB, 110 / 59; 100^3 FP32, 223 KB, 188 / 91; 60^3 FP64 restart 10, 147 KB,
+        // 29 / 33)
         const size_t basis_room = std::min<size_t>(room[kBasisShared], scattered ? 164 << 10 : room[kBasisShared]);
-        const GmForm form = small + w + v <= basis_room ? kBasisShared : small + w <= room[kWorkShared] ? kWorkShared : kAllGlobal;
+        const GmForm form = small + w + v <= basis_room      ? kBasisShared
+                            : small + w <= room[kWorkShared] ? kWorkShared
+                                                             : kAllGlobal;
         out->basis_shared = form == kBasisShared;
         out->w_shared = form != kAllGlobal;
         out->threads = form == kBasisShared ? 512 : 1024;

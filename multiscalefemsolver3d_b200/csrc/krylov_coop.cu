@@ -1,8 +1,8 @@
 // Conjugate gradients, a whole solve in one cooperative launch.
 //
 // One CTA per SM owns a contiguous range of matrix slices.  The inner products are grid sums
-// (GridSum, a barrier too) and every CTA derives the step's scalars itself from the same sums, so nothing waits for
-// the host between iterations and there is nothing to capture.  The vector that the product gathers is
+// (GridSum, a barrier too) and every CTA derives the step's scalars itself from the same sums, so nothing
+// waits for the host between iterations and there is nothing to capture.  The vector that the product gathers is
 // written to global memory by its owners; a CTA then copies the range that its columns span (its
 // window) into shared memory once per iteration and gathers there.
 //
@@ -14,13 +14,13 @@
 //  - kTurns: as kPlain, but the grid takes the rows in turn (large scalar systems, see coop_shape).
 // The other vectors are in shared memory as far as they fit, the rest in their global arrays.
 //
-// What bounds it: small systems the grid-wide waits (about 2 microseconds each), large ones the matrix
-// from L2 or HBM.  The launch-per-kernel loops this replaces (two kernels per FP32 iteration, three
-// per FP64 one, replayed as CUDA graphs) against this, us per iteration: FP64 PCG, scalar 20^3 16.0 -> 7.2,
-// 60^3 22.3 -> 12.6, 100^3 53.9 -> 38; elasticity 20^3 27.1 -> 8.0, 40^3 36.7 -> 16.4; FP32 CG, scalar 60^3 14.7 ->
-// 8.6, 100^3 32.2 -> 21.2; elasticity 40^3 25.5 -> 10.6.  What was tried and not kept for the streaming form: bulk
-// copies of the slices into per-warp shared-memory rings (15.7 against 12.1 us, FP32 80^3), columns
-// prefetched one slice ahead (19.3 against 17.4 with everything streamed).
+// What bounds it: small systems the grid-wide waits (about 2 microseconds each), large ones the matrix from L2 or
+// HBM.  The launch-per-kernel loops this replaces (two kernels per FP32 iteration, three per FP64 one, replayed as
+// CUDA graphs) against this, us per iteration: FP64 PCG, scalar 20^3 16.0 -> 7.2, 60^3 22.3 -> 12.6, 100^3 53.9 ->
+// 38, 200^3 469 -> 388; elasticity 20^3 24.8 -> 7.8, 40^3 36.7 -> 20, 128^3 572 -> 520 (CG 505 -> 495); FP32 CG,
+// scalar 60^3 14.7 -> 8.6, 100^3 32.2 -> 21.2, 200^3 260 -> 230; elasticity 40^3 24.4 -> 9.1, 128^3 295 -> 277.  What
+// was tried and not kept for the streaming form: bulk copies of the slices into per-warp shared-memory rings (15.7
+// against 12.1 us, FP32 80^3), columns prefetched one slice ahead (19.3 against 17.4 with everything streamed).
 #include <algorithm>
 #include <cstring>
 
@@ -180,7 +180,8 @@ __device__ __forceinline__ int row_step()
 
 // f(row) for every row of the thread.  The product of 3x3 blocks uses all 64 registers that 1024 threads leave, so
 // its kernels read the step anew (kept in a register through the product it costs the overlap of the matrix loads:
-// 128^3, us an iteration, CG 543 against 495, FP32 319 against 277); scalar ones keep it (PCG 140^3: 105 against 114).
+// 128^3, us an iteration, CG 543 against 495, FP32 319 against 277); scalar ones keep it (PCG 140^3: 105 against
+// 114).
 template <int MODE, int BS, class F>
 __device__ __forceinline__ void each_row(int nr, int step, F&& f)
 {
@@ -601,10 +602,10 @@ int coop_shape(System& s, int vectors, size_t width, bool col16, CoopArgs& P, Co
     const bool scattered = s.sell.scattered;
     P.W = 1;
     // The CTAs sweep their ranges at the same time, each behind its own window of the gathered vector.  Where the
-    // windows together exceed the L2, the grid takes the rows in turn, so that one window serves all.  Scalar FP64, us
-    // an iteration, ranges / turns: CG 160^3 175 / 176, 200^3 387 / 375, 240^3 683 / 635; 3x3 blocks, whose matrix is
-    // nine times the window's traffic, are faster by ranges (CG 128^3 495 / 515), and so are scattered columns, whose
-    // windows are the whole vector either way (CG 200^3 660 / 695).
+    // windows together exceed the L2, the grid takes the rows in turn, so that one window serves all.  Scalar FP64,
+    // us an iteration, ranges / turns: CG 160^3 175 / 176, 200^3 387 / 375, 240^3 683 / 635; 3x3 blocks, whose matrix
+    // is nine times the window's traffic, are faster by ranges (CG 128^3 495 / 515), and so are scattered columns,
+    // whose windows are the whole vector either way (CG 200^3 660 / 695).
     if (bs == 1 && !scattered && c->G * window_of_range * width > l2) {
         c->mode = kTurns;
         c->threads = kPlainThreads;
@@ -615,10 +616,10 @@ int coop_shape(System& s, int vectors, size_t width, bool col16, CoopArgs& P, Co
     c->mode = kPlain;
     P.keep = keep_share(s, width);
     c->threads = std::min(kPlainThreads, std::max(per * 32, 256));
-    // shared memory beyond this leaves the gathers too little L1 (FP64 at 100^3: 45 us an iteration with
-    // four vectors, 223 KB, in shared memory, 38 with three; FP32 at 140^3: 69 with three, 63 with two), and
-    // scattered columns need more of it (elasticity 64^3 in random order, CG: four 92 us, three 77, two and one 67; 80^3:
-    // two 171, one 130, none 125; FP32 128^3: one 415, none 345)
+    // shared memory beyond this leaves the gathers too little L1 (FP64 at 100^3: 45 us an iteration with four
+    // vectors, 223 KB, in shared memory, 38 with three; FP32 at 140^3: 69 with three, 63 with two), and scattered
+    // columns need more of it (elasticity 64^3 in random order, CG: four 92 us, three 77, two and one 67; 80^3: two
+    // 171, one 130, none 125; FP32 128^3: one 415, none 345)
     P.in_shared = (int)std::min<size_t>(vectors, std::min<size_t>(room, (scattered ? 64 : 176) << 10) / one);
     c->smem = one * P.in_shared;
     return MSFEM_OK;
@@ -659,7 +660,8 @@ const void* pcg_kernel(int mode, int bs)
 const void* cg2_kernel(int mode, int bs)
 {
     if (mode == kTurns) return (const void*)k_cg2_coop<kTurns, 1>;
-    if (mode == kResident) return bs == 1 ? (const void*)k_cg2_coop<kResident, 1> : (const void*)k_cg2_coop<kResident, 3>;
+    if (mode == kResident && bs == 1) return (const void*)k_cg2_coop<kResident, 1>;
+    if (mode == kResident) return (const void*)k_cg2_coop<kResident, 3>;
     return bs == 1 ? (const void*)k_cg2_coop<kPlain, 1> : (const void*)k_cg2_coop<kPlain, 3>;
 }
 

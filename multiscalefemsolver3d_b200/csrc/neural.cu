@@ -479,10 +479,10 @@ __global__ void __launch_bounds__(256, 1) k_conv32(int n_cells, const __nv_bfloa
             for (int nt = 0; nt < 4; nt++)
 #pragma unroll
                 for (int q = 0; q < 4; q++) acc[mt][nt][q] = 0.f;
-        // The k16 steps run dz, dy, dx, k half (the order of the sums on every path): with the last two fixed (i below), the x-rows of dy + 1 are
-        // those of dy moved by one, so the four fragments of each of the six (dx, half) stay in registers,
-        // the row that dy leaves behind is replaced at once (its successor is needed six steps later), and
-        // after dy = 2 the first four rows of the next plane take their places.
+        // The k16 steps run dz, dy, dx, k half (the order of the sums on every path): with the last two fixed (i below), the
+        // x-rows of dy + 1 are those of dy moved by one, so the four fragments of each of the six (dx, half) stay in registers,
+        // the row that dy leaves behind is replaced at once (its successor is needed six steps later), and after dy = 2 the first
+        // four rows of the next plane take their places.
         uint32_t a[6][4][4], b[2][4][2];
         auto fetch_a = [&](uint32_t ab, int i, int row) {
             ldsm_x4(a[i][row & 3], ab + 2 * (i & 1) * kCvChunk + (row * 18 + (i >> 1)) * 16);
@@ -1382,8 +1382,8 @@ __global__ void __launch_bounds__(kStThreads, 1) k_conv32_st(int n_cells, const 
         if (ok)
             for (int k = max(g - 2, 0); k < g; k++) mb_arrive(full(k & (kStSlots - 1)));
     } else if (warp == 9) {
-        // one thread, chosen by elect.sync: the compiler then knows that it is one and issues an instruction in
-        // 60 clocks; behind `lane == 0` it loops over the active lanes to make the operands uniform (150)
+        // one thread, chosen by elect.sync: an instruction takes 60 clocks, behind `lane == 0` 152 (measured with a
+        // loop of them alone)
         if (elect_one()) {
             const uint32_t a0 = smem_u32(sm), b0 = smem_u32(sm) + kStW;
             int g = 0, o0 = 0;  // planes so far; outputs before this segment: output q is number o0 + q - qa
